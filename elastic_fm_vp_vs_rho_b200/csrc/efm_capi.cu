@@ -22,16 +22,12 @@ extern "C" cudaError_t efm_launch_stress(int pass, const EfmInst *insts, int nin
                                          int it, cudaStream_t s);
 extern "C" cudaError_t efm_launch_velocity(int pass, const EfmInst *insts, int ninst, int tiles,
                                            int it, cudaStream_t s);
-extern "C" cudaError_t efm_launch_stream(int pass, int kind, int rows, int ring,
-                                         const EfmInst *insts, int ninst, int tiles, int it,
-                                         cudaStream_t s);
+extern "C" cudaError_t efm_launch_stream(int ps, int pv, int illum, int rows, int ring, const EfmInst *ts, int ns,
+                                         int cs, const EfmInst *tv, int nv, int cv, int grid, int it, int *counter,
+                                         unsigned int lim, unsigned int *err, cudaStream_t s);
 extern "C" cudaError_t efm_stream_init_attributes();
+extern "C" int efm_stream_slots(int rows, int ring);
 extern "C" void efm_stream_set_pdl(int enable);
-extern "C" cudaError_t efm_launch_pair(int which, int rows, int ring, const EfmInst *ts,
-                                       int tiles_s, const EfmInst *tv, int tiles_v, int ninst,
-                                       int it, cudaStream_t s);
-extern "C" cudaError_t efm_launch_image(const EfmInst *insts, int ninst, int tiles, int it,
-                                        cudaStream_t s);
 extern "C" cudaError_t efm_launch_exact(int kind, const EfmExact *t, int n, int tiles, int step,
                                         int slot, cudaStream_t s);
 extern "C" cudaError_t efm_launch_exact_stream(int kind, int rows, const EfmExact *t, int n,
@@ -70,7 +66,8 @@ struct Inst {
     uint32_t *rec_mask = nullptr;
     int *rec_lin = nullptr, *rec_id = nullptr;
     int *rec_wfirst = nullptr;    // per mask word: first sorted entry of its cells, or -1
-    uint8_t *rec_tile = nullptr;  // [ny][tiles_z][tiles_x] of the streaming layout
+    uint8_t *rec_col = nullptr;   // [tile][ny] of the streaming layout rec_shape
+    int rec_shape[6] = {};        // tw th ox oz tiles_x tiles_z rec_col was built for
     float *aux = nullptr;         // 1/mu, 1/rho
     float *fields = nullptr;  // va(3) t(6) | vb(3) bv(3) bt(6) when gradient-capable
     bool fields_grad = false;
@@ -174,8 +171,11 @@ struct efm_ctx {
     int ex_cap = 0;
     CUtensorMap *d_maps = nullptr;  // EFM_MAPS_PER_INST per instance
     int maps_cap = 0;
-    unsigned int *d_err = nullptr;
-    int tiles[16] = {};             // total tiles of each table slot (T_NSLOT <= 16)
+    unsigned int *d_err = nullptr;  // error word, then the streaming launches' chunk counter
+    int *d_count = nullptr;
+    int tiles[16] = {};             // total tiles / chunks of each table slot (T_NSLOT <= 16)
+    // per table slot (entries by falling step count): each entry's steps, chunks up to and with it
+    std::vector<int> steps[16], cum[16];
     // CUDA graphs of the time loops (0: forward, 1: gradient), replayed while the key holds
     int opt_graph = 1;
     cudaStream_t cap_stream = nullptr;  // private capture stream (the caller's may be legacy)
@@ -187,13 +187,12 @@ struct efm_ctx {
 };
 
 // table slots of efm_ctx::d_tab (n entries each)
+// (T_REV_VF*: the rebuild velocity over the whole grid, its first two steps)
 enum { T_FWD_S, T_FWD_V, T_ADJ_S, T_ADJ_V, T_REV_V0, T_REV_V1, T_REV_S0, T_REV_S1, T_IMG0,
-       T_IMG1, T_NSLOT };
+       T_IMG1, T_REV_VF0, T_REV_VF1, T_NSLOT };
 // tensor-map blocks per instance
-// (the rebuild velocity's block ends with the three maps its new velocity is stored through)
-enum { M_FWD_S = 0, M_FWD_V = 11, M_ADJ_S = 21, M_ADJ_V = 32, M_REV_S0 = 42, M_REV_S1 = 53,
-       M_REV_V0 = 64, M_REV_V1 = 77, M_IMG0 = 90, M_IMG1 = 110, EFM_MAPS_PER_INST = 130 };
-#define EFM_IMG_TZ 4
+enum { M_FWD_S = 0, M_FWD_V = 12, M_ADJ_S = 24, M_ADJ_V = 36, M_REV_S0 = 48, M_REV_S1 = 60,
+       M_REV_V0 = 72, M_REV_V1 = 84, M_IMG0 = 96, M_IMG1 = 108, EFM_MAPS_PER_INST = 120 };
 static_assert(T_NSLOT <= 16, "efm_ctx::tiles holds 16 table slots");
 
 namespace {
@@ -264,6 +263,15 @@ int run_loop(efm_ctx *ctx, int which, const std::vector<int64_t> &key, cudaStrea
     EFM_CK(cudaGraphLaunch(L.exec, s));
     for (int k = 0; k < EFM_NKERN; ++k) ctx->launches[k] += L.launches[k];
     return EFM_OK;
+}
+
+// What the launches of table slots [lo, hi] bake in: tiles, and the chunks and steps of every entry.
+void add_table_key(const efm_ctx *ctx, int lo, int hi, std::vector<int64_t> &key) {
+    for (int k = lo; k <= hi; ++k) {
+        key.push_back(ctx->tiles[k]);
+        key.insert(key.end(), ctx->steps[k].begin(), ctx->steps[k].end());
+        key.insert(key.end(), ctx->cum[k].begin(), ctx->cum[k].end());
+    }
 }
 
 void drop_loops(efm_ctx *ctx) {
@@ -339,11 +347,85 @@ void layout_naive(EfmInst &d) {
     d.ychunk = 0;
 }
 
-void layout_stream(EfmInst &d, int ychunk, int tz) {
-    d.tiles_x = (d.nx + EFM_STX - 1) / EFM_STX;
-    d.tiles_z = (d.nz + tz - 1) / tz;
-    d.ychunk = ychunk;
-    d.tiles_y = (d.ny + ychunk - 1) / ychunk;
+// A streaming pass's cells: x from x0 (a multiple of 4: TMA boxes start on 16 bytes), z from z0,
+// planes [y0, y1).
+struct Region {
+    int x0, x1, z0, z1, y0, y1;
+};
+
+// The tile of at most 2 nt cells that covers a region's planes at least cost: per tile the cells,
+// a third for the neighbour columns and rows they load, and a fixed part as large as a full tile
+// (a plane takes a block nearly the same time whatever it holds).  128 x 92: 28 tiles of 64 x 7,
+// forward stress and velocity 22.4 and 26.0 us; 31 tiles of 128 x 3, 28.0 and 32.6.
+void shape_of(const Region &r, int nt, int *tw, int *th) {
+    double best = 1e30;
+    *tw = 64;
+    *th = efm_st_cells(nt) / 64;
+    for (int w = 16; w <= 252; w += 4) {
+        const int nx = (r.x1 - r.x0 + w - 1) / w;
+        for (int h = 1; h * w <= efm_st_cells(nt); ++h) {
+            if (!efm_shape_ok(nt, w, h)) continue;
+            const double tiles = (double)nx * ((r.z1 - r.z0 + h - 1) / h);
+            const double cost = tiles * (w * h + 0.35 * (w + 8) * (h + 1) + efm_st_cells(nt));
+            if (cost < best - 1e-9) {
+                best = cost;
+                *tw = w;
+                *th = h;
+            }
+        }
+    }
+}
+
+void layout_stream(EfmInst &d, const Region &r, int nt, const int *shape = nullptr) {
+    if (shape) {
+        d.tw = shape[0];
+        d.th = shape[1];
+    } else {
+        shape_of(r, nt, &d.tw, &d.th);
+    }
+    d.ox = r.x0;
+    d.oz = r.z0;
+    d.ylo = r.y0;
+    d.yhi = r.y1;
+    d.tiles_x = (r.x1 - r.x0 + d.tw - 1) / d.tw;
+    d.tiles_z = (r.z1 - r.z0 + d.th - 1) / d.th;
+    d.ychunk = d.tiles_y = 0;  // chunk_table
+}
+
+// Planes per chunk of a launch's tables (n entries each, one or two of them).  `slots` blocks fetch
+// the chunks one by one.  While the fields fit in L2 a plane takes a block about the same time
+// whatever the others do, a chunk costs its planes and about 1.3 more (first slot, set-up), and
+// the launch lasts the rounds of chunks; a single round also lasts its slowest (CPML) chunk.
+// Larger grids wait for DRAM: the first slot loads about 0.45 of a plane's bytes, and the blocks
+// finish within most of a chunk of each other.  Forward stress, us: 128 x 128 x 96, 4 planes
+// 23.7, 6 planes 22.4 (two rounds), 8 planes 26.7, 16 planes (one round) 27.5; 256 x 256 x 128,
+// 4 planes 105.5, 8 planes 103.9, 16 planes 108.3; the rule takes 6 and 8.
+int chunk_planes(const efm_ctx *ctx, std::initializer_list<const EfmInst *> tables, int n, int slots) {
+    if (ctx->opt_ychunk > 0) return ctx->opt_ychunk;
+    double cells = 0;
+    for (int i = 0; i < n; ++i) cells += (double)(*tables.begin())[i].vol;
+    const bool dram = cells * 60 * tables.size() > 126e6;  // a pass moves about 15 volumes
+    int best = 1;
+    double score = 1e30;
+    for (int yc = 1; yc <= EFM_MAX_YCHUNK; ++yc) {
+        double chunks = 0;
+        for (const EfmInst *t : tables)
+            for (int i = 0; i < n; ++i)
+                chunks += (double)t[i].tiles_x * t[i].tiles_z * ((t[i].yhi - t[i].ylo + yc - 1) / yc);
+        const double r = chunks / slots;
+        double c;
+        if (dram)
+            c = r * (yc + 0.45) + 0.7 * yc;
+        else if (tables.size() == 1)
+            c = std::ceil(r) * (yc + 1.3) * (r <= 1 ? 1.15 : 1);
+        else
+            c = r <= 1 ? 1.3 * (yc + 1.3) : r * (yc + 1.3) + 0.5 * yc + 1;
+        if (c < score - 1e-9) {
+            score = c;
+            best = yc;
+        }
+    }
+    return best;
 }
 
 // The streaming kernels address the fields of a pass from its first volume (consecutive
@@ -367,9 +449,39 @@ int finish_table(EfmInst *t, int n) {
     return tiles;
 }
 
-// Planes per streaming block: the chunk that fills whole waves of blocks best, for tiles of
-// EFM_STX x tz cells and `per_sm` resident blocks per SM.
-int choose_ychunk(const efm_ctx *ctx, int tz, int per_sm, int tx = EFM_STX) {
+// A streaming table: entries by falling step count, so that the instances still running at any
+// step are its first ones and the blocks share exactly their chunks.
+void finish_stream(efm_ctx *ctx, int slot, EfmInst *t, int n, int yc) {
+    std::stable_sort(t, t + n, [](const EfmInst &a, const EfmInst &b) { return a.nsteps > b.nsteps; });
+    for (int i = 0; i < n; ++i) {
+        t[i].ychunk = yc;
+        t[i].tiles_y = (t[i].yhi - t[i].ylo + yc - 1) / yc;
+    }
+    ctx->tiles[slot] = finish_table(t, n);
+    ctx->steps[slot].resize(n);
+    ctx->cum[slot].resize(n);
+    for (int i = 0; i < n; ++i) {
+        ctx->steps[slot][i] = t[i].nsteps;
+        ctx->cum[slot][i] = i + 1 < n ? t[i + 1].tile_begin : ctx->tiles[slot];
+    }
+}
+
+// Leading entries of a streaming table that run step `it`, and their chunks.
+struct Active {
+    int n, chunks;
+};
+
+Active active(const efm_ctx *ctx, int slot, int it) {
+    const std::vector<int> &st = ctx->steps[slot];
+    int n = 0;
+    while (n < (int)st.size() && st[n] > it) ++n;
+    return {n, n ? ctx->cum[slot][n - 1] : 0};
+}
+
+// Planes per block of the kernels that march one chunk per block (imaging, exact adjoint): the
+// chunk that fills whole waves of blocks best, for tiles of tx x tz cells and `per_sm` resident
+// blocks per SM.
+int choose_ychunk(const efm_ctx *ctx, int tz, int per_sm, int tx) {
     if (ctx->opt_ychunk > 0) return ctx->opt_ychunk;
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess)
@@ -406,7 +518,7 @@ void free_inst(Inst &I) {
     cudaFree(I.rec_lin);
     cudaFree(I.rec_id);
     cudaFree(I.rec_wfirst);
-    cudaFree(I.rec_tile);
+    cudaFree(I.rec_col);
     cudaFree(I.aux);
     cudaFree(I.fields);
     cudaFree(I.psi);
@@ -421,7 +533,7 @@ void free_inst(Inst &I) {
     I.cpml = nullptr;
     I.rec_mask = nullptr;
     I.rec_lin = I.rec_id = I.rec_wfirst = nullptr;
-    I.rec_tile = nullptr;
+    I.rec_col = nullptr;
     I.aux = nullptr;
     I.fields = I.psi = I.border = nullptr;
 }
@@ -462,8 +574,9 @@ int ensure_layout(efm_ctx *ctx) {
     EFM_CK(cudaMemcpy(ctx->d_seg, ctx->seg_host.data(), (n + 1) * sizeof(int64_t),
                       cudaMemcpyHostToDevice));
     if (ctx->d_err == nullptr) {
-        EFM_CK(cudaMalloc(&ctx->d_err, sizeof(unsigned int)));
-        EFM_CK(cudaMemset(ctx->d_err, 0, sizeof(unsigned int)));
+        EFM_CK(cudaMalloc(&ctx->d_err, 256));
+        EFM_CK(cudaMemset(ctx->d_err, 0, 256));
+        ctx->d_count = reinterpret_cast<int *>(ctx->d_err) + 32;  // a line of its own
     }
     if (ctx->maps_cap < n) {
         cudaFree(ctx->d_maps);
@@ -550,7 +663,8 @@ EfmInst base_table(const Inst &I) {
     d.tmap = nullptr;
     d.rmu = I.aux;
     d.buoy = I.aux + I.ncell;
-    d.rec_tile = I.rec_tile;
+    d.pitch = I.nx;
+    d.vol = I.ncell;
     d.nrec = I.nrec;
     d.rec_mask = I.rec_mask;
     d.rec_lin = I.rec_lin;
@@ -653,6 +767,84 @@ int ensure_exact(efm_ctx *ctx) {
     return EFM_OK;
 }
 
+// Tensor maps of a stress pass (12): vx, vy, vz, 1/mu with their neighbours, lambda and the six
+// stresses as cells, vy as cells (the plane before a chunk).
+int stress_maps(CUtensorMap *m, const Inst &I, const EfmInst &d, const float *const *v, const float *const *t) {
+    const int w = d.tw, h = d.th;
+    const float *f[12] = {v[0], v[1], v[2], I.aux, I.lam, t[0], t[1], t[2], t[3], t[4], t[5], v[1]};
+    for (int q = 0; q < 12; ++q)
+        if (const int rc = encode_map(m + q, f[q], I, q < 4 ? w + 4 : w, q < 4 ? h + 1 : h)) return rc;
+    return EFM_OK;
+}
+
+// ... and of a velocity pass (12): txx, tzz, txy, txz, tyz, 1/rho with the neighbours each needs,
+// tyy and the old velocities as cells, txy and tyz as cells (the plane before a chunk).
+int velocity_maps(CUtensorMap *m, const Inst &I, const EfmInst &d, const float *const *v, const float *const *t) {
+    const int w = d.tw, h = d.th;
+    const float *f[12] = {t[0], t[2], t[3], t[4], t[5], I.aux + I.ncell, t[1], v[0], v[1], v[2], t[3], t[5]};
+    const int bx[12] = {w + 4, w, w + 4, w + 4, w, w + 4, w, w, w, w, w, w};
+    const int bz[12] = {h, h + 1, h, h + 1, h + 1, h + 1, h, h, h, h, h, h};
+    for (int q = 0; q < 12; ++q)
+        if (const int rc = encode_map(m + q, f[q], I, bx[q], bz[q])) return rc;
+    return EFM_OK;
+}
+
+// ... of the imaging (12): the forward velocity before the rebuild step and 1/mu with their
+// neighbours, the rebuilt and the adjoint velocity and lambda as cells, vy as cells (the planes
+// before a chunk).
+int image_maps(CUtensorMap *m, const Inst &I, const EfmInst &d) {
+    const int w = d.tw, h = d.th;
+    const float *f[12] = {d.f.v[0], d.f.v[1], d.f.v[2], I.aux, d.f.vo[0], d.f.vo[1], d.f.vo[2],
+                          d.bv[0], d.bv[1], d.bv[2], I.lam, d.f.v[1]};
+    for (int q = 0; q < 12; ++q)
+        if (const int rc = encode_map(m + q, f[q], I, q < 4 ? w + 4 : w, q < 4 ? h + 1 + (q == 2) : h)) return rc;
+    return EFM_OK;
+}
+
+// Regions of the passes.  Stress and imaging: the updated cells [2, n-2).  Velocity: the same, or the whole
+// grid when a receiver lies outside them (it records zeros and takes the adjoint source).
+// Rebuild: the non-CPML box; its velocity over the whole grid in the first two steps, which
+// write the zeros outside the box into both ping-pong buffers.
+Region stress_region(const Inst &I) {
+    return {0, I.nx, EFM_HS, I.nz - EFM_HS, EFM_HS, I.ny - EFM_HS};
+}
+
+Region whole_grid(const Inst &I) { return {0, I.nx, 0, I.nz, 0, I.ny}; }
+
+Region velocity_region(const Inst &I) {
+    for (int r = 0; r < I.nrec; ++r) {
+        const int x = I.rec[3 * r], y = I.rec[3 * r + 1], z = I.rec[3 * r + 2];
+        if (x < EFM_HS || x >= I.nx - EFM_HS || y < EFM_HS || y >= I.ny - EFM_HS || z < EFM_HS ||
+            z >= I.nz - EFM_HS)
+            return whole_grid(I);
+    }
+    return stress_region(I);
+}
+
+Region box_region(const Inst &I) {
+    return {I.W / 4 * 4, I.nx - I.W, EFM_HS, I.nz - I.W, I.W, I.ny - I.W};
+}
+
+// Receiver map of the tiles of a velocity table entry, rebuilt when their shape changes.
+int ensure_rec_col(Inst &I, EfmInst &d, cudaStream_t s) {
+    const int shape[6] = {d.tw, d.th, d.ox, d.oz, d.tiles_x, d.tiles_z};
+    if (I.rec_col == nullptr || std::memcmp(shape, I.rec_shape, sizeof(shape)) != 0) {
+        std::vector<uint8_t> m((size_t)d.tiles_x * d.tiles_z * I.ny, 0);
+        for (int r = 0; r < I.nrec; ++r) {
+            const int tx = (I.rec[3 * r] - d.ox) / d.tw, tz = (I.rec[3 * r + 2] - d.oz) / d.th;
+            m[((size_t)tz * d.tiles_x + tx) * I.ny + I.rec[3 * r + 1]] = 1;
+        }
+        EFM_CK(cudaStreamSynchronize(s));  // launches in flight may still read the old map
+        cudaFree(I.rec_col);
+        I.rec_col = nullptr;
+        EFM_CK(cudaMalloc(&I.rec_col, m.size()));
+        EFM_CK(cudaMemcpy(I.rec_col, m.data(), m.size(), cudaMemcpyHostToDevice));
+        std::memcpy(I.rec_shape, shape, sizeof(shape));
+    }
+    d.rec_col = I.rec_col;
+    return EFM_OK;
+}
+
 // Forward tables (slots T_FWD_S, T_FWD_V) and tensor maps; gathers / strips optional.
 int prepare_forward(efm_ctx *ctx, float *gathers, bool strips, bool recips, cudaStream_t s,
                     bool *stream_kernels, float *illum = nullptr) {
@@ -662,9 +854,8 @@ int prepare_forward(efm_ctx *ctx, float *gathers, bool strips, bool recips, cuda
     if (st && (rc = get_encoder())) return rc;
     efm_stream_set_pdl(ctx->opt_pdl);
     const int rows = ctx->rows = ctx->opt_rows == 1 ? 1 : 2;
-    const int ring = ctx->ring = (rows == 1 && ctx->opt_ring == 6) ? 6 : 4;
-    const int tz = efm_st_tz(rows), hz = efm_st_hz(rows);
-    const int yc = st ? choose_ychunk(ctx, tz, efm_stream_blocks(rows, ring)) : 0;
+    ctx->ring = (rows == 1 && ctx->opt_ring == 6) ? 6 : 4;
+    const int nt = efm_st_nt(rows);
     std::vector<EfmInst> tab(2 * (size_t)n);
     std::vector<CUtensorMap> maps(st ? (size_t)n * EFM_MAPS_PER_INST : 0);
     for (int i = 0; i < n; ++i) {
@@ -673,8 +864,6 @@ int prepare_forward(efm_ctx *ctx, float *gathers, bool strips, bool recips, cuda
         if ((rc = zero_psi(I, s))) return rc;
         EfmInst d = base_table(I);
         d.nsteps = I.nt;
-        d.err = ctx->d_err;
-        d.wait_lim = ctx->opt_wait;
         for (int c = 0; c < 3; ++c) d.f.v[c] = d.f.vo[c] = I.va(c);
         for (int c = 0; c < 6; ++c) d.f.t[c] = I.tt(c);
         d.gather = gathers ? gathers + I.gather_off : nullptr;
@@ -682,21 +871,14 @@ int prepare_forward(efm_ctx *ctx, float *gathers, bool strips, bool recips, cuda
         d.border = strips ? I.border : nullptr;
         EfmInst ds = d, dv = d;
         if (st) {
-            layout_stream(ds, yc, tz);
-            layout_stream(dv, yc, tz);
+            layout_stream(ds, stress_region(I), nt);
+            layout_stream(dv, velocity_region(I), nt);
+            if ((rc = ensure_rec_col(I, dv, s))) return rc;
             CUtensorMap *m = maps.data() + (size_t)i * EFM_MAPS_PER_INST;
-            const float *sf[11] = {I.va(0), I.va(1), I.va(2), I.aux, I.lam, I.tt(0), I.tt(1),
-                                   I.tt(2), I.tt(3), I.tt(4), I.tt(5)};
-            for (int q = 0; q < 11; ++q)
-                if ((rc = encode_map(m + M_FWD_S + q, sf[q], I, q < 4 ? EFM_HX : EFM_STX,
-                                     q < 4 ? hz : tz)))
-                    return rc;
-            const float *vf[10] = {I.tt(0), I.tt(2), I.tt(3), I.tt(4), I.tt(5), I.aux + I.ncell,
-                                   I.tt(1), I.va(0), I.va(1), I.va(2)};
-            for (int q = 0; q < 10; ++q)
-                if ((rc = encode_map(m + M_FWD_V + q, vf[q], I, q < 6 ? EFM_HX : EFM_STX,
-                                     q < 6 ? hz : tz)))
-                    return rc;
+            const float *v[3] = {I.va(0), I.va(1), I.va(2)};
+            const float *t[6] = {I.tt(0), I.tt(1), I.tt(2), I.tt(3), I.tt(4), I.tt(5)};
+            if ((rc = stress_maps(m + M_FWD_S, I, ds, v, t)) || (rc = velocity_maps(m + M_FWD_V, I, dv, v, t)))
+                return rc;
             ds.tmap = ctx->d_maps + (size_t)i * EFM_MAPS_PER_INST + M_FWD_S;
             dv.tmap = ctx->d_maps + (size_t)i * EFM_MAPS_PER_INST + M_FWD_V;
         } else {
@@ -709,13 +891,20 @@ int prepare_forward(efm_ctx *ctx, float *gathers, bool strips, bool recips, cuda
     if (st)
         for (const EfmInst &e : tab)
             if (!fields_contiguous(e)) return fail(EFM_ERR_STATE, "field volumes not contiguous");
-    ctx->tiles[T_FWD_S] = finish_table(tab.data(), n);
-    ctx->tiles[T_FWD_V] = finish_table(tab.data() + n, n);
+    if (st) {
+        const int slots = efm_stream_slots(rows, ctx->ring);
+        finish_stream(ctx, T_FWD_S, tab.data(), n, chunk_planes(ctx, {tab.data()}, n, slots));
+        finish_stream(ctx, T_FWD_V, tab.data() + n, n, chunk_planes(ctx, {tab.data() + n}, n, slots));
+    } else {
+        ctx->tiles[T_FWD_S] = finish_table(tab.data(), n);
+        ctx->tiles[T_FWD_V] = finish_table(tab.data() + n, n);
+    }
     if (st)
         EFM_CK(cudaMemcpyAsync(ctx->d_maps, maps.data(), maps.size() * sizeof(CUtensorMap),
                                cudaMemcpyHostToDevice, s));
     EFM_CK(cudaMemcpyAsync(ctx->d_tab, tab.data(), tab.size() * sizeof(EfmInst),
                            cudaMemcpyHostToDevice, s));
+    EFM_CK(cudaMemsetAsync(ctx->d_count, 0, sizeof(int), s));
     if (st && recips)
         for (const Inst &I : ctx->inst)
             if ((rc = timed_launch(ctx, EFM_K_MODEL_AUX, s, [&] {
@@ -726,18 +915,39 @@ int prepare_forward(efm_ctx *ctx, float *gathers, bool strips, bool recips, cuda
     return EFM_OK;
 }
 
+// One streaming launch at step `it`: stress pass ps of table `ss` and / or velocity pass pv of
+// table `sv` (-1: none).
+cudaError_t launch_stream(const efm_ctx *ctx, int ps, int ss, int pv, int sv, bool illum, int it, cudaStream_t s) {
+    const Active a = ps >= 0 ? active(ctx, ss, it) : Active{0, 0}, b = pv >= 0 ? active(ctx, sv, it) : Active{0, 0};
+    if (a.chunks + b.chunks == 0) return cudaSuccess;
+    const size_t n = ctx->inst.size();
+    return efm_launch_stream(ps, pv, illum, ctx->rows, ctx->ring, ctx->d_tab + (ps >= 0 ? ss : 0) * n, a.n, a.chunks,
+                             ctx->d_tab + (pv >= 0 ? sv : 0) * n, b.n, b.chunks,
+                             std::min(a.chunks + b.chunks, efm_stream_slots(ctx->rows, ctx->ring)), it, ctx->d_count,
+                             ctx->opt_wait, ctx->d_err, s);
+}
+
+// The rebuild velocity's table at step `it`.
+int rev_v_slot(int it) { return it < 2 ? (it & 1 ? T_REV_VF1 : T_REV_VF0) : (it & 1 ? T_REV_V1 : T_REV_V0); }
+
+// The paired launches of an imaging-gradient step (0: adjoint stress | rebuild velocity, 1: rebuild
+// stress | adjoint velocity).
+cudaError_t launch_pair(const efm_ctx *ctx, int which, int it, cudaStream_t s) {
+    return which == 0 ? launch_stream(ctx, EFM_ADJ, T_ADJ_S, EFM_REV, rev_v_slot(it), false, it, s)
+                      : launch_stream(ctx, EFM_REV, it & 1 ? T_REV_S1 : T_REV_S0, EFM_ADJ, T_ADJ_V, false, it, s);
+}
+
 int forward_step(efm_ctx *ctx, bool st, int it, cudaStream_t s, bool illum = false) {
     const int n = (int)ctx->inst.size();
     const EfmInst *ts = ctx->d_tab, *tv = ctx->d_tab + n;
     int rc;
     if ((rc = timed_launch(ctx, EFM_K_FWD_STRESS, s, [&] {
-             return st ? efm_launch_stream(EFM_FWD, 0, ctx->rows, ctx->ring, ts, n, ctx->tiles[T_FWD_S], it, s)
+             return st ? launch_stream(ctx, EFM_FWD, T_FWD_S, -1, 0, false, it, s)
                        : efm_launch_stress(EFM_FWD, ts, n, ctx->tiles[T_FWD_S], it, s);
          })))
         return rc;
     return timed_launch(ctx, EFM_K_FWD_VELOCITY, s, [&] {
-        return st ? efm_launch_stream(EFM_FWD, illum ? 2 : 1, ctx->rows, ctx->ring, tv, n,
-                                      ctx->tiles[T_FWD_V], it, s)
+        return st ? launch_stream(ctx, -1, 0, EFM_FWD, T_FWD_V, illum, it, s)
                   : efm_launch_velocity(EFM_FWD, tv, n, ctx->tiles[T_FWD_V], it, s);
     });
 }
@@ -921,31 +1131,24 @@ int gradient_loop(efm_ctx *ctx, bool st, bool model, int n, int maxsteps, cudaSt
             // within a step the adjoint chain and the rebuild write disjoint fields, and the
             // imaging reads neither the rebuild's stress nor anything the next step's first
             // pair writes before this step's imaging has finished (stream order)
-            const int kv = (it & 1) ? T_REV_V1 : T_REV_V0, ks = (it & 1) ? T_REV_S1 : T_REV_S0;
             const int ki = (it & 1) ? T_IMG1 : T_IMG0;
-            if ((rc = timed_launch(ctx, EFM_K_PAIR_ADJS_REVV, s, [&] {
-                     return efm_launch_pair(0, ctx->rows, ctx->ring, dtab(T_ADJ_S), ctx->tiles[T_ADJ_S],
-                                            dtab(kv), ctx->tiles[kv], n, it, s);
-                 })))
+            if ((rc = timed_launch(ctx, EFM_K_PAIR_ADJS_REVV, s, [&] { return launch_pair(ctx, 0, it, s); })))
                 return rc;
-            if ((rc = timed_launch(ctx, EFM_K_PAIR_REVS_ADJV, s, [&] {
-                     return efm_launch_pair(1, ctx->rows, ctx->ring, dtab(ks), ctx->tiles[ks],
-                                            dtab(T_ADJ_V), ctx->tiles[T_ADJ_V], n, it, s);
-                 })))
+            if ((rc = timed_launch(ctx, EFM_K_PAIR_REVS_ADJV, s, [&] { return launch_pair(ctx, 1, it, s); })))
                 return rc;
             if ((rc = timed_launch(ctx, EFM_K_IMAGING, s, [&] {
-                     return efm_launch_image(dtab(ki), n, ctx->tiles[ki], it, s);
+                     return launch_stream(ctx, -1, 0, EFM_IMG, ki, false, it, s);
                  })))
                 return rc;
             continue;
         }
         if ((rc = timed_launch(ctx, EFM_K_ADJ_STRESS, s, [&] {
-                 return st ? efm_launch_stream(EFM_ADJ, 0, ctx->rows, ctx->ring, dtab(T_ADJ_S), n, ctx->tiles[T_ADJ_S], it, s)
+                 return st ? launch_stream(ctx, EFM_ADJ, T_ADJ_S, -1, 0, false, it, s)
                            : efm_launch_stress(EFM_ADJ, dtab(T_ADJ_S), n, ctx->tiles[T_ADJ_S], it, s);
              })))
             return rc;
         if ((rc = timed_launch(ctx, EFM_K_ADJ_VELOCITY, s, [&] {
-                 return st ? efm_launch_stream(EFM_ADJ, 1, ctx->rows, ctx->ring, dtab(T_ADJ_V), n, ctx->tiles[T_ADJ_V], it, s)
+                 return st ? launch_stream(ctx, -1, 0, EFM_ADJ, T_ADJ_V, false, it, s)
                            : efm_launch_velocity(EFM_ADJ, dtab(T_ADJ_V), n, ctx->tiles[T_ADJ_V], it, s);
              })))
             return rc;
@@ -954,16 +1157,16 @@ int gradient_loop(efm_ctx *ctx, bool st, bool model, int n, int maxsteps, cudaSt
             const int ki = (it & 1) ? T_IMG1 : T_IMG0;
             // stream kernels: rebuild, then imaging; otherwise one fused rebuild + imaging kernel
             if ((rc = timed_launch(ctx, EFM_K_REV_VELOCITY, s, [&] {
-                     return st ? efm_launch_stream(EFM_REV, 1, ctx->rows, ctx->ring, dtab(kv), n, ctx->tiles[kv], it, s)
+                     return st ? launch_stream(ctx, -1, 0, EFM_REV, rev_v_slot(it), false, it, s)
                                : efm_launch_velocity(EFM_REV, dtab(kv), n, ctx->tiles[kv], it, s);
                  })))
                 return rc;
             if (st && (rc = timed_launch(ctx, EFM_K_IMAGING, s, [&] {
-                           return efm_launch_image(dtab(ki), n, ctx->tiles[ki], it, s);
+                           return launch_stream(ctx, -1, 0, EFM_IMG, ki, false, it, s);
                        })))
                 return rc;
             if ((rc = timed_launch(ctx, EFM_K_REV_STRESS, s, [&] {
-                     return st ? efm_launch_stream(EFM_REV, 0, ctx->rows, ctx->ring, dtab(ks), n, ctx->tiles[ks], it, s)
+                     return st ? launch_stream(ctx, EFM_REV, ks, -1, 0, false, it, s)
                                : efm_launch_stress(EFM_REV, dtab(ks), n, ctx->tiles[ks], it, s);
                  })))
                 return rc;
@@ -1117,16 +1320,6 @@ int efm_add_instance(efm_ctx *ctx, const efm_instance_desc *d, int *id) {
     if ((e = cudaMemcpy(I.rec_id, rid.data(), I.nrec * sizeof(int), cudaMemcpyHostToDevice))) return bad(e);
     if ((e = cudaMemcpy(I.rec_wfirst, wfirst.data(), wfirst.size() * sizeof(int), cudaMemcpyHostToDevice)))
         return bad(e);
-    {
-        const int tx = (I.nx + EFM_STX - 1) / EFM_STX, tz = (I.nz + EFM_REC_TZ - 1) / EFM_REC_TZ;
-        std::vector<uint8_t> rt((size_t)I.ny * tz * tx, 0);
-        for (int r = 0; r < I.nrec; ++r) {
-            const int x = I.rec[3 * r], y = I.rec[3 * r + 1], z = I.rec[3 * r + 2];
-            rt[((size_t)y * tz + z / EFM_REC_TZ) * tx + x / EFM_STX] = 1;
-        }
-        if ((e = cudaMalloc(&I.rec_tile, rt.size()))) return bad(e);
-        if ((e = cudaMemcpy(I.rec_tile, rt.data(), rt.size(), cudaMemcpyHostToDevice))) return bad(e);
-    }
     ctx->inst.push_back(std::move(I));
     ctx->ck_auto = 0;  // the automatic checkpoint interval is chosen for the new instance set
     ctx->layout_ready = false;
@@ -1201,9 +1394,10 @@ int efm_forward_illumination(efm_ctx *ctx, float *gathers, int save, float *illu
         I.fwd_saved = false;
         I.ck_saved = false;
     }
-    std::vector<int64_t> key = {st, ctx->rows, ctx->ring, ctx->opt_pdl, (int64_t)ctx->inst.size(),
+    std::vector<int64_t> key = {st, ctx->rows, ctx->ring, ctx->opt_pdl, ctx->opt_wait, (int64_t)ctx->inst.size(),
                                 maxnt, (int64_t)(uintptr_t)ctx->d_tab, ctx->tiles[T_FWD_S],
                                 ctx->tiles[T_FWD_V], ckpts, illum != nullptr};
+    add_table_key(ctx, T_FWD_S, T_FWD_V, key);
     if (ckpts)
         for (const Inst &I : ctx->inst)
             key.insert(key.end(), {I.ck_every, I.nt, (int64_t)(uintptr_t)I.ckpt,
@@ -1280,10 +1474,8 @@ int efm_gradient(efm_ctx *ctx, const float *res, float *grad, double *mtg, int f
     if (st && (rc = get_encoder())) return rc;
     efm_stream_set_pdl(ctx->opt_pdl);
     const int rows = ctx->rows = ctx->opt_rows == 1 ? 1 : 2;
-    const int ring = ctx->ring = (rows == 1 && ctx->opt_ring == 6) ? 6 : 4;
-    const int tz = efm_st_tz(rows), hz = efm_st_hz(rows);
-    const int yc = st ? choose_ychunk(ctx, tz, efm_stream_blocks(rows, ring)) : 0;
-    const int yci = st ? choose_ychunk(ctx, EFM_IMG_TZ, 3) : 0;
+    ctx->ring = (rows == 1 && ctx->opt_ring == 6) ? 6 : 4;
+    const int nt = efm_st_nt(rows);
     std::vector<EfmInst> tab((size_t)T_NSLOT * n);
     std::vector<CUtensorMap> maps(st ? (size_t)n * EFM_MAPS_PER_INST : 0);
     auto slot = [&](int k, int i) -> EfmInst & { return tab[(size_t)k * n + i]; };
@@ -1301,28 +1493,19 @@ int efm_gradient(efm_ctx *ctx, const float *res, float *grad, double *mtg, int f
         // adjoint propagation
         EfmInst a = base_table(I);
         a.nsteps = steps;
-        a.err = ctx->d_err;
-        a.wait_lim = ctx->opt_wait;
         for (int c = 0; c < 3; ++c) a.f.v[c] = a.f.vo[c] = I.bv(c);
         for (int c = 0; c < 6; ++c) a.f.t[c] = I.bt(c);
         a.res = res + I.gather_off;
         a.mtg = mt ? mtg + (size_t)i * EFM_NSRC * 6 : nullptr;
         EfmInst as = a, av = a;
         if (st) {
-            layout_stream(as, yc, tz);
-            layout_stream(av, yc, tz);
-            const float *sf[11] = {I.bv(0), I.bv(1), I.bv(2), I.aux, I.lam, I.bt(0), I.bt(1),
-                                   I.bt(2), I.bt(3), I.bt(4), I.bt(5)};
-            for (int q = 0; q < 11; ++q)
-                if ((rc = encode_map(m + M_ADJ_S + q, sf[q], I, q < 4 ? EFM_HX : EFM_STX,
-                                     q < 4 ? hz : tz)))
-                    return rc;
-            const float *vf[10] = {I.bt(0), I.bt(2), I.bt(3), I.bt(4), I.bt(5), I.aux + I.ncell,
-                                   I.bt(1), I.bv(0), I.bv(1), I.bv(2)};
-            for (int q = 0; q < 10; ++q)
-                if ((rc = encode_map(m + M_ADJ_V + q, vf[q], I, q < 6 ? EFM_HX : EFM_STX,
-                                     q < 6 ? hz : tz)))
-                    return rc;
+            layout_stream(as, stress_region(I), nt);
+            layout_stream(av, velocity_region(I), nt);
+            if ((rc = ensure_rec_col(I, av, s))) return rc;
+            const float *v[3] = {I.bv(0), I.bv(1), I.bv(2)};
+            const float *t[6] = {I.bt(0), I.bt(1), I.bt(2), I.bt(3), I.bt(4), I.bt(5)};
+            if ((rc = stress_maps(m + M_ADJ_S, I, as, v, t)) || (rc = velocity_maps(m + M_ADJ_V, I, av, v, t)))
+                return rc;
             as.tmap = dm + M_ADJ_S;
             av.tmap = dm + M_ADJ_V;
         } else {
@@ -1335,8 +1518,6 @@ int efm_gradient(efm_ctx *ctx, const float *res, float *grad, double *mtg, int f
         for (int p = 0; p < 2; ++p) {
             EfmInst r = base_table(I);
             r.nsteps = I.nt - 1;
-            r.err = ctx->d_err;
-            r.wait_lim = ctx->opt_wait;
             r.k = -r.k;
             for (int c = 0; c < 3; ++c) {
                 r.f.v[c] = p == 0 ? I.va(c) : I.vb(c);
@@ -1353,72 +1534,73 @@ int efm_gradient(efm_ctx *ctx, const float *res, float *grad, double *mtg, int f
                 r.g_mu = grad + I.grad_off + I.ncell;
                 r.g_rho = grad + I.grad_off + 2 * I.ncell;
             }
-            EfmInst rv = r, rs = r, ri = r;
+            EfmInst rv = r, rs = r, ri = r, rf = r;
             if (st) {
-                layout_stream(rs, yc, tz);
-                const int mb = p == 0 ? M_REV_S0 : M_REV_S1;
-                const float *sf[11] = {r.f.vo[0], r.f.vo[1], r.f.vo[2], I.aux, I.lam, I.tt(0),
-                                       I.tt(1), I.tt(2), I.tt(3), I.tt(4), I.tt(5)};
-                for (int q = 0; q < 11; ++q)
-                    if ((rc = encode_map(m + mb + q, sf[q], I, q < 4 ? EFM_HX : EFM_STX,
-                                         q < 4 ? hz : tz)))
-                        return rc;
-                rs.tmap = dm + mb;
-                // reverse velocity rebuild: the velocity pass's fields, old velocity in f.v
-                layout_stream(rv, yc, tz);
-                const int mv = p == 0 ? M_REV_V0 : M_REV_V1;
-                const float *vf[13] = {I.tt(0), I.tt(2), I.tt(3), I.tt(4), I.tt(5), I.aux + I.ncell,
-                                       I.tt(1), r.f.v[0], r.f.v[1], r.f.v[2], r.f.vo[0], r.f.vo[1],
-                                       r.f.vo[2]};
-                for (int q = 0; q < 13; ++q)
-                    if ((rc = encode_map(m + mv + q, vf[q], I, q < 6 ? EFM_HX : EFM_STX,
-                                         q < 6 ? hz : tz)))
-                        return rc;
-                rv.tmap = dm + mv;
-                // imaging: halo fV_present + 1/mu (72 x 7 from z0-2), cells 64 x 4
+                const Region box = box_region(I);
+                layout_stream(rs, box, nt);
+                layout_stream(rv, box, nt);
+                const int shape[2] = {rv.tw, rv.th};
+                layout_stream(rf, whole_grid(I), nt, shape);
+                const float *t[6] = {I.tt(0), I.tt(1), I.tt(2), I.tt(3), I.tt(4), I.tt(5)};
+                const int ms = p == 0 ? M_REV_S0 : M_REV_S1, mv = p == 0 ? M_REV_V0 : M_REV_V1;
+                if ((rc = stress_maps(m + ms, I, rs, r.f.vo, t)) || (rc = velocity_maps(m + mv, I, rv, r.f.v, t)))
+                    return rc;
+                rs.tmap = dm + ms;
+                rv.tmap = rf.tmap = dm + mv;
                 if (model) {
-                    layout_stream(ri, yci, EFM_IMG_TZ);
+                    layout_stream(ri, stress_region(I), nt);
+                    ri.gvec = I.nx % 2 == 0 && ((uintptr_t)r.g_lam | (uintptr_t)r.g_mu | (uintptr_t)r.g_rho) % 8 == 0;
                     const int mi = p == 0 ? M_IMG0 : M_IMG1;
-                    const float *hf[4] = {r.f.v[0], r.f.v[1], r.f.v[2], I.aux};
-                    for (int q = 0; q < 4; ++q)
-                        if ((rc = encode_map(m + mi + q, hf[q], I, EFM_HX, EFM_IMG_TZ + 3))) return rc;
-                    const float *cf[16] = {r.f.vo[0], r.f.vo[1], r.f.vo[2], I.bv(0), I.bv(1), I.bv(2),
-                                           I.bt(0), I.bt(1), I.bt(2), I.bt(3), I.bt(4), I.bt(5),
-                                           I.lam, r.g_lam, r.g_mu, r.g_rho};
-                    for (int q = 0; q < 16; ++q)
-                        if ((rc = encode_map(m + mi + 4 + q, cf[q], I, EFM_STX, EFM_IMG_TZ))) return rc;
+                    if ((rc = image_maps(m + mi, I, ri))) return rc;
                     ri.tmap = dm + mi;
-                } else {
-                    layout_stream(ri, yci, EFM_IMG_TZ);
                 }
             } else {
                 layout_naive(rs);
                 layout_naive(rv);
                 layout_naive(ri);
+                layout_naive(rf);
             }
             slot(p == 0 ? T_REV_V0 : T_REV_V1, i) = rv;
             slot(p == 0 ? T_REV_S0 : T_REV_S1, i) = rs;
             slot(p == 0 ? T_IMG0 : T_IMG1, i) = ri;
+            slot(p == 0 ? T_REV_VF0 : T_REV_VF1, i) = rf;
         }
     }
     if (st)
         for (const EfmInst &e : tab)
             if (!fields_contiguous(e)) return fail(EFM_ERR_STATE, "field volumes not contiguous");
-    for (int k = T_ADJ_S; k < T_NSLOT; ++k) ctx->tiles[k] = finish_table(&slot(k, 0), n);
+    if (st) {
+        // the pairs' tables share a launch's rounds (unpaired launches use the same chunks)
+        const int slots = efm_stream_slots(rows, ctx->ring);
+        for (int q = 0; q < 2; ++q) {
+            EfmInst *a = &slot(q ? T_ADJ_V : T_ADJ_S, 0), *r = &slot(q ? T_REV_S0 : T_REV_V0, 0);
+            const int yc = model ? chunk_planes(ctx, {a, r}, n, slots) : chunk_planes(ctx, {a}, n, slots);
+            finish_stream(ctx, q ? T_ADJ_V : T_ADJ_S, a, n, yc);
+            if (!model) continue;
+            for (int k : {T_REV_S0, T_REV_S1, T_REV_V0, T_REV_V1, T_REV_VF0, T_REV_VF1})
+                if ((k == T_REV_S0 || k == T_REV_S1) == (q == 1)) finish_stream(ctx, k, &slot(k, 0), n, yc);
+        }
+        if (model)
+            for (int k : {T_IMG0, T_IMG1})
+                finish_stream(ctx, k, &slot(k, 0), n, chunk_planes(ctx, {&slot(k, 0)}, n, slots));
+    }
+    for (int k = T_ADJ_S; k < T_NSLOT; ++k)
+        if (!st) ctx->tiles[k] = finish_table(&slot(k, 0), n);
     if (st)
         EFM_CK(cudaMemcpyAsync(ctx->d_maps, maps.data(), maps.size() * sizeof(CUtensorMap),
                                cudaMemcpyHostToDevice, s));
     EFM_CK(cudaMemcpyAsync(ctx->d_tab, tab.data(), tab.size() * sizeof(EfmInst),
                            cudaMemcpyHostToDevice, s));
+    EFM_CK(cudaMemsetAsync(ctx->d_count, 0, sizeof(int), s));
     if (st)
         for (const Inst &I : ctx->inst)
             if ((rc = timed_launch(ctx, EFM_K_MODEL_AUX, s, [&] {
                      return efm_launch_reciprocals(I.mu, I.rho, I.aux, I.aux + I.ncell, I.ncell, s);
                  })))
                 return rc;
-    std::vector<int64_t> key = {st, model, ctx->opt_pair, ctx->rows, ctx->ring, ctx->opt_pdl, n,
+    std::vector<int64_t> key = {st, model, ctx->opt_pair, ctx->rows, ctx->ring, ctx->opt_pdl, ctx->opt_wait, n,
                                 maxsteps, (int64_t)(uintptr_t)ctx->d_tab};
-    key.insert(key.end(), ctx->tiles + T_ADJ_S, ctx->tiles + T_NSLOT);
+    add_table_key(ctx, T_ADJ_S, T_NSLOT - 1, key);
     rc = run_loop(ctx, 1, key, s, [&](cudaStream_t ls) { return gradient_loop(ctx, st, model, n, maxsteps, ls); });
     if (rc) return rc;
     if (model)
@@ -1442,8 +1624,6 @@ int efm_kernel_time(efm_ctx *ctx, int kind, int reps, int it, double *ms_per_lau
     if (it < 0 || it + 1 >= ctx->time_steps)
         return fail(EFM_ERR_ARG, "step index must satisfy 0 <= it and it + 1 < the tables' steps");
     cudaStream_t s = (cudaStream_t)stream;
-    const int n = (int)ctx->inst.size();
-    auto dtab = [&](int k) { return (const EfmInst *)(ctx->d_tab + (size_t)k * n); };
     efm_stream_set_pdl(ctx->opt_pdl);
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     EFM_CK(cudaEventCreate(&e0));
@@ -1454,26 +1634,13 @@ int efm_kernel_time(efm_ctx *ctx, int kind, int reps, int it, double *ms_per_lau
     cudaError_t e = cudaEventRecord(e0, s);
     for (int r = 0; r < reps && e == cudaSuccess; ++r) {
         const int i = it + (r & 1);  // alternate two steps, as the ping-pong tables do
-        const int kv = (i & 1) ? T_REV_V1 : T_REV_V0, ks = (i & 1) ? T_REV_S1 : T_REV_S0;
         const int ki = (i & 1) ? T_IMG1 : T_IMG0;
         switch (kind) {
-            case EFM_K_FWD_STRESS:
-                e = efm_launch_stream(EFM_FWD, 0, ctx->rows, ctx->ring, dtab(T_FWD_S), n,
-                                      ctx->tiles[T_FWD_S], i, s);
-                break;
-            case EFM_K_FWD_VELOCITY:
-                e = efm_launch_stream(EFM_FWD, 1, ctx->rows, ctx->ring, dtab(T_FWD_V), n,
-                                      ctx->tiles[T_FWD_V], i, s);
-                break;
-            case EFM_K_PAIR_ADJS_REVV:
-                e = efm_launch_pair(0, ctx->rows, ctx->ring, dtab(T_ADJ_S), ctx->tiles[T_ADJ_S],
-                                    dtab(kv), ctx->tiles[kv], n, i, s);
-                break;
-            case EFM_K_PAIR_REVS_ADJV:
-                e = efm_launch_pair(1, ctx->rows, ctx->ring, dtab(ks), ctx->tiles[ks],
-                                    dtab(T_ADJ_V), ctx->tiles[T_ADJ_V], n, i, s);
-                break;
-            default: e = efm_launch_image(dtab(ki), n, ctx->tiles[ki], i, s); break;
+            case EFM_K_FWD_STRESS: e = launch_stream(ctx, EFM_FWD, T_FWD_S, -1, 0, false, i, s); break;
+            case EFM_K_FWD_VELOCITY: e = launch_stream(ctx, -1, 0, EFM_FWD, T_FWD_V, false, i, s); break;
+            case EFM_K_PAIR_ADJS_REVV: e = launch_pair(ctx, 0, i, s); break;
+            case EFM_K_PAIR_REVS_ADJV: e = launch_pair(ctx, 1, i, s); break;
+            default: e = launch_stream(ctx, -1, 0, EFM_IMG, ki, false, i, s); break;
         }
     }
     if (e == cudaSuccess) e = cudaEventRecord(e1, s);

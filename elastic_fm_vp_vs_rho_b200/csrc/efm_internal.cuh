@@ -34,7 +34,7 @@ struct EfmInst {
     int nx, ny, nz, W;
     int tiles_x, tiles_z, tiles_y;  // tile grid of the kernel family this table is built for
     int tile_begin;
-    int ychunk;        // planes per block of the plane-streaming kernels
+    int ychunk;        // planes per chunk of the plane-streaming kernels
     int nsteps;        // iterations this instance performs in the current pass
     int nt;            // record length
     float k;           // dt/dx of this pass (negative for the reverse rebuild)
@@ -69,14 +69,21 @@ struct EfmInst {
     const float *bv[3];
     const float *bt[6];
     float *g_lam, *g_mu, *g_rho;
-    // plane-streaming kernels: this pass's tensor maps, the context's error word, 1/mu and
-    // 1/rho, and a byte per (plane, tile) telling whether the tile holds a receiver
+    // plane-streaming kernels: this pass's tensor maps, 1/mu and 1/rho, and a byte per (tile,
+    // plane) telling whether the tile holds a receiver there
     const CUtensorMap *tmap;
-    unsigned int *err;
-    unsigned int wait_lim;  // polls per tile wait (0: the default bound; efm_mbar_wait)
     const float *rmu, *buoy;
-    const uint8_t *rec_tile;
+    const uint8_t *rec_col;
+    int tw, th;            // tile (x, z), the first tile's corner and the planes covered
+    int ox, oz, ylo, yhi;
+    int pitch;             // floats from one row of an internal volume to the next (nx)
+    bool gvec;             // pairs of gradient cells start on 8 bytes
+    int64_t vol;           // floats from one internal volume to the next
 };
+// The streaming kernels copy table entries in 16-byte pieces.  (Not alignas(16): the compiler then
+// pairs the other kernels' pointer loads, and the thread-per-cell rebuild takes 52 registers and
+// 5% more time instead of 48.)
+static_assert(sizeof(EfmInst) % 16 == 0, "pad EfmInst to 16 bytes");
 
 __device__ __forceinline__ int efm_find_inst(const EfmInst *__restrict__ insts, int n, int b) {
     int lo = 0, hi = n - 1;

@@ -1,32 +1,51 @@
-// Plane-streaming stress / velocity kernels: TMA-fed shared-memory rings.
+// Plane-streaming stress / velocity / imaging kernels: a TMA producer warp feeding shared-memory rings.
 //
-// Each block owns a 64 x TZ (x, z) column of the grid (TZ = 4 * ROWS) and marches along y
-// over a chunk of planes.  One thread issues, per plane, a TMA tile load of every field the
-// half-step reads into one stage of a 4-deep ring (x/z-neighbour fields with a halo box
-// 72 x (TZ + 2) starting at (x0-4, z0-1); cell-only fields with a 64 x TZ box).  While the
-// block computes plane j from the stages of planes j-1, j, j+1, plane j+2 is in flight, so
-// the resident blocks keep ~100 KB per SM in flight without spending registers.  Each
-// thread computes the cells (x, z0 + r + 4h), h < ROWS, of every plane.
+// A block takes chunks -- a tile of tw x th (x, z) cells over a run of y planes -- from the
+// launch's counter.  Its producer warp issues, per plane, a TMA tile load of every field the
+// half-step reads: fields whose x / y / z neighbours enter (boxes with just the neighbour columns
+// / rows that are used) and cell-only fields.  Slot q of the ring holds the neighbour fields of
+// plane p + 1 and the cell fields of plane p, so computing plane p needs slot q and the neighbour
+// part of slot q - 1; what the stencil reads of plane p - 1 is this thread's own column and stays
+// in registers.  A ring of D + 1 slots keeps D - 1 planes in flight while one is computed, and
+// the loads of the next chunk follow the last plane of the current one without a gap.  A chunk's
+// first slot brings the neighbour fields of its first plane and, in the unused cell part, the
+// own-column values of the plane before.
 //
-// Per plane the compute touches no global memory it has to wait for except the compact
-// CPML memory variables of PML cells, which are requested before the stage wait.  Sources
-// and receivers are located once per block (a flag, and a bit per plane from a per-tile map
-// built on the host), reciprocals of mu and rho come precomputed, and one block barrier
-// per plane both frees the oldest stage and makes a timed-out wait end every thread's loop.
+// Each consumer thread computes a pair of x-neighbours: operands come as 8-byte shared-memory
+// loads (the x neighbour inside the pair is already in a register), results go straight to global
+// memory as 8-byte stores, so the slot is free as soon as it has been read, and addresses, tests
+// and waits are shared by two cells.  Consumer warps never wait for one another: each waits for
+// the plane's full barrier and arrives on its empty barrier.  Before, one thread computed two
+// separate cells of a 64 x 8 tile with a block barrier per plane, 4-byte loads and TMA stores out
+// of the ring.  The imaging runs the same way: as a kernel of its own with another amount of shared
+// memory it also left the next stress launch, which starts while it drains, with its smaller L1
+// (256 x 256 x 128 gradient step: 491 us, 465 now).
 //
-// Each thread writes its new values over the old ones in the plane's stage (cell fields are
-// read only by their own thread); after the barrier one thread stores the plane's updated
-// fields with TMA tile stores (one bulk group per plane) and refills the oldest stage once
-// the store out of it has been read.  The per-cell work is then shared-memory loads, the
-// arithmetic and shared-memory stores; global addresses are formed only for the CPML memory
-// variables (offsets hoisted per thread row, plane bases per plane), receivers and strips.
+// us per launch, before and now: 128 x 128 x 96 forward stress 23.4, 22.5, velocity 24.6, 24.9;
+// 256 x 256 x 128: 114.6, 103.4 and 115.5, 94.2 (the DRAM rate: a pass moves 15 volumes and the
+// memory variables), adjoint stress + rebuild velocity 193.7, 168.9, rebuild stress + adjoint
+// velocity 190.2, 171.7, imaging 127.1, 119.2; 64 x 64 x 64 forward 10.1, 7.0 and 12.0, 8.2
+// (launch and first loads).  Small grids are bound by issue and latency: about 260 instructions
+// per warp and plane of pairs without memory variables, 16 warps per SM.
 //
+// Sources are looked up once per chunk, receivers per plane from a map built on the host.
 // Arithmetic, guards, CPML, sources, receivers, strips and MT strain follow efm_stencil.cu
-// (kernel_Tau :59-128, kernel_Vx_Vy_Vz :133-188 of mainPropElastic3D_MT.py); harmonic means
+// (kernel_Tau :59-128, kernel_Vx_Vy_Vz :133-188, kernel_Gradients_* :191-294 of
+// mainPropElastic3D_MT.py); harmonic means
 // use the hardware reciprocal (relative error ~1 ulp).
 #include "efm_internal.cuh"
 #include "efm_stream.cuh"
 #include "efm_tma.cuh"
+
+// A launch: the chunks of a stress pass (table s), then of a velocity or imaging pass (table v).
+struct EfmStream {
+    const EfmInst *s, *v;
+    int ns, nv, cs, cv;  // table entries still active, and their chunks
+    int it;
+    int *counter;
+    uint32_t lim;
+    unsigned int *err;
+};
 
 namespace {
 
@@ -36,845 +55,1268 @@ __device__ __forceinline__ float frcp(float a) {
     return r;
 }
 
-// Compile-time flag for the two instantiations of a plane's update (with / without the CPML
-// memory-variable code); a warp picks one per plane with a warp-uniform test.
-template <bool B>
+// a x + b y, rounded as fma(b, y, a x): written out where a compiler is free to fuse either product,
+// so that every instantiation of a plane's update rounds alike.
+__device__ __forceinline__ float two_products(float a, float x, float b, float y) {
+    return __fmaf_rn(b, y, __fmul_rn(a, x));
+}
+
+// The instantiations of a plane's update, picked per plane by a warp-uniform test: no memory
+// variables (0), those of the x slabs (1: every plane of the tiles at the x faces), every family
+// and, in the velocity, receivers (2: few planes, and the registers of all three families).
+template <int V>
 struct Tag {
-    static constexpr bool value = B;
+    static constexpr int value = V;
 };
 
-template <int ROWS, int SR>
-struct Ring {
-    static constexpr int HB = efm_halo_bytes(ROWS), CB = efm_center_bytes(ROWS);
-    static constexpr int CF = CB / 4;  // floats per cell field
-    unsigned char *base;
-    uint64_t *bar;
-    int stage_bytes;
-    int nh;
-    int p0;  // plane held by stage 0 at its first use (planes only grow from p0)
-    __device__ __forceinline__ int stage(int p) const { return (int)((unsigned)(p - p0) % SR); }
-    __device__ __forceinline__ uint32_t parity(int p) const { return ((unsigned)(p - p0) / SR) & 1u; }
-    __device__ __forceinline__ const float *halo(int s, int f) const {
-        return reinterpret_cast<const float *>(base + s * stage_bytes + f * HB);
-    }
-    __device__ __forceinline__ float *center(int s, int f) const {
-        return reinterpret_cast<float *>(base + s * stage_bytes + nh * HB + f * CB);
-    }
+constexpr int VX = 2;  // cells per thread along x
+
+struct QV {
+    float v[VX];
 };
 
-template <int ROWS, int SR, int NH, int NC>
-__device__ __forceinline__ void issue_plane(const Ring<ROWS, SR> &R, const CUtensorMap *tm, int x0,
-                                            int z0, int p) {
-    constexpr int HB = efm_halo_bytes(ROWS), CB = efm_center_bytes(ROWS);
-    const int s = R.stage(p);
-    uint64_t *bar = &R.bar[s];
-    unsigned char *st = R.base + s * R.stage_bytes;
-    efm_mbar_expect_tx(bar, NH * efm_halo_tx(ROWS) + NC * CB);
-#pragma unroll
-    for (int f = 0; f < NH; ++f)
-        efm_tma_load_3d(st + f * HB, tm + f, bar, x0 - EFM_HX_OFF, z0 - 1, p);
-#pragma unroll
-    for (int f = 0; f < NC; ++f)
-        efm_tma_load_3d(st + NH * HB + f * CB, tm + NH + f, bar, x0, z0, p);
+__device__ __forceinline__ QV ldv(const unsigned char *f, int i) {
+    const float2 a = *reinterpret_cast<const float2 *>(reinterpret_cast<const float *>(f) + i);
+    return QV{{a.x, a.y}};
 }
 
-// End of plane j, issuing thread, after the block barrier: store the n updated cell fields
-// [f0, f0 + n) of plane j's stage through the maps sm[0 .. n) (when `store`), close plane j's
-// bulk group, and refill the stage of plane j-1 with plane j-1+SR once the store out of it
-// (closed one plane earlier) has finished reading it.
-template <int ROWS, int SR, int NH, int NC>
-__device__ __forceinline__ void advance(const Ring<ROWS, SR> &R, const CUtensorMap *tm,
-                                        const CUtensorMap *sm, int f0, int n, bool store, int x0,
-                                        int z0, int j, int last) {
-    if (store) {
-        const int s = R.stage(j);
-        for (int f = 0; f < n; ++f) efm_tma_store_3d(sm + f, R.center(s, f0 + f), x0, z0, j);
-    }
-    efm_bulk_commit();
-    if (j - 1 + SR <= last) {
-        efm_bulk_wait_read<1>();
-        issue_plane<ROWS, SR, NH, NC>(R, tm, x0, z0, j - 1 + SR);
-    }
+__device__ __forceinline__ float2 ld2(const unsigned char *f, int i) {
+    return *reinterpret_cast<const float2 *>(reinterpret_cast<const float *>(f) + i);
 }
 
-struct Tile {
-    int tx, tz, x0, z0, ys, ye;
-};
-
-template <int ROWS>
-__device__ __forceinline__ Tile stream_tile(const EfmInst &I, int block) {
-    const int lt = block - I.tile_begin;
-    Tile t;
-    t.tx = lt % I.tiles_x;
-    const int rem = lt / I.tiles_x;
-    t.tz = rem % I.tiles_z;
-    const int ty = rem / I.tiles_z;
-    t.x0 = t.tx * EFM_STX;
-    t.z0 = t.tz * efm_st_tz(ROWS);
-    t.ys = ty * I.ychunk;
-    t.ye = min(I.ny, t.ys + I.ychunk);
-    return t;
+__device__ __forceinline__ float ld1(const unsigned char *f, int i) {
+    return reinterpret_cast<const float *>(f)[i];
 }
 
-// After a wait gave up: wait (with the default bound) for the loads still in flight, planes
-// first..last, so that no TMA write into this block's shared memory outlives the block.
-// `first` is the oldest plane no block-wide wait has confirmed; planes in flight occupy
-// distinct stages whose current phase is theirs, so each wait is well defined (an older
-// plane's stage may already be two phases further, where its parity would be ambiguous).
-template <int ROWS, int SR>
-__device__ void drain(const Ring<ROWS, SR> &R, int first, int last) {
-    for (int p = first; p <= last; ++p) efm_mbar_wait(&R.bar[R.stage(p)], R.parity(p), nullptr);
+// two consecutive floats (8-byte aligned) of memory this launch also writes
+__device__ __forceinline__ QV ldgv(const float *p) {
+    QV a;
+    asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(a.v[0]), "=f"(a.v[1]) : "l"(p) : "memory");
+    return a;
 }
 
-// The thread that issues the block's TMA loads and stores: lane 0 of a warp of the first
-// thread row whose 32 cells of x hold no x-CPML cell, when there is one.  Such a warp
-// finishes each plane before the CPML warps, so the issue work stays off the slowest warp.
-__device__ __forceinline__ int stream_issuer(const Tile &T, int nx, int W) {
-    for (int half = 1; half >= 0; --half) {
-        const int xa = T.x0 + 32 * half;
-        if (xa >= W && xa + 31 < nx - W) return 32 * half;
-    }
-    return 0;
+__device__ __forceinline__ void stv(float *p, const QV &a) {
+    asm volatile("st.global.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(a.v[0]), "f"(a.v[1]) : "memory");
 }
 
-// Block set-up shared by both kernels: barriers, prologue loads, source flag, receiver bits.
-template <int ROWS, int SR, int NH, int NC>
-__device__ __forceinline__ void stream_setup(const EfmInst &I, const Tile &T, Ring<ROWS, SR> &R,
-                                             const CUtensorMap *tm, int *s_flags,
-                                             unsigned long long *s_recbits, int iss) {
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < SR; ++s) efm_mbar_init(&R.bar[s], 1);
-        efm_fence_barrier_init();
-        int f = 0;
-        for (int s = 0; s < I.nsrc; ++s)
-            if (I.sx[s] >= T.x0 && I.sx[s] < T.x0 + EFM_STX && I.sz[s] >= T.z0 &&
-                I.sz[s] < T.z0 + efm_st_tz(ROWS) && I.sy[s] >= T.ys && I.sy[s] < T.ye)
-                f = 1;
-        *s_flags = f;
-    }
-    if (threadIdx.x < 32) {
-        // bit q: plane ys + q holds a receiver inside this tile (map rows are EFM_REC_TZ high)
-        const int l = threadIdx.x;
-        const int nz4 = (I.nz + EFM_REC_TZ - 1) / EFM_REC_TZ;
-        const int64_t row = (int64_t)nz4 * I.tiles_x;
-        bool a = false, b = false;
-#pragma unroll
-        for (int r = 0; r < ROWS; ++r) {
-            const int z4 = T.tz * ROWS + r;
-            if (z4 >= nz4) break;
-            const int64_t off = (int64_t)z4 * I.tiles_x + T.tx;
-            a = a || (T.ys + l < T.ye && I.rec_tile[(int64_t)(T.ys + l) * row + off]);
-            b = b || (T.ys + 32 + l < T.ye && I.rec_tile[(int64_t)(T.ys + 32 + l) * row + off]);
+__device__ __forceinline__ void st1(float *p, float a) {
+    asm volatile("st.global.f32 [%0], %1;" ::"l"(p), "f"(a) : "memory");
+}
+
+// A cell's memory variables (one family, three components and a pad).
+__device__ __forceinline__ void ld_psi(const float4 *p, float (&a)[3]) {
+    float pad;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(a[0]), "=f"(a[1]), "=f"(a[2]), "=f"(pad)
+                 : "l"(p)
+                 : "memory");
+}
+
+__device__ __forceinline__ void st_psi_if(bool c, float4 *p, float x, float y, float z) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %0, 0;\n\t@q st.global.v4.f32 [%1], {%2, %3, %4, %5};\n\t}" ::"r"(
+            (uint32_t)c),
+        "l"(p), "f"(x), "f"(y), "f"(z), "f"(0.f)
+        : "memory");
+}
+
+// ------------------------------------------------------------------------------- the ring
+// Position in the ring: slot q (of D + 1) and the one before it, its barrier (q mod D) and phase.
+template <int D>
+struct Cursor {
+    int cs = 0, hs = 0, hp = D;
+    uint32_t ph = 0;
+    __device__ __forceinline__ void next() {
+        hp = hs;
+        hs = hs == D ? 0 : hs + 1;
+        if (++cs == D) {
+            cs = 0;
+            ph ^= 1u;
         }
-        const unsigned lo = __ballot_sync(0xffffffffu, a), hi = __ballot_sync(0xffffffffu, b);
-        if (l == 0) *s_recbits = (unsigned long long)lo | ((unsigned long long)hi << 32);
     }
-    // everything above reads only the call's static tables; the fields come after the
-    // preceding kernel has finished
-    efm_pdl_wait();
-    __syncthreads();
-    if ((int)threadIdx.x == iss) {
-        for (int q = 0; q < NH + NC; ++q) efm_prefetch_tmap(tm + q);
-        for (int p = R.p0; p <= min(T.ye, R.p0 + SR - 1); ++p)
-            issue_plane<ROWS, SR, NH, NC>(R, tm, T.x0, T.z0, p);
-    }
+};
+
+// One chunk: a tile over the planes [ys, ye) of a stress (0), velocity (1) or imaging (2) pass; -1: no more.
+struct Chunk {
+    int type, x0, z0, ys, ye, col, tw, th;
+};
+
+// The block's shared memory: D + 1 ring slots, then this.  The barriers: a slot's loads have
+// arrived (full), every consumer warp has read it (empty), a chunk's description is in place
+// (ready: the consumers set up a chunk while its first loads travel).  Two descriptions with their
+// table entries (three for the deeper ring): a chunk has at least two slots, so the producer, with
+// the first slot of chunk c in hand -- the consumers have left the slot D before it -- knows that
+// they have left chunk c - N.
+template <int D>
+struct Block {
+    static constexpr int N = D / 2 + 1;
+    uint64_t full[D], empty[D], ready[N];
+    Chunk chunk[N];
+    alignas(16) EfmInst inst[N];
+    int abort;
+    uint32_t lim;       // polls per wait (0: the default bound)
+    unsigned int *err;  // the context's error word
+    static __device__ __forceinline__ int next(int i) { return i == N - 1 ? 0 : i + 1; }
+};
+
+template <int D, int SLOT>
+__device__ __forceinline__ Block<D> &block_state() {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    return *reinterpret_cast<Block<D> *>(smem + (D + 1) * SLOT);
 }
 
-// Per-block constants of the plane loop, read from the instance table once.  The loop's
-// mbarrier waits are asm statements with a memory clobber, after which the compiler would
-// otherwise reload every table field it touches.  The memory variables of a pass are one
-// group of each slab family (0: stress, 1: velocity), a 16-byte vector per cell; every cell
-// offset into a family fits 32 bits (the host checks), so an address is one 32-bit add and
-// one wide multiply-add off a 64-bit base.
-struct Hot {
-    float4 *psx, *psy, *psz;  // this pass's group of each family
-    int pxs, pys, pzs;        // plane strides in cells: nz*2W (x slabs), nz*nx (y slabs), W*nx (z)
-    float k;
-    int nx, ny, nz, W;
-};
-
-__device__ __forceinline__ Hot make_hot(const EfmInst &I, int group) {
-    Hot h;
-    h.nx = I.nx;
-    h.ny = I.ny;
-    h.nz = I.nz;
-    h.W = I.W;
-    h.pxs = I.nz * 2 * I.W;
-    h.pys = I.nz * I.nx;
-    h.pzs = I.W * I.nx;
-    h.psx = reinterpret_cast<float4 *>(I.psi_x) + (int64_t)group * I.ny * h.pxs;
-    h.psy = reinterpret_cast<float4 *>(I.psi_y) + (int64_t)group * 2 * I.W * h.pys;
-    h.psz = reinterpret_cast<float4 *>(I.psi_z) + (int64_t)group * I.ny * h.pzs;
-    h.k = I.k;
-    return h;
+template <int SLOT>
+__device__ __forceinline__ unsigned char *ring_slot(int i) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    return smem + i * SLOT;
 }
 
-// One thread row (cells (x, z0 + r + 4h) of every plane): ring indices, whether the stencil
-// updates it, and its memory-variable offsets inside a plane of each slab family (-1: none).
-struct Row {
-    int hidx, cidx;
-    int pxo, pyo, pzo;
-    bool in;
-    bool wx, wz;  // some lane of this warp has an x (z) memory variable in this row
+template <int D>
+__device__ __forceinline__ void give_up(Block<D> &B) {
+    *(volatile int *)&B.abort = 1;
+    if (B.err) atomicOr(B.err, EFM_ERR_FLAG_TIMEOUT);
+}
+
+// Wait (bounded) that also gives up once another warp of the block has given up.
+template <int D>
+__device__ __forceinline__ bool ring_wait(Block<D> &B, uint64_t *bar, uint32_t parity, uint32_t lim) {
+    if (lim == 0) {
+        for (uint32_t i = 0; i < EFM_WAIT_LIMIT; ++i) {
+            if (efm_mbar_try_wait(bar, parity)) return true;
+            if ((i & 255u) == 255u && *(volatile int *)&B.abort) return false;
+        }
+    } else {
+        for (uint32_t i = 0; i < lim; ++i)
+            if (efm_mbar_test_wait(bar, parity)) return true;
+    }
+    give_up(B);
+    return false;
+}
+
+// What a consumer warp walks the ring with.
+template <int D, int SLOT>
+struct Ctx {
+    Block<D> &B;
+    uint32_t lim;
+    bool lane0;
+    Cursor<D> cur;
+    static constexpr int START = D << 8;  // slot 0, before it slot D
+    __device__ __forceinline__ Ctx(int packed)
+        : B(block_state<D, SLOT>()), lim(B.lim), lane0((threadIdx.x & 31) == 0) {
+        cur.cs = packed & 15;
+        cur.hs = (packed >> 4) & 15;
+        cur.hp = (packed >> 8) & 15;
+        cur.ph = (packed >> 12) & 1;
+    }
+    __device__ __forceinline__ int packed() const {
+        return cur.cs | cur.hs << 4 | cur.hp << 8 | (int)cur.ph << 12;
+    }
+    __device__ __forceinline__ const unsigned char *slot() const { return ring_slot<SLOT>(cur.hs); }
+    __device__ __forceinline__ const unsigned char *prev() const { return ring_slot<SLOT>(cur.hp); }
+    __device__ __forceinline__ bool wait() { return ring_wait(B, &B.full[cur.cs], cur.ph, lim); }
+    // this warp is done with the slot
+    __device__ __forceinline__ void release() {
+        __syncwarp();
+        if (lane0) efm_mbar_arrive(&B.empty[cur.cs]);
+        cur.next();
+    }
 };
 
-// Plane offsets of the three families (y: only on the planes of the y slabs).
-struct PsiPlane {
-    int x, y, z;
-    bool has_y;
+// ------------------------------------------------------------- per-thread state of a chunk
+// The thread's pair (x, x + 1) at z: its place in the boxes of a plane (i0: rows of tw + 4, k0:
+// rows of tw) and what applies to its cells.
+enum {
+    F_IN = 3,           // bit v: the stencil updates cell v (planes permitting)
+    F_PX = 3 << 4,      // ... and it has x memory variables
+    F_ACT = 3 << 8,     // cell v lies in the grid and the pair in the tile
+    F_PZ = 1 << 12,     // the updated cells have z memory variables
+    F_WX = 1 << 13,     // some lane of the warp has x memory variables
+    F_WZ = 1 << 14,     // ... z memory variables
+    F_PART = 1 << 15    // ... updates some but not all of its cells
 };
 
-__device__ __forceinline__ PsiPlane psi_plane(const Hot &H, int y) {
-    PsiPlane P;
-    P.x = y * H.pxs;
-    P.z = y * H.pzs;
-    P.has_y = y < H.W || y >= H.ny - H.W;
-    P.y = (y < H.W ? y : y - (H.ny - 2 * H.W)) * H.pys;
+struct Pair {
+    int x, z;
+    int i0, k0, hp, tw;  // hp = tw + 4
+    int fl;
+    __device__ __forceinline__ bool in(int v) const { return (fl >> v) & 1; }
+    __device__ __forceinline__ bool px(int v) const { return (fl >> (4 + v)) & 1; }
+    __device__ __forceinline__ bool act(int v) const { return (fl >> (8 + v)) & 1; }
+    __device__ __forceinline__ bool any_in() const { return fl & F_IN; }
+};
+
+template <bool BOX>
+__device__ __forceinline__ Pair make_pair(const EfmInst &I, const Chunk &T) {
+    Pair p;
+    const int nx = I.nx, nz = I.nz, W = I.W, per_row = T.tw / VX;
+    int r = threadIdx.x / per_row;
+    int c = VX * ((int)threadIdx.x - r * per_row);
+    const bool mine = r < T.th;
+    if (!mine) r = c = 0;
+    p.tw = T.tw;
+    p.hp = T.tw + 4;
+    p.x = T.x0 + c;
+    p.z = T.z0 + r;
+    p.i0 = r * p.hp + c;
+    p.k0 = r * T.tw + c;
+    const bool row = mine && p.z < nz;
+    const bool zin = row && p.z >= EFM_HS && p.z < nz - EFM_HS && !(BOX && p.z >= nz - W);
+    p.fl = 0;
+#pragma unroll
+    for (int v = 0; v < VX; ++v) {
+        const int x = p.x + v;
+        const bool slab = x < W || x >= nx - W;
+        const bool in = zin && x >= EFM_HS && x < nx - EFM_HS && !(BOX && slab);
+        p.fl |= (in ? 1 << v : 0) | (in && slab ? 16 << v : 0) | (row && x < nx ? 256 << v : 0);
+    }
+    if ((p.fl & F_IN) && p.z >= nz - W) p.fl |= F_PZ;
+    if (__any_sync(0xffffffffu, p.fl & F_PX)) p.fl |= F_WX;
+    if (__any_sync(0xffffffffu, p.fl & F_PZ)) p.fl |= F_WZ;
+    if (__any_sync(0xffffffffu, (p.fl & F_IN) != 0 && (p.fl & F_IN) != F_IN)) p.fl |= F_PART;
+    return p;
+}
+
+// CPML memory variables of the pair: a 16-byte vector (three components) per cell, group 0 the
+// stress pass's, 1 the velocity pass's of each slab family.  The first slab's base and 32-bit
+// offsets address all three families (one allocation; the host checks the range).  x and z
+// follow the planes; y is looked up on the planes of the y slabs.
+struct Psi {
+    float4 *base;
+    int x, z, sx, sz;
+    float ax[VX], bx[VX], az, bz;
+};
+
+__device__ __forceinline__ Psi psi_at(const EfmInst &I, const Pair &p, int group, int y) {
+    const int nx = I.nx, ny = I.ny, nz = I.nz, W = I.W;
+    Psi P;
+    P.base = reinterpret_cast<float4 *>(I.psi_x);
+    P.sx = nz * 2 * W;
+    P.sz = W * nx;
+    P.x = ((group * ny + y) * nz + p.z) * 2 * W + (p.x + VX - 1 < nx - W ? p.x : p.x - (nx - 2 * W));
+    P.z = 4 * W * ny * nz + 4 * W * nz * nx + ((group * ny + y) * W + p.z - (nz - W)) * nx + p.x;
+#pragma unroll
+    for (int v = 0; v < VX; ++v) {
+        P.ax[v] = p.px(v) ? I.cpml[p.x + v] : 0.f;
+        P.bx[v] = p.px(v) ? I.cpml[nx + p.x + v] : 0.f;
+    }
+    P.az = p.fl & F_PZ ? I.cpml[2 * (nx + ny) + p.z] : 0.f;
+    P.bz = p.fl & F_PZ ? I.cpml[2 * (nx + ny) + nz + p.z] : 0.f;
     return P;
 }
 
-// Request the old memory variables of one cell that it has (0-2 x family, 3-5 y family, 6-8
-// z family; the others are left unset and never read).  Each family sits behind a test that
-// is uniform over the warp (the row flags) or the block (the plane), so warps without memory
-// variables of a family branch past its code.
-__device__ __forceinline__ void load_psi(const Hot &H, const PsiPlane &P, const Row &r, float *pp) {
-    if (r.wx && r.pxo >= 0) {
-        const float4 v = H.psx[P.x + r.pxo];
-        pp[0] = v.x;
-        pp[1] = v.y;
-        pp[2] = v.z;
-    }
-    if (P.has_y) {
-        const float4 v = H.psy[P.y + r.pyo];
-        pp[3] = v.x;
-        pp[4] = v.y;
-        pp[5] = v.z;
-    }
-    if (r.wz && r.pzo >= 0) {
-        const float4 v = H.psz[P.z + r.pzo];
-        pp[6] = v.x;
-        pp[7] = v.y;
-        pp[8] = v.z;
-    }
+__device__ __forceinline__ int psi_y(const EfmInst &I, const Pair &p, int group, int y) {
+    const int nx = I.nx, ny = I.ny, nz = I.nz, W = I.W;
+    return 4 * W * ny * nz + ((group * 2 * W + (y < W ? y : y - (ny - 2 * W))) * nz + p.z) * nx + p.x;
 }
 
-// Pull the next plane's memory variables of one row into L1 (no register, no wait); the
-// plane after the current one is then an L1 hit instead of an L2 round trip that the warp
-// would wait for right after the stage wait.
-__device__ __forceinline__ void prefetch_psi(const Hot &H, const PsiPlane &P, const Row &r) {
-    if (r.wx && r.pxo >= 0)
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(H.psx + (P.x + r.pxo)));
-    if (P.has_y) asm volatile("prefetch.global.L1 [%0];" ::"l"(H.psy + (P.y + r.pyo)));
-    if (r.wz && r.pzo >= 0)
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(H.psz + (P.z + r.pzo)));
+// Pull the next plane's memory variables into L1 (no register, no wait).
+__device__ __forceinline__ void prefetch2(const float4 *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+
+__device__ __forceinline__ void prefetch_psi(const Pair &p, const Psi &P) {
+    if (p.fl & F_PX) prefetch2(P.base + (P.x + P.sx));
+    if (p.fl & F_PZ) prefetch2(P.base + (P.z + P.sz));
+}
+
+// ... and a chunk's first plane's.
+__device__ __forceinline__ void prefetch_first(const EfmInst &I, const Pair &p, const Psi &P, int group, int y) {
+    if (p.fl & F_PX) prefetch2(P.base + P.x);
+    if (p.fl & F_PZ) prefetch2(P.base + P.z);
+    if ((p.fl & F_IN) && (y < I.W || y >= I.ny - I.W)) prefetch2(P.base + psi_y(I, p, group, y));
+}
+
+// The old memory variables of the pair's cells, [cell][component] by family, zero where the pair has
+// none (a vector next to a slab cell's may be another cell's: it is read and not used).  Each
+// family sits behind a test that is uniform over the warp (x, z) or the block (y).  Requested
+// before the plane's wait, so the wait covers their latency; with YZ false only the x family, and
+// the others (12 registers per pair that would spill beside the plane's operands) are read where
+// they are used, from L1.  YZ pays where it does not spill (forward stress 128 x 128 x 96: 22.5 us,
+// 24.2 without) or little, for the adjoint velocity in a pair with much CPML (100 x 100 x 100, 20
+// layers: 25.3 us, 28.8 without); the adjoint stress and the velocity passes by themselves spill
+// more (forward velocity 256 x 256 x 128: 98.6 us with YZ, 93.9 without).
+template <int PML, bool YZ>
+struct PsiOld {
+    static constexpr bool EARLY = YZ && PML == 2;
+    float x[VX][3], y[EARLY ? VX : 1][3], z[EARLY ? VX : 1][3];
+    __device__ __forceinline__ void load(const Pair &p, const Psi &P, bool ypml, int py) {
+#pragma unroll
+        for (int v = 0; v < VX; ++v) x[v][0] = x[v][1] = x[v][2] = 0.f;
+        if (p.fl & F_PX) {
+#pragma unroll
+            for (int v = 0; v < VX; ++v) ld_psi(P.base + (P.x + v), x[v]);
+        }
+        if (EARLY) {
+#pragma unroll
+            for (int v = 0; v < VX; ++v) y[v][0] = y[v][1] = y[v][2] = z[v][0] = z[v][1] = z[v][2] = 0.f;
+            if (ypml && (p.fl & F_IN)) {
+#pragma unroll
+                for (int v = 0; v < VX; ++v) ld_psi(P.base + (py + v), y[v]);
+            }
+            if (p.fl & F_PZ) {
+#pragma unroll
+                for (int v = 0; v < VX; ++v) ld_psi(P.base + (P.z + v), z[v]);
+            }
+        }
+    }
+};
+
+// psi <- b psi + a d for one cell's three components of a family (o: old in, new out); cells
+// without them (c false) get zeros.
+__device__ __forceinline__ void psi_step(bool c, float4 *q, float (&o)[3], float a, float b, float d0, float d1,
+                                         float d2) {
+    const float n0 = b * o[0] + a * d0, n1 = b * o[1] + a * d1, n2 = b * o[2] + a * d2;
+    o[0] = c ? n0 : 0.f;
+    o[1] = c ? n1 : 0.f;
+    o[2] = c ? n2 : 0.f;
+    st_psi_if(c, q, n0, n1, n2);
+}
+
+// The same with the old values read here (late) or handed in (early).
+template <bool EARLY>
+__device__ __forceinline__ void psi_step_yz(bool c, float4 *q, float (&o)[3], const float (&early)[3], float a, float b,
+                                            float d0, float d1, float d2) {
+    o[0] = o[1] = o[2] = 0.f;
+    if (EARLY) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) o[k] = early[k];
+        psi_step(c, q, o, a, b, d0, d1, d2);
+    } else if (c) {
+        ld_psi(q, o);
+        o[0] = b * o[0] + a * d0;
+        o[1] = b * o[1] + a * d1;
+        o[2] = b * o[2] + a * d2;
+        st_psi_if(true, q, o[0], o[1], o[2]);
+    }
 }
 
 // ------------------------------------------------------------------------------ stress
-// CPML coefficients of one cell, loaded once per block (x, z) or per plane (y)
-struct Coef {
-    float ax, bx, ay, by, az, bz;
-};
-
-// New stress of one cell, written over its old stress in the ring (the block stores the
-// plane with TMA afterwards).
-template <int PASS, int ROWS, int SR, bool PML>
-__device__ __forceinline__ void stress_cell(const EfmInst &I, const Ring<ROWS, SR> &R, int sm, int s0,
-                                            int sp, int it, int x, int y, int z, const Row &rw,
-                                            bool has_src, const float *pp, const Coef &C,
-                                            const Hot &H, const PsiPlane &P) {
-    constexpr int CF = Ring<ROWS, SR>::CF;
-    const int hidx = rw.hidx;
-    const float *vx0 = R.halo(s0, 0), *vy0 = R.halo(s0, 1), *vz0 = R.halo(s0, 2);
-    const float *rm0 = R.halo(s0, 3), *rm1 = R.halo(sp, 3);
-    const float vxc = vx0[hidx], vyc = vy0[hidx], vzc = vz0[hidx];
-    const float dvx_dx = vxc - vx0[hidx - 1];
-    const float dvy_dy = vyc - R.halo(sm, 1)[hidx];
-    const float dvz_dz = vzc - vz0[hidx - EFM_HX];
-    const float dvx_dz = vx0[hidx + EFM_HX] - vxc;
-    const float dvx_dy = R.halo(sp, 0)[hidx] - vxc;
-    const float dvy_dx = vy0[hidx + 1] - vyc;
-    const float dvy_dz = vy0[hidx + EFM_HX] - vyc;
-    const float dvz_dx = vz0[hidx + 1] - vzc;
-    const float dvz_dy = R.halo(sp, 2)[hidx] - vzc;
-    float pvx_x = 0.f, pvy_x = 0.f, pvz_x = 0.f, pvy_y = 0.f, pvx_y = 0.f, pvz_y = 0.f;
-    float pvz_z = 0.f, pvx_z = 0.f, pvy_z = 0.f;
-    if (PML && PASS != EFM_REV) {
-        // pp: the old memory variables requested at the top of the iteration
-        if (rw.wx && rw.pxo >= 0) {
-            const float a = C.ax, b = C.bx;
-            pvx_x = b * pp[0] + a * dvx_dx;
-            pvy_x = b * pp[1] + a * dvy_dx;
-            pvz_x = b * pp[2] + a * dvz_dx;
-            H.psx[P.x + rw.pxo] = make_float4(pvx_x, pvy_x, pvz_x, 0.f);
-        }
-        if (P.has_y) {
-            const float a = C.ay, b = C.by;
-            pvy_y = b * pp[3] + a * dvy_dy;
-            pvx_y = b * pp[4] + a * dvx_dy;
-            pvz_y = b * pp[5] + a * dvz_dy;
-            H.psy[P.y + rw.pyo] = make_float4(pvy_y, pvx_y, pvz_y, 0.f);
-        }
-        if (rw.wz && rw.pzo >= 0) {
-            const float a = C.az, b = C.bz;
-            pvz_z = b * pp[6] + a * dvz_dz;
-            pvx_z = b * pp[7] + a * dvx_dz;
-            pvy_z = b * pp[8] + a * dvy_dz;
-            H.psz[P.z + rw.pzo] = make_float4(pvz_z, pvx_z, pvy_z, 0.f);
-        }
-    }
-    // harmonic 4-point averages of mu from the precomputed 1/mu (:80-89)
-    const float r0 = rm0[hidx], ri = rm0[hidx + 1], rk = rm0[hidx + EFM_HX];
-    const float rik = rm0[hidx + 1 + EFM_HX];
-    const float rj = rm1[hidx], rjk = rm1[hidx + EFM_HX], rij = rm1[hidx + 1];
-    const float mu0 = frcp(r0);
-    const float mu_xz = 4.f * frcp(r0 + ri + rk + rik);
-    const float mu_xy = 4.f * frcp(r0 + ri + rj + rij);
-    const float mu_yz = 4.f * frcp(r0 + rj + rk + rjk);
-    float *cw = R.center(s0, 0) + rw.cidx;  // lambda, then txx tyy tzz txy txz tyz
-    const float lam = cw[0];
-    const float k = H.k;
-    const float l2m = lam + 2.f * mu0;
-    float txx = cw[CF] + k * (l2m * (dvx_dx + pvx_x) + lam * (dvy_dy + dvz_dz + pvy_y + pvz_z));
-    float tyy = cw[2 * CF] + k * (l2m * (dvy_dy + pvy_y) + lam * (dvx_dx + dvz_dz + pvx_x + pvz_z));
-    float tzz = cw[3 * CF] + k * (l2m * (dvz_dz + pvz_z) + lam * (dvx_dx + dvy_dy + pvx_x + pvy_y));
-    float txy = cw[4 * CF] + k * mu_xy * ((dvx_dy + pvx_y) + (dvy_dx + pvy_x));
-    float txz = cw[5 * CF] + k * mu_xz * ((dvx_dz + pvx_z) + (dvz_dx + pvz_x));
-    float tyz = cw[6 * CF] + k * mu_yz * ((dvy_dz + pvy_z) + (dvz_dy + pvz_y));
-    if (PASS != EFM_ADJ && has_src) {
-        const int widx = (PASS == EFM_FWD) ? it : I.nt - 1 - it;
-        for (int s = 0; s < I.nsrc; ++s) {
-            if (x == I.sx[s] && y == I.sy[s] && z == I.sz[s]) {
-                const float w = I.wav[widx];
-                const float sg = (PASS == EFM_FWD) ? 1.f : -1.f;
-                txx = __fadd_rn(txx, sg * __fmul_rn(I.mt[s][0], w));
-                tyy = __fadd_rn(tyy, sg * __fmul_rn(I.mt[s][1], w));
-                tzz = __fadd_rn(tzz, sg * __fmul_rn(I.mt[s][2], w));
-                txy = __fadd_rn(txy, sg * __fmul_rn(I.mt[s][3], w));
-                txz = __fadd_rn(txz, sg * __fmul_rn(I.mt[s][4], w));
-                tyz = __fadd_rn(tyz, sg * __fmul_rn(I.mt[s][5], w));
+// Neighbour fields: vx (x0-4, z0), vy (x0, z0), vz (x0, z0-1), 1/mu (x0, z0), each tw+4 columns
+// and th+1 rows; cell fields: lambda txx tyy tzz txy txz tyz.  First slot's cell part: vy of the
+// plane before the chunk.
+// New stress of the pair on plane y.  h: neighbour fields of plane y, hn: of plane y + 1, cc: the
+// cell fields; vym: vy of plane y - 1 (in), of plane y (out).
+template <int PASS, int NT, int PML>
+__device__ __forceinline__ void stress_pair(const EfmInst &I, const unsigned char *h, const unsigned char *hn,
+                                            const unsigned char *cc, int it, int y, const Pair &p, bool has_src,
+                                            float k, const Psi &P, bool ypml, int py, float ay, float by,
+                                            PsiOld<PML, PASS == EFM_FWD> &O, QV &vym, float *t0, int64_t N) {
+    constexpr int XZ = efm_slot_xz(NT), CF = efm_slot_c(NT);
+    const int i0 = p.i0, i1 = p.i0 + p.hp;
+    const QV vx = ldv(h, i0 + 4), vxz = ldv(h, i1 + 4), vxj = ldv(hn, i0 + 4);
+    const float vxm = ld1(h, i0 + 3);
+    const QV vy = ldv(h + XZ, i0), vyz = ldv(h + XZ, i1);
+    const float vyx = ld1(h + XZ, i0 + VX);
+    const QV vz = ldv(h + 2 * XZ, i1), vzm = ldv(h + 2 * XZ, i0), vzj = ldv(hn + 2 * XZ, i1);
+    const float vzx = ld1(h + 2 * XZ, i1 + VX);
+    const QV m0 = ldv(h + 3 * XZ, i0), mk = ldv(h + 3 * XZ, i1), mj = ldv(hn + 3 * XZ, i0);
+    const QV mjk = ldv(hn + 3 * XZ, i1);
+    const float mi = ld1(h + 3 * XZ, i0 + VX), mik = ld1(h + 3 * XZ, i1 + VX), mij = ld1(hn + 3 * XZ, i0 + VX);
+    const QV lam4 = ldv(cc, p.k0);
+    QV t[6];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) t[q] = ldv(cc + (1 + q) * CF, p.k0);
+    QV o[6];
+#pragma unroll
+    for (int v = 0; v < VX; ++v) {
+        const float vxc = vx.v[v], vyc = vy.v[v], vzc = vz.v[v];
+        const float dvx_dx = vxc - (v ? vx.v[v - 1] : vxm);
+        const float dvy_dy = vyc - vym.v[v];
+        const float dvz_dz = vzc - vzm.v[v];
+        const float dvx_dz = vxz.v[v] - vxc;
+        const float dvx_dy = vxj.v[v] - vxc;
+        const float dvy_dx = (v < VX - 1 ? vy.v[v + 1] : vyx) - vyc;
+        const float dvy_dz = vyz.v[v] - vyc;
+        const float dvz_dx = (v < VX - 1 ? vz.v[v + 1] : vzx) - vzc;
+        const float dvz_dy = vzj.v[v] - vzc;
+        // harmonic 4-point averages of mu from the precomputed 1/mu (:80-89)
+        const float r0 = m0.v[v], ri = v < VX - 1 ? m0.v[v + 1] : mi, rk = mk.v[v];
+        const float rik = v < VX - 1 ? mk.v[v + 1] : mik;
+        const float rj = mj.v[v], rjk = mjk.v[v], rij = v < VX - 1 ? mj.v[v + 1] : mij;
+        const float mu0 = frcp(r0);
+        const float mu_xz = 4.f * frcp(r0 + ri + rk + rik);
+        const float mu_xy = 4.f * frcp(r0 + ri + rj + rij);
+        const float mu_yz = 4.f * frcp(r0 + rj + rk + rjk);
+        const float lam = lam4.v[v];
+        const float l2m = lam + 2.f * mu0;
+        float txx, tyy, tzz, txy, txz, tyz;
+        if (PML == 0) {  // (the sums below without their zero terms)
+            txx = t[0].v[v] + k * two_products(l2m, dvx_dx, lam, (dvy_dy + dvz_dz));
+            tyy = t[1].v[v] + k * two_products(l2m, dvy_dy, lam, (dvx_dx + dvz_dz));
+            tzz = t[2].v[v] + k * two_products(l2m, dvz_dz, lam, (dvx_dx + dvy_dy));
+            txy = t[3].v[v] + k * mu_xy * (dvx_dy + dvy_dx);
+            txz = t[4].v[v] + k * mu_xz * (dvx_dz + dvz_dx);
+            tyz = t[5].v[v] + k * mu_yz * (dvy_dz + dvz_dy);
+        } else {
+            float pvx_x = 0.f, pvy_x = 0.f, pvz_x = 0.f, pvy_y = 0.f, pvx_y = 0.f, pvz_y = 0.f;
+            float pvz_z = 0.f, pvx_z = 0.f, pvy_z = 0.f;
+            if (PML == 1 || (p.fl & F_WX)) {
+                psi_step(p.px(v), P.base + (P.x + v), O.x[v], P.ax[v], P.bx[v], dvx_dx, dvy_dx, dvz_dx);
+                pvx_x = O.x[v][0];
+                pvy_x = O.x[v][1];
+                pvz_x = O.x[v][2];
             }
-        }
-    }
-    cw[CF] = txx;
-    cw[2 * CF] = tyy;
-    cw[3 * CF] = tzz;
-    cw[4 * CF] = txy;
-    cw[5 * CF] = txz;
-    cw[6 * CF] = tyz;
-    if (PASS == EFM_ADJ && has_src && I.mtg != nullptr) {
-        for (int s = 0; s < I.nsrc; ++s) {
-            if (x == I.sx[s] && y == I.sy[s] && z == I.sz[s]) {
-                const float w = I.wav[I.nt - 1 - it];
-                const float f = __frcp_rn(2.f * mu0 * (3.f * lam + 2.f * mu0));
-                const float lpm2 = 2.f * (lam + mu0);
-                double *g = I.mtg + 6 * s;
-                g[0] += (double)(w * (f * (lpm2 * txx - lam * tyy - lam * tzz)));
-                g[1] += (double)(w * (f * (lpm2 * tyy - lam * txx - lam * tzz)));
-                g[2] += (double)(w * (f * (lpm2 * tzz - lam * txx - lam * tyy)));
-                g[3] += (double)(w * (txy * __frcp_rn(mu_xy)));
-                g[4] += (double)(w * (txz * __frcp_rn(mu_xz)));
-                g[5] += (double)(w * (tyz * __frcp_rn(mu_yz)));
+            float oy[3], oz[3];
+            if (PML == 2 && ypml) {
+                psi_step_yz<O.EARLY>(p.in(v), P.base + (py + v), oy, O.y[O.EARLY ? v : 0], ay, by, dvy_dy, dvx_dy,
+                                     dvz_dy);
+                pvy_y = oy[0];
+                pvx_y = oy[1];
+                pvz_y = oy[2];
             }
+            if (PML == 2 && (p.fl & F_WZ)) {
+                psi_step_yz<O.EARLY>((p.fl & F_PZ) && p.in(v), P.base + (P.z + v), oz, O.z[O.EARLY ? v : 0], P.az,
+                                     P.bz, dvz_dz, dvx_dz, dvy_dz);
+                pvz_z = oz[0];
+                pvx_z = oz[1];
+                pvy_z = oz[2];
+            }
+            txx = t[0].v[v] + k * two_products(l2m, (dvx_dx + pvx_x), lam, (dvy_dy + dvz_dz + pvy_y + pvz_z));
+            tyy = t[1].v[v] + k * two_products(l2m, (dvy_dy + pvy_y), lam, (dvx_dx + dvz_dz + pvx_x + pvz_z));
+            tzz = t[2].v[v] + k * two_products(l2m, (dvz_dz + pvz_z), lam, (dvx_dx + dvy_dy + pvx_x + pvy_y));
+            txy = t[3].v[v] + k * mu_xy * ((dvx_dy + pvx_y) + (dvy_dx + pvy_x));
+            txz = t[4].v[v] + k * mu_xz * ((dvx_dz + pvx_z) + (dvz_dx + pvz_x));
+            tyz = t[5].v[v] + k * mu_yz * ((dvy_dz + pvy_z) + (dvz_dy + pvz_y));
         }
-    }
-}
-
-// Row constants of the thread's cells (x, z0 + lr + 4h).
-template <int PASS, int ROWS>
-__device__ __forceinline__ void make_rows(const Hot &H, const Tile &T, int x, int lx, int lr,
-                                          bool stress, Row *rw) {
-    const int nx = H.nx, nz = H.nz, W = H.W;
-    const bool xpml = x < nx && (x < W || x >= nx - W);
-    const int xs = x < W ? x : x - (nx - 2 * W);
-#pragma unroll
-    for (int h = 0; h < ROWS; ++h) {
-        const int lz = lr + 4 * h, z = T.z0 + lz;
-        rw[h].hidx = (lz + 1) * EFM_HX + lx + EFM_HX_OFF;
-        rw[h].cidx = lz * EFM_STX + lx;
-        rw[h].in = x >= EFM_HS && x < nx - EFM_HS && z >= EFM_HS && z < nz - EFM_HS &&
-                   !(stress && PASS == EFM_REV && (x < W || x >= nx - W || z >= nz - W));
-        rw[h].pxo = xpml && z < nz ? z * 2 * W + xs : -1;
-        rw[h].pyo = z * nx + x;
-        rw[h].pzo = z < nz && z >= nz - W && x < nx ? (z - (nz - W)) * nx + x : -1;
-        rw[h].wx = __any_sync(0xffffffffu, rw[h].pxo >= 0);
-        rw[h].wz = __any_sync(0xffffffffu, rw[h].pzo >= 0);
-    }
-}
-
-// Boundary-strip slots of one thread row (efm_strip_slots_v with the plane terms split off):
-// X faces xf + yr*bz, Y faces yf + row*bz*bx on the two planes next to each y face of the box,
-// Z faces zf + yr*bx; -1 where the row owns no slot of that family (yf < 0: (x, z) outside the
-// box).
-struct StripRow {
-    int xf, yf, zf;
-};
-
-__device__ __forceinline__ StripRow strip_row(int nx, int nz, int by, int W, int x, int z) {
-    const int bx = nx - 2 * W, bz = nz - W - 2;
-    const int xr = x - W, zr = z - 2;
-    StripRow s{-1, -1, -1};
-    if (xr < 0 || xr >= bx || zr < 0 || zr >= bz) return s;
-    const int offY = 4 * by * bz, offZ = offY + 4 * bz * bx;
-    const int col = xr < 2 ? xr : (xr >= bx - 2 ? 2 + (xr - (bx - 2)) : -1);
-    if (col >= 0) s.xf = col * by * bz + zr;
-    s.yf = offY + zr * bx + xr;
-    const int pl = zr < 2 ? zr : (zr >= bz - 2 ? 2 + (zr - (bz - 2)) : -1);
-    if (pl >= 0) s.zf = offZ + pl * by * bx + xr;
-    return s;
-}
-
-}  // namespace
-
-// halo fields: vx vy vz 1/mu ; center fields: lambda txx tyy tzz txy txz tyz
-template <int PASS, int ROWS, int SR>
-__device__ __forceinline__ void stress_body(const EfmInst *__restrict__ insts, int ninst, int it,
-                                            int block, unsigned char *smem) {
-    constexpr int NH = 4, NC = 7;
-    __shared__ uint64_t bars[SR];
-    __shared__ int s_src;
-    __shared__ unsigned long long s_rec;
-    efm_pdl_trigger();
-    const EfmInst &I = insts[efm_find_inst(insts, ninst, block)];
-    if (it >= I.nsteps) return;
-    Tile T = stream_tile<ROWS>(I, block);
-    const int nx = I.nx, ny = I.ny, nz = I.nz, W = I.W;
-    if (PASS == EFM_REV) {
-        // the rebuild updates only the box x in [W, nx-W), y in [W, ny-W), z < nz-W and leaves
-        // every other stress as it is: march only over the box planes, skip tiles outside it
-        T.ys = max(T.ys, W);
-        T.ye = min(T.ye, ny - W);
-        if (T.ys >= T.ye || T.z0 >= nz - W || T.x0 >= nx - W || T.x0 + EFM_STX <= W) return;
-    }
-    const int lx = threadIdx.x % EFM_STX, lr = threadIdx.x / EFM_STX;
-    const int x = T.x0 + lx;
-    const CUtensorMap *tm = I.tmap;
-    Ring<ROWS, SR> R{smem, bars, NH * Ring<ROWS, SR>::HB + NC * Ring<ROWS, SR>::CB, NH, T.ys - 1};
-    const int iss = stream_issuer(T, nx, W);
-    stream_setup<ROWS, SR, NH, NC>(I, T, R, tm, &s_src, &s_rec, iss);
-    const bool has_src = s_src != 0;
-    unsigned int *const err = I.err;  // read once: the waits' clobbers would reload it
-    const uint32_t wl = I.wait_lim;
-    const Hot H = make_hot(I, 0);
-    Row rw[ROWS];
-    make_rows<PASS, ROWS>(H, T, x, lx, lr, true, rw);
-    Coef cf[ROWS];
-    const bool xpml = x < nx && (x < W || x >= nx - W);
-    const float cx_a = xpml ? I.cpml[x] : 0.f, cx_b = xpml ? I.cpml[nx + x] : 0.f;
-#pragma unroll
-    for (int h = 0; h < ROWS; ++h) {
-        const int z = T.z0 + lr + 4 * h;
-        const bool zpml = z < nz && z >= nz - W;
-        cf[h].ax = cx_a;
-        cf[h].bx = cx_b;
-        cf[h].az = zpml ? I.cpml[2 * nx + 2 * ny + z] : 0.f;
-        cf[h].bz = zpml ? I.cpml[2 * nx + 2 * ny + nz + z] : 0.f;
-    }
-    const int last = T.ye;
-    int issued_hi = min(last, R.p0 + SR - 1);
-    int pend = R.p0;  // oldest plane no block-wide wait has confirmed yet
-    bool ok;
-    {
-        const bool mine = efm_mbar_wait(&bars[R.stage(R.p0)], R.parity(R.p0), err, wl) &&
-                          efm_mbar_wait(&bars[R.stage(T.ys)], R.parity(T.ys), err, wl);
-        ok = __syncthreads_and(mine) != 0;
-        if (ok) pend = T.ys + 1;
-    }
-    for (int j = T.ys; j < T.ye && ok; ++j) {
-        const bool plane_in = j >= EFM_HS && j < ny - EFM_HS && !(PASS == EFM_REV && (j < W || j >= ny - W));
-        const bool ypml = j < W || j >= ny - W;
-        const float cy_a = ypml ? I.cpml[2 * nx + j] : 0.f, cy_b = ypml ? I.cpml[2 * nx + ny + j] : 0.f;
-#pragma unroll
-        for (int h = 0; h < ROWS; ++h) {
-            cf[h].ay = cy_a;
-            cf[h].by = cy_b;
-        }
-        // the plane's update, with or without the memory-variable code
-        auto plane = [&](auto tag) -> bool {
-            constexpr bool PML = decltype(tag)::value;
-            PsiPlane P{0, 0, 0, false};
-            float pp[ROWS][9];
-            if (PML) {
-                P = psi_plane(H, j);
-#pragma unroll
-                for (int h = 0; h < ROWS; ++h)
-                    if (plane_in && rw[h].in) load_psi(H, P, rw[h], pp[h]);
-                if (j + 1 < T.ye) {
-                    const PsiPlane Pn = psi_plane(H, j + 1);
-#pragma unroll
-                    for (int h = 0; h < ROWS; ++h)
-                        if (rw[h].in) prefetch_psi(H, Pn, rw[h]);
+        if (has_src && p.in(v)) {
+            for (int s = 0; s < I.nsrc; ++s) {
+                if (p.x + v != I.sx[s] || y != I.sy[s] || p.z != I.sz[s]) continue;
+                if (PASS != EFM_ADJ) {
+                    const float w = I.wav[PASS == EFM_FWD ? it : I.nt - 1 - it];
+                    const float sg = PASS == EFM_FWD ? 1.f : -1.f;
+                    txx = __fadd_rn(txx, sg * __fmul_rn(I.mt[s][0], w));
+                    tyy = __fadd_rn(tyy, sg * __fmul_rn(I.mt[s][1], w));
+                    tzz = __fadd_rn(tzz, sg * __fmul_rn(I.mt[s][2], w));
+                    txy = __fadd_rn(txy, sg * __fmul_rn(I.mt[s][3], w));
+                    txz = __fadd_rn(txz, sg * __fmul_rn(I.mt[s][4], w));
+                    tyz = __fadd_rn(tyz, sg * __fmul_rn(I.mt[s][5], w));
+                } else if (I.mtg != nullptr) {
+                    const float w = I.wav[I.nt - 1 - it];
+                    const float f = __frcp_rn(2.f * mu0 * (3.f * lam + 2.f * mu0));
+                    const float lpm2 = 2.f * (lam + mu0);
+                    // one thread adds to these per step: a reduction in L2 need not wait for the old value
+                    double *g = I.mtg + 6 * s;
+                    atomicAdd(g + 0, (double)(w * (f * (lpm2 * txx - lam * tyy - lam * tzz))));
+                    atomicAdd(g + 1, (double)(w * (f * (lpm2 * tyy - lam * txx - lam * tzz))));
+                    atomicAdd(g + 2, (double)(w * (f * (lpm2 * tzz - lam * txx - lam * tyy))));
+                    atomicAdd(g + 3, (double)(w * (txy * __frcp_rn(mu_xy))));
+                    atomicAdd(g + 4, (double)(w * (txz * __frcp_rn(mu_xz))));
+                    atomicAdd(g + 5, (double)(w * (tyz * __frcp_rn(mu_yz))));
                 }
             }
-            const bool mine = efm_mbar_wait(&bars[R.stage(j + 1)], R.parity(j + 1), err, wl);
-            if (mine && plane_in) {
-                const int sm = R.stage(j - 1), s0 = R.stage(j), sp = R.stage(j + 1);
-#pragma unroll
-                for (int h = 0; h < ROWS; ++h)
-                    if (rw[h].in)
-                        stress_cell<PASS, ROWS, SR, PML>(I, R, sm, s0, sp, it, x, j, T.z0 + lr + 4 * h,
-                                                         rw[h], has_src, pp[h], cf[h], H, P);
-                efm_fence_async_smem();
-            }
-            return mine;
-        };
-        bool wpml = false;  // warp-uniform: some lane of this warp has memory variables here
-        if (PASS != EFM_REV) {
-            wpml = ypml;
-#pragma unroll
-            for (int h = 0; h < ROWS; ++h) wpml = wpml || rw[h].wx || rw[h].wz;
         }
-        const bool mine = wpml ? plane(Tag<true>{}) : plane(Tag<false>{});
-        ok = __syncthreads_and(mine) != 0;  // frees plane j-1's stage; uniform timeout exit
-        if (!ok) break;
-        pend = j + 2;
-        if ((int)threadIdx.x == iss)
-            advance<ROWS, SR, NH, NC>(R, tm, tm + NH + 1, 1, 6, plane_in, T.x0, T.z0, j, last);
-        if (j - 1 + SR <= last) issued_hi = j - 1 + SR;
+        o[0].v[v] = txx;
+        o[1].v[v] = tyy;
+        o[2].v[v] = tzz;
+        o[3].v[v] = txy;
+        o[4].v[v] = txz;
+        o[5].v[v] = tyz;
     }
-    if ((int)threadIdx.x == iss) efm_bulk_wait_all();
-    if (!ok) drain(R, pend, issued_hi);  // no load may still target this block's smem
+    vym = vy;
+    if (p.fl & F_PART) {  // a pair at the edge of the updated cells keeps the others' values
+#pragma unroll
+        for (int v = 0; v < VX; ++v)
+#pragma unroll
+            for (int q = 0; q < 6; ++q) o[q].v[v] = p.in(v) ? o[q].v[v] : t[q].v[v];
+    }
+    if (p.any_in()) {
+#pragma unroll
+        for (int q = 0; q < 6; ++q) stv(t0 + q * N, o[q]);
+    }
 }
 
-// halo fields: txx tzz txy txz tyz 1/rho ; center fields: tyy vx vy vz   (forward / adjoint);
-// the rebuild stores its new velocity through three more maps (tm[NH + NC ..]) into f.vo
-template <int PASS, int ROWS, int SR, bool ILLUM = false>
-__device__ __forceinline__ void velocity_body(const EfmInst *__restrict__ insts, int ninst, int it,
-                                              int block, unsigned char *smem) {
-    constexpr int NH = 6, NC = 4;
-    constexpr int CF = Ring<ROWS, SR>::CF;
-    __shared__ uint64_t bars[SR];
-    __shared__ int s_src;
-    __shared__ unsigned long long s_rec;
-    efm_pdl_trigger();
-    const EfmInst &I = insts[efm_find_inst(insts, ninst, block)];
-    if (it >= I.nsteps) return;
-    Tile T = stream_tile<ROWS>(I, block);
-    const int nx = I.nx, ny = I.ny, nz = I.nz, W = I.W;
-    if (PASS == EFM_REV && it >= 2) {
-        // the rebuild writes zeros outside the box x in [W, nx-W), y in [W, ny-W), z < nz-W;
-        // from the third step on both ping-pong buffers already hold them there (steps 0 and
-        // 1 wrote them), so only the box planes and the tiles reaching into the box are swept
-        T.ys = max(T.ys, W);
-        T.ye = min(T.ye, ny - W);
-        if (T.ys >= T.ye || T.z0 >= nz - W || T.x0 >= nx - W || T.x0 + EFM_STX <= W) return;
+template <int PASS, int NT, int D, int SLOT>
+__device__ __forceinline__ int stress_chunk(int packed, int ib, int it) {
+    Ctx<D, SLOT> X(packed);
+    const EfmInst &I = X.B.inst[ib];
+    const Chunk &T = X.B.chunk[ib];
+    constexpr int HB = efm_halo_s(NT);
+    const Pair p = make_pair<PASS == EFM_REV>(I, T);
+    const int ylo_in = I.W, yhi_in = I.ny - I.W, plane = I.nz * I.pitch;
+    const float k = I.k;
+    bool has_src = false;
+    for (int s = 0; s < I.nsrc; ++s)
+        has_src = has_src || (I.sx[s] >= T.x0 && I.sx[s] < T.x0 + T.tw && I.sz[s] >= T.z0 &&
+                              I.sz[s] < T.z0 + T.th && I.sy[s] >= T.ys && I.sy[s] < T.ye);
+    const int64_t N = I.vol;
+    float *t0 = I.f.t[0] + (int64_t)T.ys * plane + p.z * I.pitch + p.x;
+    Psi P = psi_at(I, p, 0, T.ys);
+    const int ye = T.ye;
+    efm_pdl_wait();
+    if (PASS != EFM_REV && T.ys >= EFM_HS) prefetch_first(I, p, P, 0, T.ys);
+    if (!__all_sync(0xffffffffu, X.wait())) return -1;
+    QV vym = ldv(X.slot() + HB, p.k0);
+    X.release();
+    for (int j = T.ys; j < ye; ++j, t0 += plane, P.x += P.sx, P.z += P.sz) {
+        const bool plane_in = j >= EFM_HS && j < ylo_in + yhi_in - EFM_HS;
+        const bool ypml = PASS != EFM_REV && (j < ylo_in || j >= yhi_in);
+        auto update = [&](auto tag) -> bool {
+            constexpr int PML = decltype(tag)::value;
+            PsiOld<PML, PASS == EFM_FWD> O;
+            float ay = 0.f, by = 0.f;
+            int py = 0;
+            if (PML) {
+                if (PML == 2 && ypml) {
+                    py = psi_y(I, p, 0, j);
+                    ay = I.cpml[2 * I.nx + j];
+                    by = I.cpml[2 * I.nx + I.ny + j];
+                }
+                O.load(p, P, ypml, py);
+                if (j + 1 < ye) {
+                    prefetch_psi(p, P);
+                    if (PML == 2 && ypml && (p.fl & F_IN) && (j + 1 < ylo_in || j >= yhi_in))
+                        prefetch2(P.base + (py + I.nz * I.nx));
+                }
+            }
+            if (!X.wait()) return false;
+            stress_pair<PASS, NT, PML>(I, X.prev(), X.slot(), X.slot() + HB, it, j, p, has_src, k, P, ypml, py, ay, by,
+                                       O, vym, t0, N);
+            return true;
+        };
+        bool mine;
+        if (!plane_in) {  // (a region that reaches past the updated planes)
+            mine = X.wait();
+            vym = ldv(X.prev() + efm_slot_xz(NT), p.i0);
+        } else {
+            mine = PASS != EFM_REV && (ypml || (p.fl & F_WZ)) ? update(Tag<2>{})
+                   : PASS != EFM_REV && (p.fl & F_WX)         ? update(Tag<1>{})
+                                                              : update(Tag<0>{});
+        }
+        if (!__all_sync(0xffffffffu, mine)) return -1;
+        X.release();
     }
-    const int lx = threadIdx.x % EFM_STX, lr = threadIdx.x / EFM_STX;
-    const int x = T.x0 + lx;
-    const CUtensorMap *tm = I.tmap;
-    Ring<ROWS, SR> R{smem, bars, NH * Ring<ROWS, SR>::HB + NC * Ring<ROWS, SR>::CB, NH, T.ys - 1};
-    const int iss = stream_issuer(T, nx, W);
-    stream_setup<ROWS, SR, NH, NC>(I, T, R, tm, &s_src, &s_rec, iss);
-    const unsigned long long recbits = s_rec;
-    unsigned int *const err = I.err;  // read once: the waits' clobbers would reload it
-    const uint32_t wl = I.wait_lim;
-    const Hot H = make_hot(I, 1);
-    float *const border = I.border;
-    float *const illum = ILLUM ? I.illum : nullptr;
-    const int64_t strip_n = I.strip_n;
-    const int by = ny - 2 * W, bx = nx - 2 * W, bz = nz - W - 2;
-    Row rw[ROWS];
-    make_rows<PASS, ROWS>(H, T, x, lx, lr, false, rw);
-    StripRow sr[ROWS];
-    bool colgrid[ROWS], zone_xz[ROWS];
-    float cz_a[ROWS], cz_b[ROWS];
-    const bool xpml = x < nx && (x < W || x >= nx - W);
-    const float cx_a = xpml ? I.cpml[x] : 0.f, cx_b = xpml ? I.cpml[nx + x] : 0.f;
+    return X.packed();
+}
+
+// ---------------------------------------------------------------------------- velocity
+// Boundary-strip slot of a box cell (xr, yr, zr from the box's corner) in one of its families
+// (efm_strip_slots_v): 0 the x faces, 1 the y faces, 2 the z faces.
+__device__ __forceinline__ int strip_slot(int bx, int by, int bz, int xr, int yr, int zr, int family) {
+    if (family == 0) return ((xr < 2 ? xr : 4 + xr - bx) * by + yr) * bz + zr;
+    if (family == 1) return 4 * by * bz + ((yr < 2 ? yr : 4 + yr - by) * bz + zr) * bx + xr;
+    return 4 * by * bz + 4 * bz * bx + ((zr < 2 ? zr : 4 + zr - bz) * by + yr) * bx + xr;
+}
+
+// Neighbour fields: txx (x0, z0; tw+4 columns), tzz (th+1 rows), txy (x0-4; tw+4), txz (x0-4, z0-1;
+// both), tyz (z0-1; th+1), 1/rho (x0, z0; both), tyy (cells); cell fields: vx vy vz.  First slot's
+// cell part: txy and tyz of the plane before the chunk.
+template <int NT>
+struct VOff {
+    static constexpr int X = efm_slot_x(NT), Z = efm_slot_z(NT), XZ = efm_slot_xz(NT), CF = efm_slot_c(NT);
+    static constexpr int txx = 0, tzz = X, txy = X + Z, txz = 2 * X + Z, tyz = 2 * X + Z + XZ,
+                         bu = 2 * X + 2 * Z + XZ, tyy = 2 * X + 2 * Z + 2 * XZ;
+};
+
+// The stress differences' operands and the buoyancies of the pair on one plane.
+struct VelIn {
+    QV txx, tzz, tzzk, txy, txz, txzk, tyz, tyzk, tyy, tyyj, b0, bk, bj;
+    float txxi, txym, txzm, bi;
+};
+
+template <int NT>
+__device__ __forceinline__ VelIn velocity_in(const Pair &p, const unsigned char *h, const unsigned char *hn) {
+    using O = VOff<NT>;
+    const int i0 = p.i0, i1 = p.i0 + p.hp, k0 = p.k0, k1 = p.k0 + p.tw;
+    VelIn a;
+    a.txx = ldv(h + O::txx, i0);
+    a.txxi = ld1(h + O::txx, i0 + VX);
+    a.tzz = ldv(h + O::tzz, k0);
+    a.tzzk = ldv(h + O::tzz, k1);
+    a.txy = ldv(h + O::txy, i0 + 4);
+    a.txym = ld1(h + O::txy, i0 + 3);
+    a.txz = ldv(h + O::txz, i1 + 4);
+    a.txzm = ld1(h + O::txz, i1 + 3);
+    a.txzk = ldv(h + O::txz, i0 + 4);
+    a.tyz = ldv(h + O::tyz, k1);
+    a.tyzk = ldv(h + O::tyz, k0);
+    a.b0 = ldv(h + O::bu, i0);
+    a.bi = ld1(h + O::bu, i0 + VX);
+    a.bk = ldv(h + O::bu, i1);
+    a.bj = ldv(hn + O::bu, i0);
+    a.tyy = ldv(h + O::tyy, k0);
+    a.tyyj = ldv(hn + O::tyy, k0);
+    return a;
+}
+
+template <int PASS, int NT, int D, int SLOT, bool ILLUM, bool YZ>
+__device__ __forceinline__ int velocity_chunk(int packed, int ib, int it) {
+    using OF = VOff<NT>;
+    Ctx<D, SLOT> X(packed);
+    const EfmInst &I = X.B.inst[ib];
+    const Chunk &T = X.B.chunk[ib];
+    constexpr int HB = efm_halo_v(NT);
+    const Pair p = make_pair<false>(I, T);
+    const int ylo_in = I.W, yhi_in = I.ny - I.W, plane = I.nz * I.pitch;
+    const float k = I.k;
+    // strips: which cells lie in the box (bit v), next to an x face (4 + v) or a z face (8)
+    int sf = 0;
+    if (PASS == EFM_REV || (PASS == EFM_FWD && I.border != nullptr)) {
+        const int bx = I.nx - 2 * I.W, bz = I.nz - I.W - 2, zr = p.z - 2;
 #pragma unroll
-    for (int h = 0; h < ROWS; ++h) {
-        const int z = T.z0 + lr + 4 * h;
-        colgrid[h] = x < nx && z < nz;
-        zone_xz[h] = x < W || x >= nx - W || z >= nz - W;
-        sr[h] = strip_row(nx, nz, by, W, x, z);
-        const bool zpml = z < nz && z >= nz - W;
-        cz_a[h] = zpml ? I.cpml[2 * nx + 2 * ny + z] : 0.f;
-        cz_b[h] = zpml ? I.cpml[2 * nx + 2 * ny + nz + z] : 0.f;
+        for (int v = 0; v < VX; ++v) {
+            const int xr = p.x + v - I.W;
+            if (!p.act(v) || xr < 0 || xr >= bx || zr < 0 || zr >= bz) continue;
+            sf |= 1 << v;
+            if (xr < 2 || xr >= bx - 2) sf |= 16 << v;
+            if (zr < 2 || zr >= bz - 2) sf |= 256;
+        }
     }
-    const CUtensorMap *stm = PASS == EFM_REV ? tm + NH + NC : tm + NH + 1;
-    const int last = T.ye;
-    int issued_hi = min(last, R.p0 + SR - 1);
-    int pend = R.p0;  // oldest plane no block-wide wait has confirmed yet
-    bool ok;
-    {
-        bool mine = efm_mbar_wait(&bars[R.stage(R.p0)], R.parity(R.p0), err, wl) &&
-                    efm_mbar_wait(&bars[R.stage(T.ys)], R.parity(T.ys), err, wl);
-        ok = __syncthreads_and(mine) != 0;
-        if (ok) pend = T.ys + 1;
-    }
-    for (int j = T.ys; j < T.ye && ok; ++j) {
-        const int y = j;
-        const bool plane_in = j >= EFM_HS && j < ny - EFM_HS;
-        const bool rec_plane = (recbits >> (j - T.ys)) & 1ull;
-        const bool ypml = j < W || j >= ny - W;
-        const float cy_a = ypml ? I.cpml[2 * nx + j] : 0.f, cy_b = ypml ? I.cpml[2 * nx + ny + j] : 0.f;
-        // plane terms of the strip slots
-        const int yr = j - W;
-        const bool yin = yr >= 0 && yr < by;
-        const int yrow = yr < 2 ? yr : (yr >= by - 2 ? 2 + (yr - (by - 2)) : -1);
-        const bool store = PASS == EFM_REV || plane_in || rec_plane;
+    const int64_t N = I.vol;
+    float *v0 = I.f.vo[0] + (int64_t)T.ys * plane + p.z * I.pitch + p.x;
+    const uint8_t *const recs = PASS == EFM_REV ? nullptr : I.rec_col + (int64_t)T.col * I.ny;
+    Psi P = psi_at(I, p, 1, T.ys);
+    uint8_t rec_now = PASS == EFM_REV ? 0 : __ldg(recs + T.ys);
+    const int ye = T.ye;
+    efm_pdl_wait();
+    if (PASS != EFM_REV && T.ys >= EFM_HS) prefetch_first(I, p, P, 1, T.ys);
+    if (!__all_sync(0xffffffffu, X.wait())) return -1;
+    QV txym = ldv(X.slot() + HB, p.k0), tyzm = ldv(X.slot() + HB + OF::CF, p.k0);
+    X.release();
+    for (int j = T.ys; j < ye; ++j, v0 += plane, P.x += P.sx, P.z += P.sz) {
+        const bool plane_in = j >= EFM_HS && j < yhi_in + ylo_in - EFM_HS;
+        const bool ypml = j < ylo_in || j >= yhi_in;
+        // the plane is one of the outer two of the box on either side of y (strips)
+        const bool yface = !ypml && (j < ylo_in + 2 || j >= yhi_in - 2);
         bool mine;
         if (PASS == EFM_REV) {
             // reverse rebuild (-dt, no CPML) into the ping-pong partner f.vo: CPML slabs -> 0,
             // boundary strips -> the values saved at forward step nt-2-it (:1955-1960),
             // box interior -> stencil update, never-updated cells -> 0.  The strip values of
-            // this plane are requested before the stage wait, the next plane's pulled into L1.
-            const float *sv = border + (int64_t)(I.nt - 2 - it) * 3 * strip_n;
-            // first strip slot of row h on plane y (its three families hold the same values)
-            auto slot_of = [&](int h, int y) -> int {
-                const int r = y - W;
-                if (zone_xz[h] || y < W || y >= ny - W || r >= by || sr[h].yf < 0) return -1;
-                if (sr[h].xf >= 0) return sr[h].xf + r * bz;
-                const int row = r < 2 ? r : (r >= by - 2 ? 2 + (r - (by - 2)) : -1);
-                if (row >= 0) return sr[h].yf + row * bz * bx;
-                if (sr[h].zf >= 0) return sr[h].zf + r * bx;
-                return -1;
-            };
-            int slot[ROWS];
-            float sval[ROWS][3];
+            // this plane are requested before the wait.
+            int slot[VX];
+            float sval[VX][3];
+            const bool strips = !ypml && (sf & (yface ? 15 : (15 << 4) | 256)) != 0;
 #pragma unroll
-            for (int h = 0; h < ROWS; ++h) {
-                slot[h] = colgrid[h] ? slot_of(h, j) : -1;
-                if (slot[h] >= 0) {
-                    sval[h][0] = sv[slot[h]];
-                    sval[h][1] = sv[strip_n + slot[h]];
-                    sval[h][2] = sv[2 * strip_n + slot[h]];
-                }
-                const int sn = j + 1 < T.ye && colgrid[h] ? slot_of(h, j + 1) : -1;
-                if (sn >= 0) {
-                    asm volatile("prefetch.global.L1 [%0];" ::"l"(sv + sn));
-                    asm volatile("prefetch.global.L1 [%0];" ::"l"(sv + strip_n + sn));
-                    asm volatile("prefetch.global.L1 [%0];" ::"l"(sv + 2 * strip_n + sn));
+            for (int v = 0; v < VX; ++v) slot[v] = -1;
+            if (strips) {
+                const int W = I.W, by = I.ny - 2 * W, bx = I.nx - 2 * W, bz = I.nz - W - 2;
+                const float *sv = I.border + (int64_t)(I.nt - 2 - it) * 3 * I.strip_n;
+                const int64_t strip_n = I.strip_n;
+#pragma unroll
+                for (int v = 0; v < VX; ++v) {
+                    const bool xf = sf & (16 << v);
+                    if (!(sf & (1 << v)) || !(xf || yface || (sf & 256))) continue;
+                    // (a cell's families hold the same values)
+                    slot[v] = strip_slot(bx, by, bz, p.x + v - W, j - W, p.z - 2, xf ? 0 : yface ? 1 : 2);
+                    sval[v][0] = sv[slot[v]];
+                    sval[v][1] = sv[strip_n + slot[v]];
+                    sval[v][2] = sv[2 * strip_n + slot[v]];
                 }
             }
-            mine = efm_mbar_wait(&bars[R.stage(j + 1)], R.parity(j + 1), err, wl);
+            mine = X.wait();
             if (mine) {
-                const int s0 = R.stage(j), sp = R.stage(j + 1), sm = R.stage(j - 1);
+                const VelIn a = velocity_in<NT>(p, X.prev(), X.slot());
+                QV old[3], o[3];
 #pragma unroll
-                for (int h = 0; h < ROWS; ++h) {
-                    if (!colgrid[h]) continue;
-                    const int hi = rw[h].hidx, ci = rw[h].cidx;
-                    float nvx = 0.f, nvy = 0.f, nvz = 0.f;
-                    const bool zone = zone_xz[h] || ypml;
-                    if (slot[h] >= 0) {
-                        nvx = sval[h][0];
-                        nvy = sval[h][1];
-                        nvz = sval[h][2];
-                    } else if (!zone && plane_in && rw[h].in) {
-                        const float *t0 = R.halo(s0, 0), *t2 = R.halo(s0, 1), *t3 = R.halo(s0, 2);
-                        const float *t4 = R.halo(s0, 3), *t5 = R.halo(s0, 4), *bu = R.halo(s0, 5);
-                        const float *c0 = R.center(s0, 0) + ci;
-                        const float dtxx_dx = t0[hi + 1] - t0[hi];
-                        const float dtzz_dz = t2[hi + EFM_HX] - t2[hi];
-                        const float dtyy_dy = R.center(sp, 0)[ci] - c0[0];
-                        const float txyc = t3[hi], txzc = t4[hi], tyzc = t5[hi];
-                        const float dtxy_dy = txyc - R.halo(sm, 2)[hi];
-                        const float dtxy_dx = txyc - t3[hi - 1];
-                        const float dtxz_dz = txzc - t4[hi - EFM_HX];
-                        const float dtxz_dx = txzc - t4[hi - 1];
-                        const float dtyz_dz = tyzc - t5[hi - EFM_HX];
-                        const float dtyz_dy = tyzc - R.halo(sm, 4)[hi];
-                        const float b0 = bu[hi], bi = bu[hi + 1], bk = bu[hi + EFM_HX];
-                        const float bj = R.halo(sp, 5)[hi];
-                        const float b_x = 2.f * b0 * bi * frcp(b0 + bi);
-                        const float b_y = 2.f * b0 * bj * frcp(b0 + bj);
-                        const float b_z = 2.f * b0 * bk * frcp(b0 + bk);
-                        const float k = H.k;
-                        nvx = c0[CF] + k * b_x * (dtxx_dx + dtxy_dy + dtxz_dz);
-                        nvy = c0[2 * CF] + k * b_y * (dtxy_dx + dtyy_dy + dtyz_dz);
-                        nvz = c0[3 * CF] + k * b_z * (dtxz_dx + dtyz_dy + dtzz_dz);
-                    }
-                    float *cw = R.center(s0, 1) + ci;
-                    cw[0] = nvx;
-                    cw[CF] = nvy;
-                    cw[2 * CF] = nvz;
+                for (int c = 0; c < 3; ++c) old[c] = ldv(X.slot() + HB + c * OF::CF, p.k0);
+#pragma unroll
+                for (int v = 0; v < VX; ++v) {
+                    const float dtxx_dx = (v < VX - 1 ? a.txx.v[v + 1] : a.txxi) - a.txx.v[v];
+                    const float dtzz_dz = a.tzzk.v[v] - a.tzz.v[v];
+                    const float dtyy_dy = a.tyyj.v[v] - a.tyy.v[v];
+                    const float txyc = a.txy.v[v], txzc = a.txz.v[v], tyzc = a.tyz.v[v];
+                    const float dtxy_dy = txyc - txym.v[v];
+                    const float dtxy_dx = txyc - (v ? a.txy.v[v - 1] : a.txym);
+                    const float dtxz_dz = txzc - a.txzk.v[v];
+                    const float dtxz_dx = txzc - (v ? a.txz.v[v - 1] : a.txzm);
+                    const float dtyz_dz = tyzc - a.tyzk.v[v];
+                    const float dtyz_dy = tyzc - tyzm.v[v];
+                    const float b0 = a.b0.v[v], bi = v < VX - 1 ? a.b0.v[v + 1] : a.bi, bk = a.bk.v[v];
+                    const float bj = a.bj.v[v];
+                    const float b_x = 2.f * b0 * bi * frcp(b0 + bi);
+                    const float b_y = 2.f * b0 * bj * frcp(b0 + bj);
+                    const float b_z = 2.f * b0 * bk * frcp(b0 + bk);
+                    const float nvx = old[0].v[v] + k * b_x * (dtxx_dx + dtxy_dy + dtxz_dz);
+                    const float nvy = old[1].v[v] + k * b_y * (dtxy_dx + dtyy_dy + dtyz_dz);
+                    const float nvz = old[2].v[v] + k * b_z * (dtxz_dx + dtyz_dy + dtzz_dz);
+                    const bool in = (sf & (1 << v)) && !ypml && plane_in && p.in(v);
+                    o[0].v[v] = in ? nvx : 0.f;
+                    o[1].v[v] = in ? nvy : 0.f;
+                    o[2].v[v] = in ? nvz : 0.f;
                 }
-                efm_fence_async_smem();
+                if (strips) {
+#pragma unroll
+                    for (int v = 0; v < VX; ++v)
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) o[c].v[v] = slot[v] >= 0 ? sval[v][c] : o[c].v[v];
+                }
+                txym = a.txy;
+                tyzm = a.tyz;
+                if (p.fl & F_ACT) {
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) stv(v0 + c * N, o[c]);
+                }
             }
         } else {
-            // forward / adjoint: the plane's update, with or without the memory-variable code
-            auto plane = [&](auto tag, auto rtag) -> bool {
-                constexpr bool PML = decltype(tag)::value;
-                constexpr bool REC = decltype(rtag)::value;  // this plane of the tile has receivers
-                PsiPlane P{0, 0, 0, false};
-                float pp[ROWS][9];
+            const bool rec_plane = rec_now != 0;
+            if (j + 1 < ye) rec_now = __ldg(recs + j + 1);
+            // the plane's update (see Tag)
+            auto update = [&](auto tag) -> bool {
+                constexpr int PML = decltype(tag)::value;
+                constexpr bool REC = PML == 2;
+                PsiOld<PML, YZ> O;
+                float ay = 0.f, by_ = 0.f;
+                int py = 0;
                 if (PML) {
-                    P = psi_plane(H, j);
-#pragma unroll
-                    for (int h = 0; h < ROWS; ++h)
-                        if (plane_in && rw[h].in) load_psi(H, P, rw[h], pp[h]);
-                    if (j + 1 < T.ye) {
-                        const PsiPlane Pn = psi_plane(H, j + 1);
-#pragma unroll
-                        for (int h = 0; h < ROWS; ++h)
-                            if (rw[h].in) prefetch_psi(H, Pn, rw[h]);
+                    if (PML == 2 && ypml) {
+                        py = psi_y(I, p, 1, j);
+                        ay = I.cpml[2 * I.nx + j];
+                        by_ = I.cpml[2 * I.nx + I.ny + j];
+                    }
+                    if (plane_in) O.load(p, P, ypml, py);
+                    if (j + 1 < ye) {
+                        prefetch_psi(p, P);
+                        if (PML == 2 && ypml && (p.fl & F_IN) && (j + 1 < ylo_in || j >= yhi_in))
+                            prefetch2(P.base + (py + I.nz * I.nx));
                     }
                 }
-                const bool mine = efm_mbar_wait(&bars[R.stage(j + 1)], R.parity(j + 1), err, wl);
-                if (!mine) return false;
-                const int sm = R.stage(j - 1), s0 = R.stage(j), sp = R.stage(j + 1);
+                int rq[VX];
+                bool more[VX];  // the cell may hold several receivers
 #pragma unroll
-                for (int h = 0; h < ROWS; ++h) {
-                    const int z = T.z0 + lr + 4 * h;
-                    const bool guard = plane_in && rw[h].in;
-                    bool more = false;  // the cell may hold several receivers
-                    const int rq = REC && colgrid[h] ? efm_rec_first(I, x, y, z, &more) : -1;
-                    const bool rec = rq >= 0;
-                    if (!(guard || rec)) continue;
-                    const int hi = rw[h].hidx, ci = rw[h].cidx;
-                    float *cw = R.center(s0, 1) + ci;  // vx, vy, vz of this cell
-                    float nvx = cw[0];
-                    float nvy = cw[CF];
-                    float nvz = cw[2 * CF];
-                    if (guard) {
-                        const float *t0 = R.halo(s0, 0), *t2 = R.halo(s0, 1), *t3 = R.halo(s0, 2);
-                        const float *t4 = R.halo(s0, 3), *t5 = R.halo(s0, 4), *bu = R.halo(s0, 5);
-                        const float dtxx_dx = t0[hi + 1] - t0[hi];
-                        const float dtzz_dz = t2[hi + EFM_HX] - t2[hi];
-                        const float dtyy_dy = R.center(sp, 0)[ci] - cw[-CF];
-                        const float txyc = t3[hi], txzc = t4[hi], tyzc = t5[hi];
-                        const float dtxy_dy = txyc - R.halo(sm, 2)[hi];
-                        const float dtxy_dx = txyc - t3[hi - 1];
-                        const float dtxz_dz = txzc - t4[hi - EFM_HX];
-                        const float dtxz_dx = txzc - t4[hi - 1];
-                        const float dtyz_dz = tyzc - t5[hi - EFM_HX];
-                        const float dtyz_dy = tyzc - R.halo(sm, 4)[hi];
-                        const float *p9 = pp[h];
-                        float q1 = 0.f, q2 = 0.f, q3 = 0.f, q4 = 0.f, q5 = 0.f, q6 = 0.f, q7 = 0.f,
-                              q8 = 0.f, q9 = 0.f;
-                        if (PML && rw[h].wx && rw[h].pxo >= 0) {
-                            const float a = cx_a, b = cx_b;
-                            q1 = b * p9[0] + a * dtxx_dx;
-                            q2 = b * p9[1] + a * dtxy_dx;
-                            q3 = b * p9[2] + a * dtxz_dx;
-                            H.psx[P.x + rw[h].pxo] = make_float4(q1, q2, q3, 0.f);
-                        }
-                        if (PML && P.has_y) {
-                            const float a = cy_a, b = cy_b;
-                            q4 = b * p9[3] + a * dtyy_dy;
-                            q5 = b * p9[4] + a * dtxy_dy;
-                            q6 = b * p9[5] + a * dtyz_dy;
-                            H.psy[P.y + rw[h].pyo] = make_float4(q4, q5, q6, 0.f);
-                        }
-                        if (PML && rw[h].wz && rw[h].pzo >= 0) {
-                            const float a = cz_a[h], b = cz_b[h];
-                            q7 = b * p9[6] + a * dtzz_dz;
-                            q8 = b * p9[7] + a * dtxz_dz;
-                            q9 = b * p9[8] + a * dtyz_dz;
-                            H.psz[P.z + rw[h].pzo] = make_float4(q7, q8, q9, 0.f);
-                        }
-                        // harmonic 2-point buoyancy from the precomputed 1/rho (:153-159)
-                        const float b0 = bu[hi], bi = bu[hi + 1], bk = bu[hi + EFM_HX];
-                        const float bj = R.halo(sp, 5)[hi];
-                        const float b_x = 2.f * b0 * bi * frcp(b0 + bi);
-                        const float b_y = 2.f * b0 * bj * frcp(b0 + bj);
-                        const float b_z = 2.f * b0 * bk * frcp(b0 + bk);
-                        const float k = H.k;
-                        nvx = nvx + k * b_x * ((dtxx_dx + q1) + (dtxy_dy + q5) + (dtxz_dz + q8));
-                        nvy = nvy + k * b_y * ((dtxy_dx + q2) + (dtyy_dy + q4) + (dtyz_dz + q9));
-                        nvz = nvz + k * b_z * ((dtxz_dx + q3) + (dtyz_dy + q6) + (dtzz_dz + q7));
+                for (int v = 0; v < VX; ++v) {
+                    rq[v] = -1;
+                    more[v] = false;
+                    if (REC && rec_plane && p.act(v)) rq[v] = efm_rec_first(I, p.x + v, j, p.z, &more[v]);
+                }
+                if (!X.wait()) return false;
+                const VelIn a = velocity_in<NT>(p, X.prev(), X.slot());
+                QV old[3], o[3];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) old[c] = ldv(X.slot() + HB + c * OF::CF, p.k0);
+#pragma unroll
+                for (int v = 0; v < VX; ++v) {
+                    const float dtxx_dx = (v < VX - 1 ? a.txx.v[v + 1] : a.txxi) - a.txx.v[v];
+                    const float dtzz_dz = a.tzzk.v[v] - a.tzz.v[v];
+                    const float dtyy_dy = a.tyyj.v[v] - a.tyy.v[v];
+                    const float txyc = a.txy.v[v], txzc = a.txz.v[v], tyzc = a.tyz.v[v];
+                    const float dtxy_dy = txyc - txym.v[v];
+                    const float dtxy_dx = txyc - (v ? a.txy.v[v - 1] : a.txym);
+                    const float dtxz_dz = txzc - a.txzk.v[v];
+                    const float dtxz_dx = txzc - (v ? a.txz.v[v - 1] : a.txzm);
+                    const float dtyz_dz = tyzc - a.tyzk.v[v];
+                    const float dtyz_dy = tyzc - tyzm.v[v];
+                    // harmonic 2-point buoyancy from the precomputed 1/rho (:153-159)
+                    const float b0 = a.b0.v[v], bi = v < VX - 1 ? a.b0.v[v + 1] : a.bi, bk = a.bk.v[v];
+                    const float bj = a.bj.v[v];
+                    const float b_x = 2.f * b0 * bi * frcp(b0 + bi);
+                    const float b_y = 2.f * b0 * bj * frcp(b0 + bj);
+                    const float b_z = 2.f * b0 * bk * frcp(b0 + bk);
+                    if (PML == 0) {  // (the sums below without their zero terms)
+                        o[0].v[v] = old[0].v[v] + k * b_x * (dtxx_dx + dtxy_dy + dtxz_dz);
+                        o[1].v[v] = old[1].v[v] + k * b_y * (dtxy_dx + dtyy_dy + dtyz_dz);
+                        o[2].v[v] = old[2].v[v] + k * b_z * (dtxz_dx + dtyz_dy + dtzz_dz);
+                        continue;
                     }
-                    if (PASS == EFM_ADJ && rec) {
-                        const int tr = I.nt - 1 - it;
+                    float q1 = 0.f, q2 = 0.f, q3 = 0.f, q4 = 0.f, q5 = 0.f, q6 = 0.f, q7 = 0.f, q8 = 0.f, q9 = 0.f;
+                    if (PML && plane_in) {
+                        if (PML == 1 || (p.fl & F_WX)) {
+                            psi_step(p.px(v), P.base + (P.x + v), O.x[v], P.ax[v], P.bx[v], dtxx_dx, dtxy_dx, dtxz_dx);
+                            q1 = O.x[v][0];
+                            q2 = O.x[v][1];
+                            q3 = O.x[v][2];
+                        }
+                        float oy[3], oz[3];
+                        if (PML == 2 && ypml) {
+                            psi_step_yz<O.EARLY>(p.in(v), P.base + (py + v), oy, O.y[O.EARLY ? v : 0], ay, by_,
+                                                 dtyy_dy, dtxy_dy, dtyz_dy);
+                            q4 = oy[0];
+                            q5 = oy[1];
+                            q6 = oy[2];
+                        }
+                        if (PML == 2 && (p.fl & F_WZ)) {
+                            psi_step_yz<O.EARLY>((p.fl & F_PZ) && p.in(v), P.base + (P.z + v), oz, O.z[O.EARLY ? v : 0],
+                                                 P.az, P.bz, dtzz_dz, dtxz_dz, dtyz_dz);
+                            q7 = oz[0];
+                            q8 = oz[1];
+                            q9 = oz[2];
+                        }
+                    }
+                    o[0].v[v] = old[0].v[v] + k * b_x * ((dtxx_dx + q1) + (dtxy_dy + q5) + (dtxz_dz + q8));
+                    o[1].v[v] = old[1].v[v] + k * b_y * ((dtxy_dx + q2) + (dtyy_dy + q4) + (dtyz_dz + q9));
+                    o[2].v[v] = old[2].v[v] + k * b_z * ((dtxz_dx + q3) + (dtyz_dy + q6) + (dtzz_dz + q7));
+                }
+                txym = a.txy;
+                tyzm = a.tyz;
+                // cells the stencil does not update keep their values
+                if (!plane_in || (p.fl & F_PART) || REC) {
+#pragma unroll
+                    for (int v = 0; v < VX; ++v) {
+                        const bool guard = plane_in && p.in(v);
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) o[c].v[v] = guard ? o[c].v[v] : old[c].v[v];
+                    }
+                }
+                bool any = plane_in && p.any_in();
+                if (REC && rec_plane) {
+#pragma unroll
+                    for (int v = 0; v < VX; ++v) {
+                        if (rq[v] < 0) continue;
                         const int64_t ntr = (int64_t)I.nt * I.nrec;
-                        const int c = x + nx * (z + nz * y);
-                        for (int q = rq;;) {
-                            const int64_t o = (int64_t)tr * I.nrec + I.rec_id[q];
-                            nvx = __fadd_rn(nvx, I.res[o]);
-                            nvy = __fadd_rn(nvy, I.res[ntr + o]);
-                            nvz = __fadd_rn(nvz, I.res[2 * ntr + o]);
-                            if (!more || ++q >= I.nrec || I.rec_lin[q] != c) break;
-                        }
-                    }
-                    cw[0] = nvx;
-                    cw[CF] = nvy;
-                    cw[2 * CF] = nvz;
-                    if (PASS == EFM_FWD) {
-                        // cells the stencil never updates keep v = 0 and add nothing
-                        if (ILLUM && guard)
-                            illum[x + nx * (z + nz * y)] += nvx * nvx + nvy * nvy + nvz * nvz;
-                        if (rec && I.gather != nullptr) {
-                            const int64_t ntr = (int64_t)I.nt * I.nrec;
-                            const int c = x + nx * (z + nz * y);
-                            for (int q = rq;;) {
-                                const int64_t o = (int64_t)it * I.nrec + I.rec_id[q];
-                                I.gather[o] = nvx;
-                                I.gather[ntr + o] = nvy;
-                                I.gather[2 * ntr + o] = nvz;
-                                if (!more || ++q >= I.nrec || I.rec_lin[q] != c) break;
+                        const int c = p.x + v + I.nx * (p.z + I.nz * j);
+                        if (PASS == EFM_ADJ) {
+                            any = true;
+                            for (int q = rq[v];;) {
+                                const int64_t e = (int64_t)(I.nt - 1 - it) * I.nrec + I.rec_id[q];
+                                o[0].v[v] = __fadd_rn(o[0].v[v], I.res[e]);
+                                o[1].v[v] = __fadd_rn(o[1].v[v], I.res[ntr + e]);
+                                o[2].v[v] = __fadd_rn(o[2].v[v], I.res[2 * ntr + e]);
+                                if (!more[v] || ++q >= I.nrec || I.rec_lin[q] != c) break;
+                            }
+                        } else if (I.gather != nullptr) {
+                            for (int q = rq[v];;) {
+                                const int64_t e = (int64_t)it * I.nrec + I.rec_id[q];
+                                I.gather[e] = o[0].v[v];
+                                I.gather[ntr + e] = o[1].v[v];
+                                I.gather[2 * ntr + e] = o[2].v[v];
+                                if (!more[v] || ++q >= I.nrec || I.rec_lin[q] != c) break;
                             }
                         }
-                        if (border != nullptr && yin && sr[h].yf >= 0) {
-                            float *s = border + (int64_t)it * 3 * strip_n;
-                            auto put = [&](int sl) {
-                                s[sl] = nvx;
-                                s[strip_n + sl] = nvy;
-                                s[2 * strip_n + sl] = nvz;
-                            };
-                            if (sr[h].xf >= 0) put(sr[h].xf + yr * bz);
-                            if (yrow >= 0) put(sr[h].yf + yrow * bz * bx);
-                            if (sr[h].zf >= 0) put(sr[h].zf + yr * bx);
+                    }
+                }
+                if (any) {
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) stv(v0 + c * N, o[c]);
+                }
+                if (PASS == EFM_FWD) {
+                    if (ILLUM && plane_in) {
+#pragma unroll
+                        for (int v = 0; v < VX; ++v) {
+                            const float nvx = o[0].v[v], nvy = o[1].v[v], nvz = o[2].v[v];
+                            if (p.in(v))
+                                I.illum[p.x + v + I.nx * (p.z + I.nz * j)] += nvx * nvx + nvy * nvy + nvz * nvz;
+                        }
+                    }
+                    // the strips the pair's box cells belong to (sf is zero without strips)
+                    if (!ypml && (sf & (yface ? 15 : (15 << 4) | 256))) {
+                        const int W = I.W, by = I.ny - 2 * W, bx = I.nx - 2 * W, bz = I.nz - W - 2;
+                        float *s = I.border + (int64_t)it * 3 * I.strip_n;
+                        const int64_t strip_n = I.strip_n;
+#pragma unroll
+                        for (int f = 0; f < 3; ++f) {
+                            if (!(f == 0 ? (sf & (15 << 4)) != 0 : f == 1 ? yface : (sf & 256) != 0)) continue;
+#pragma unroll
+                            for (int v = 0; v < VX; ++v) {
+                                if (!(sf & ((f == 0 ? 16 : 1) << v))) continue;
+                                float *e = s + strip_slot(bx, by, bz, p.x + v - W, j - W, p.z - 2, f);
+                                st1(e, o[0].v[v]);
+                                st1(e + strip_n, o[1].v[v]);
+                                st1(e + 2 * strip_n, o[2].v[v]);
+                            }
                         }
                     }
                 }
-                if (store) efm_fence_async_smem();
                 return true;
             };
-            bool wpml = ypml;  // warp-uniform: some lane of this warp has memory variables here
-#pragma unroll
-            for (int h = 0; h < ROWS; ++h) wpml = wpml || rw[h].wx || rw[h].wz;
-            // four instantiations: the receiver code only runs on the few planes that hold
-            // receivers of this tile (block-uniform), the CPML code in the warps that need it
-            if (rec_plane)
-                mine = wpml ? plane(Tag<true>{}, Tag<true>{}) : plane(Tag<false>{}, Tag<true>{});
-            else
-                mine = wpml ? plane(Tag<true>{}, Tag<false>{}) : plane(Tag<false>{}, Tag<false>{});
+            mine = ypml || rec_plane || (p.fl & F_WZ) ? update(Tag<2>{})
+                   : p.fl & F_WX                      ? update(Tag<1>{})
+                                                      : update(Tag<0>{});
         }
-        ok = __syncthreads_and(mine) != 0;
-        if (!ok) break;
-        pend = j + 2;
-        if ((int)threadIdx.x == iss)
-            advance<ROWS, SR, NH, NC>(R, tm, stm, 1, 3, store, T.x0, T.z0, j, last);
-        if (j - 1 + SR <= last) issued_hi = j - 1 + SR;
+        if (!__all_sync(0xffffffffu, mine)) return -1;
+        X.release();
     }
-    if ((int)threadIdx.x == iss) efm_bulk_wait_all();
-    if (!ok) drain(R, pend, issued_hi);
+    return X.packed();
 }
 
-template <int PASS, int ROWS, int SR>
-__global__ void __launch_bounds__(EFM_STHREADS, efm_stream_blocks(ROWS, SR))
-efm_stress_stream(const EfmInst *__restrict__ insts, int ninst, int it) {
-    extern __shared__ __align__(1024) unsigned char smem[];
-    stress_body<PASS, ROWS, SR>(insts, ninst, it, blockIdx.x, smem);
+// ----------------------------------------------------------------------------- imaging
+// Zero-lag imaging of a reverse step (kernel_Gradients_Rho/Lambda/Mu, :191-294): fV_present (the
+// forward velocity before the rebuild step), fV (after it), the adjoint fields after the adjoint
+// step, into the lambda / mu / rho gradients.  Neighbour fields: fV_present vx (x0-4, z0), vy (x0,
+// z0), vz (x0, z0-2; two rows below), 1/mu (x0, z0); cell fields: fV vx vy vz, adjoint vx vy vz,
+// lambda.  The adjoint stresses (in L2 from the velocity pass) and the gradients are requested
+// with plain loads before the plane's wait.  First slot's cell part: fV_present vy of the two
+// planes before the chunk.
+template <int NT>
+struct IOff {
+    static constexpr int XZ = efm_slot_xz(NT), CF = efm_slot_c(NT);
+    static constexpr int px = 0, py = XZ, rm = 2 * XZ, pz = 3 * XZ;
+};
+
+template <int NT, int D, int SLOT>
+__device__ __forceinline__ int image_chunk(int packed, int ib) {
+    using O = IOff<NT>;
+    Ctx<D, SLOT> X(packed);
+    const EfmInst &I = X.B.inst[ib];
+    const Chunk &T = X.B.chunk[ib];
+    constexpr int HB = efm_halo_i(NT), CF = O::CF;
+    const Pair p = make_pair<false>(I, T);
+    const int plane = I.nz * I.pitch, gplane = I.nz * I.nx;
+    const int64_t N = I.vol;
+    const float *bt = I.bt[0] + (int64_t)T.ys * plane + p.z * I.pitch + p.x;
+    int64_t go = (int64_t)T.ys * gplane + p.z * I.nx + p.x;
+    float *const g_[3] = {I.g_lam, I.g_mu, I.g_rho};
+    const bool vec = I.gvec;  // 8-byte gradient rows
+    const float idt = I.inv_dt, idx = I.inv_dx;
+    const int ye = T.ye, jlo = EFM_HS, jhi = I.ny - EFM_HS;
+    const int i0 = p.i0, i1 = p.i0 + p.hp, i2 = i1 + p.hp;
+    efm_pdl_wait();
+    if (!__all_sync(0xffffffffu, X.wait())) return -1;
+    QV py1 = ldv(X.slot() + HB, p.k0), py2 = ldv(X.slot() + HB + CF, p.k0);
+    X.release();
+    for (int j = T.ys; j < ye; ++j, bt += plane, go += gplane) {
+        const bool live = j >= jlo && j < jhi && p.any_in();
+        QV b[6], g[3];
+        if (live) {
+#pragma unroll
+            for (int q = 0; q < 6; ++q) b[q] = ldgv(bt + q * N);
+            if (vec) {
+#pragma unroll
+                for (int q = 0; q < 3; ++q) g[q] = ldgv(g_[q] + go);
+            } else {
+#pragma unroll
+                for (int q = 0; q < 3; ++q)
+#pragma unroll
+                    for (int v = 0; v < VX; ++v) g[q].v[v] = p.in(v) ? g_[q][go + v] : 0.f;
+            }
+        }
+        if (!__all_sync(0xffffffffu, X.wait())) return -1;
+        const unsigned char *h = X.prev(), *hn = X.slot(), *cc = X.slot() + HB;
+        const QV py = ldv(h + O::py, i0);
+        if (live) {
+            const QV px = ldv(h + O::px, i0 + 4), pxz = ldv(h + O::px, i1 + 4), pxj = ldv(hn + O::px, i0 + 4);
+            const float2 pxm2 = ld2(h + O::px, i0 + 2);  // x - 2, x - 1
+            const QV pyz = ldv(h + O::py, i1);
+            const float pyx = ld1(h + O::py, i0 + VX);
+            const QV pz = ldv(h + O::pz, i2), pzm1 = ldv(h + O::pz, i1), pzm2 = ldv(h + O::pz, i0);
+            const QV pzj = ldv(hn + O::pz, i2);
+            const float pzx = ld1(h + O::pz, i2 + VX);
+            const QV m0 = ldv(h + O::rm, i0), mk = ldv(h + O::rm, i1);
+            const QV mj = ldv(hn + O::rm, i0), mjk = ldv(hn + O::rm, i1);
+            const float mi = ld1(h + O::rm, i0 + VX), mik = ld1(h + O::rm, i1 + VX), mij = ld1(hn + O::rm, i0 + VX);
+            QV c[7], o[3];
+#pragma unroll
+            for (int q = 0; q < 7; ++q) c[q] = ldv(cc + q * CF, p.k0);
+#pragma unroll
+            for (int v = 0; v < VX; ++v) {
+                const float pxc = px.v[v], pyc = py.v[v], pzc = pz.v[v];
+                const float nvx = c[0].v[v], nvy = c[1].v[v], nvz = c[2].v[v];
+                const float bvx = c[3].v[v], bvy = c[4].v[v], bvz = c[5].v[v], lam = c[6].v[v];
+                const float btxx = b[0].v[v], btyy = b[1].v[v], btzz = b[2].v[v];
+                const float btxy = b[3].v[v], btxz = b[4].v[v], btyz = b[5].v[v];
+                const float grho = -((bvx * ((pxc - nvx) * idt)) + (bvy * ((pyc - nvy) * idt)) +
+                                     (bvz * ((pzc - nvz) * idt)));
+                // lambda: average of two backward differences / dx (:234-238)
+                const float pxm = v ? px.v[v - 1] : pxm2.y, pym = py1.v[v], pzm = pzm1.v[v];
+                const float pxmm = v == 0 ? pxm2.x : pxm2.y;
+                const float dvx = two_products(0.5f * (pxm - pxmm), idx, 0.5f * (pxc - pxm), idx);
+                const float dvy = two_products(0.5f * (pym - py2.v[v]), idx, 0.5f * (pyc - pym), idx);
+                const float dvz = two_products(0.5f * (pzm - pzm2.v[v]), idx, 0.5f * (pzc - pzm), idx);
+                const float r0 = m0.v[v], ri = v < VX - 1 ? m0.v[v + 1] : mi, rk = mk.v[v];
+                const float rik = v < VX - 1 ? mk.v[v + 1] : mik;
+                const float rj = mj.v[v], rjk = mjk.v[v], rij = v < VX - 1 ? mj.v[v + 1] : mij;
+                const float mu0 = frcp(r0);
+                const float glam = (btxx + btyy + btzz) * (dvx + dvy + dvz) * frcp(3.f * lam + 2.f * mu0);
+                // mu: forward strain differences, not divided by dx (:277-291)
+                const float ex = pxc - pxm, ey = pyc - pym, ez = pzc - pzm;
+                const float exz = pxz.v[v] - pxc, exy = pxj.v[v] - pxc;
+                const float eyx = (v < VX - 1 ? py.v[v + 1] : pyx) - pyc, eyz = pyz.v[v] - pyc;
+                const float ezx = (v < VX - 1 ? pz.v[v + 1] : pzx) - pzc, ezy = pzj.v[v] - pzc;
+                const float imu_xy = 0.25f * (r0 + ri + rj + rij);
+                const float imu_xz = 0.25f * (r0 + ri + rk + rik);
+                const float imu_yz = 0.25f * (r0 + rj + rk + rjk);
+                const float f = frcp(mu0 * (3.f * lam + 2.f * mu0));
+                const float lpm2 = 2.f * (lam + mu0);
+                const float gmu = f * (lpm2 * btxx - lam * btyy - lam * btzz) * ex +
+                                  f * (lpm2 * btyy - lam * btxx - lam * btzz) * ey +
+                                  f * (lpm2 * btzz - lam * btxx - lam * btyy) * ez +
+                                  imu_xy * btxy * (eyx + exy) + imu_xz * btxz * (exz + ezx) +
+                                  imu_yz * btyz * (ezy + eyz);
+                o[0].v[v] = g[0].v[v] + glam;
+                o[1].v[v] = g[1].v[v] + gmu;
+                o[2].v[v] = g[2].v[v] + grho;
+            }
+            if (vec) {
+                if (p.fl & F_PART) {
+#pragma unroll
+                    for (int v = 0; v < VX; ++v)
+#pragma unroll
+                        for (int q = 0; q < 3; ++q) o[q].v[v] = p.in(v) ? o[q].v[v] : g[q].v[v];
+                }
+#pragma unroll
+                for (int q = 0; q < 3; ++q) stv(g_[q] + go, o[q]);
+            } else {
+#pragma unroll
+                for (int q = 0; q < 3; ++q)
+#pragma unroll
+                    for (int v = 0; v < VX; ++v)
+                        if (p.in(v)) st1(g_[q] + go + v, o[q].v[v]);
+            }
+        }
+        py2 = py1;
+        py1 = py;
+        X.release();
+    }
+    return X.packed();
 }
 
-template <int PASS, int ROWS, int SR>
-__global__ void __launch_bounds__(EFM_STHREADS, efm_stream_blocks(ROWS, SR))
-efm_velocity_stream(const EfmInst *__restrict__ insts, int ninst, int it) {
-    extern __shared__ __align__(1024) unsigned char smem[];
-    velocity_body<PASS, ROWS, SR>(insts, ninst, it, blockIdx.x, smem);
+// ------------------------------------------------------------------------------ the loads
+// One load of a slot: where the field goes, its map, the box's corner relative to the tile's and
+// the plane relative to the slot's, and the box's size class.  The producer's lanes
+// take one each (one lane issuing them all takes longer than a plane's computation).
+enum { BOX_C, BOX_X, BOX_Z, BOX_XZ, BOX_XZ2 = 5 };  // cells; + 4 columns; + a row; both; two rows
+
+struct LoadOp {
+    int off;
+    signed char map, dx, dz, dy, box;
+};
+
+struct LoadTab {
+    int n[2];          // loads of a slot, of a chunk's first slot
+    LoadOp op[2][12];
+};
+
+template <int NT>
+struct Loads {
+    static constexpr int X = efm_slot_x(NT), Z = efm_slot_z(NT), XZ = efm_slot_xz(NT), C = efm_slot_c(NT);
+    static constexpr int HS = efm_halo_s(NT), HV = efm_halo_v(NT), HI = efm_halo_i(NT);
+    using V = VOff<NT>;
+    using M = IOff<NT>;
+    static constexpr LoadTab stress() {
+        return {{11, 5},
+                {{{0, 0, -4, 0, 1, BOX_XZ}, {XZ, 1, 0, 0, 1, BOX_XZ}, {2 * XZ, 2, 0, -1, 1, BOX_XZ},
+                  {3 * XZ, 3, 0, 0, 1, BOX_XZ}, {HS, 4, 0, 0, 0, BOX_C}, {HS + C, 5, 0, 0, 0, BOX_C},
+                  {HS + 2 * C, 6, 0, 0, 0, BOX_C}, {HS + 3 * C, 7, 0, 0, 0, BOX_C}, {HS + 4 * C, 8, 0, 0, 0, BOX_C},
+                  {HS + 5 * C, 9, 0, 0, 0, BOX_C}, {HS + 6 * C, 10, 0, 0, 0, BOX_C}},
+                 {{0, 0, -4, 0, 1, BOX_XZ}, {XZ, 1, 0, 0, 1, BOX_XZ}, {2 * XZ, 2, 0, -1, 1, BOX_XZ},
+                  {3 * XZ, 3, 0, 0, 1, BOX_XZ}, {HS, 11, 0, 0, 0, BOX_C}}}};
+    }
+    static constexpr LoadTab velocity() {
+        return {{10, 9},
+                {{{V::txx, 0, 0, 0, 1, BOX_X}, {V::tzz, 1, 0, 0, 1, BOX_Z}, {V::txy, 2, -4, 0, 1, BOX_X},
+                  {V::txz, 3, -4, -1, 1, BOX_XZ}, {V::tyz, 4, 0, -1, 1, BOX_Z}, {V::bu, 5, 0, 0, 1, BOX_XZ},
+                  {V::tyy, 6, 0, 0, 1, BOX_C}, {HV, 7, 0, 0, 0, BOX_C}, {HV + C, 8, 0, 0, 0, BOX_C},
+                  {HV + 2 * C, 9, 0, 0, 0, BOX_C}},
+                 {{V::txx, 0, 0, 0, 1, BOX_X}, {V::tzz, 1, 0, 0, 1, BOX_Z}, {V::txy, 2, -4, 0, 1, BOX_X},
+                  {V::txz, 3, -4, -1, 1, BOX_XZ}, {V::tyz, 4, 0, -1, 1, BOX_Z}, {V::bu, 5, 0, 0, 1, BOX_XZ},
+                  {V::tyy, 6, 0, 0, 1, BOX_C}, {HV, 10, 0, 0, 0, BOX_C}, {HV + C, 11, 0, 0, 0, BOX_C}}}};
+    }
+    static constexpr LoadTab image() {
+        return {{11, 6},
+                {{{M::px, 0, -4, 0, 1, BOX_XZ}, {M::py, 1, 0, 0, 1, BOX_XZ}, {M::pz, 2, 0, -2, 1, BOX_XZ2},
+                  {M::rm, 3, 0, 0, 1, BOX_XZ}, {HI, 4, 0, 0, 0, BOX_C}, {HI + C, 5, 0, 0, 0, BOX_C},
+                  {HI + 2 * C, 6, 0, 0, 0, BOX_C}, {HI + 3 * C, 7, 0, 0, 0, BOX_C}, {HI + 4 * C, 8, 0, 0, 0, BOX_C},
+                  {HI + 5 * C, 9, 0, 0, 0, BOX_C}, {HI + 6 * C, 10, 0, 0, 0, BOX_C}},
+                 {{M::px, 0, -4, 0, 1, BOX_XZ}, {M::py, 1, 0, 0, 1, BOX_XZ}, {M::pz, 2, 0, -2, 1, BOX_XZ2},
+                  {M::rm, 3, 0, 0, 1, BOX_XZ}, {HI, 11, 0, 0, 0, BOX_C}, {HI + C, 11, 0, 0, -1, BOX_C}}}};
+    }
+};
+
+__constant__ LoadTab g_loads[2][3] = {{Loads<224>::stress(), Loads<224>::velocity(), Loads<224>::image()},
+                                      {Loads<96>::stress(), Loads<96>::velocity(), Loads<96>::image()}};
+
+// This lane's loads of a chunk's slots ([1]: of the first one), and the bytes of all of them.
+struct LaneLoads {
+    int off[2], x[2], z[2], dy[2], map[2], bytes[2];
+    bool on[2];
+};
+
+template <int NT>
+__device__ __forceinline__ LaneLoads lane_loads(const Chunk &T, int lane) {
+    const LoadTab &L = g_loads[NT == 96][T.type];
+    LaneLoads r;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        r.on[k] = lane < L.n[k];
+        const LoadOp o = L.op[k][r.on[k] ? lane : 0];
+        r.off[k] = o.off;
+        r.x[k] = T.x0 + o.dx;
+        r.z[k] = T.z0 + o.dz;
+        r.dy[k] = o.dy;
+        r.map[k] = o.map;
+        const int w = T.tw + (o.box & 1 ? 4 : 0), h = T.th + (o.box >> 1);  // (BOX_XZ2 >> 1 = 2 rows)
+        r.bytes[k] = __reduce_add_sync(0xffffffffu, r.on[k] ? 4 * w * h : 0);
+    }
+    return r;
 }
 
-// Forward velocity that also sums |v|^2 into the table's illumination volume.
-template <int ROWS, int SR>
-__global__ void __launch_bounds__(EFM_STHREADS, efm_stream_blocks(ROWS, SR))
-efm_velocity_illum_stream(const EfmInst *__restrict__ insts, int ninst, int it) {
-    extern __shared__ __align__(1024) unsigned char smem[];
-    velocity_body<EFM_FWD, ROWS, SR, true>(insts, ninst, it, blockIdx.x, smem);
+// ---------------------------------------------------------------------------- the producer
+// Chunk `id` of an instance: tiles first, then y; the last run of planes comes second, so that
+// the slower CPML planes at both ends of y start early.
+__device__ __forceinline__ Chunk chunk_at(const EfmInst &I, int type, int id) {
+    const int l = id - I.tile_begin;
+    const int cols = I.tiles_x * I.tiles_z;
+    int ty = l / cols;
+    Chunk c;
+    c.type = type;
+    c.tw = I.tw;
+    c.th = I.th;
+    c.col = l - ty * cols;
+    ty = ty == 0 ? 0 : ty == 1 ? I.tiles_y - 1 : ty - 1;
+    const int tz = c.col / I.tiles_x;
+    c.x0 = I.ox + (c.col - tz * I.tiles_x) * I.tw;
+    c.z0 = I.oz + tz * I.th;
+    c.ys = I.ylo + ty * I.ychunk;
+    c.ye = min(I.yhi, c.ys + I.ychunk);
+    return c;
 }
 
-// Two independent half-steps in one launch: blocks [0, tiles_s) run the stress pass PS of
-// table ts, the rest the velocity pass PV of table tv.  The gradient's adjoint chain and its
-// reverse-time rebuild touch disjoint fields within a step, so (adjoint stress, rebuild
-// velocity) and (rebuild stress, adjoint velocity) can share a grid and fill the SMs
-// together instead of running back to back.
-template <int PS, int PV, int ROWS, int SR>
-__global__ void __launch_bounds__(EFM_STHREADS, efm_stream_blocks(ROWS, SR))
-efm_pair_stream(const EfmInst *__restrict__ ts, int tiles_s, const EfmInst *__restrict__ tv,
-                int ninst, int it) {
-    extern __shared__ __align__(1024) unsigned char smem[];
-    if ((int)blockIdx.x < tiles_s)
-        stress_body<PS, ROWS, SR>(ts, ninst, it, blockIdx.x, smem);
-    else
-        velocity_body<PV, ROWS, SR>(tv, ninst, it, blockIdx.x - tiles_s, smem);
+// The producer warp: every chunk's slots in order, its lanes issuing one field each.  Block b
+// starts with chunk b; the numbers of the next chunks, and their table entries, are fetched while
+// the current one is loaded.  CPML chunks take longer than interior ones: dealt out in turn
+// instead, the slowest block of a 256 x 256 x 128 launch ran a quarter longer than the mean.
+// Every block fetches until its first number past the end, `total` fetches in all, so the last
+// one resets the counter for the next launch (which waits for this grid); a call starts with the
+// counter cleared, in case a wait ran out before.  After a wait that gave up it waits (default
+// bound) for its own loads still in flight, so that none outlives the block.
+template <int NT, int D, int SLOT, int VT>
+struct Producer {
+    static constexpr int PARTS = (int)((sizeof(EfmInst) / 16 + 31) / 32);
+    const EfmStream &A;
+    Block<D> &B;
+    const int lane, total;
+    int id, pend;  // the next chunk, lane 0's number after it
+    int4 part[PARTS];
+    Chunk T;
+    const CUtensorMap *tm;
+
+    __device__ __forceinline__ Producer(const EfmStream &A_)
+        : A(A_), B(block_state<D, SLOT>()), lane(threadIdx.x & 31), total(A.cs + A.cv), id(blockIdx.x), pend(0) {}
+
+    __device__ __forceinline__ void fetch() {
+        if (lane == 0) {
+            const int v = atomicAdd(A.counter, 1);
+            if (v == total - 1) *(volatile int *)A.counter = 0;
+            pend = (int)gridDim.x + v;
+        }
+    }
+
+    // chunk id's table entry (the call's static tables)
+    __device__ __forceinline__ void entry() {
+        if (id >= total) return;
+        const int type = id < A.cs ? 0 : VT, k = id - (type ? A.cs : 0);
+        const EfmInst &I = type ? A.v[efm_find_inst(A.v, A.nv, k)] : A.s[efm_find_inst(A.s, A.ns, k)];
+#pragma unroll
+        for (int q = 0; q < PARTS; ++q)
+            if (lane + 32 * q < (int)(sizeof(EfmInst) / 16))
+                part[q] = __ldg(reinterpret_cast<const int4 *>(&I) + lane + 32 * q);
+        T = chunk_at(I, type, k);
+        tm = I.tmap;
+    }
+
+    // Hand the description to the consumers.
+    __device__ __forceinline__ void announce(int ib) {
+        int4 *o = reinterpret_cast<int4 *>(&B.inst[ib]);
+#pragma unroll
+        for (int q = 0; q < PARTS; ++q)
+            if (lane + 32 * q < (int)(sizeof(EfmInst) / 16)) o[lane + 32 * q] = part[q];
+        if (lane == 0) B.chunk[ib] = T;
+        __syncwarp();
+        if (lane == 0) efm_mbar_arrive(&B.ready[ib]);
+    }
+
+    // The first chunk, before the preceding kernel has finished.
+    __device__ __forceinline__ void prepare() {
+        entry();
+        const LaneLoads ll = lane_loads<NT>(T, lane);
+#pragma unroll
+        for (int f = 0; f < 2; ++f)
+            if (ll.on[f]) efm_prefetch_tmap(tm + ll.map[f]);
+        announce(0);
+    }
+
+    __device__ __forceinline__ void run() {
+        const uint32_t lim = B.lim;
+        Cursor<D> c;
+        int q = 0;
+        bool ok = true;
+        fetch();
+        int ib = 0;
+        while (true) {
+            const LaneLoads ll = lane_loads<NT>(T, lane);
+            const int ys = T.ys, ye = T.ye;
+            const CUtensorMap *const m = tm;
+            for (int p = ys - 1; p < ye; ++p) {
+                ok = __all_sync(0xffffffffu, ring_wait(B, &B.empty[c.cs], c.ph ^ 1u, lim));
+                if (!ok) break;
+                const int f = p < ys;
+                if (f && q) announce(ib);
+                if (lane == 0) efm_mbar_expect_tx(&B.full[c.cs], ll.bytes[f]);
+                __syncwarp();
+                if (ll.on[f])
+                    efm_tma_load_3d(ring_slot<SLOT>(c.hs) + ll.off[f], m + ll.map[f], &B.full[c.cs], ll.x[f], ll.z[f],
+                                    p + ll.dy[f]);
+                __syncwarp();
+                if (p == min(ys, ye - 1)) {  // (the first slots are on their way)
+                    id = __shfl_sync(0xffffffffu, pend, 0);
+                    if (id < total) fetch();
+                    entry();
+                }
+                c.next();
+                ++q;
+            }
+            if (!ok) break;
+            ib = B.next(ib);
+            if (id >= total) {
+                ok = __all_sync(0xffffffffu, ring_wait(B, &B.empty[c.cs], c.ph ^ 1u, lim));
+                if (ok && lane == 0) {
+                    B.chunk[ib].type = -1;
+                    efm_mbar_arrive(&B.ready[ib]);
+                }
+                break;
+            }
+        }
+        if (!ok && lane == 0)
+            for (int s = max(0, q - D); s < q; ++s) efm_mbar_wait(&B.full[s % D], (s / D) & 1, nullptr);
+    }
+};
+
+// The consumers' side of one pass: the launch's chunks of type TYPE, n the number of chunks done
+// before.  Returns the ring position (negative: a wait gave up).
+template <int TYPE, int D, int SLOT, class F>
+__device__ __forceinline__ int consume(int cur, int &n, F &&chunk) {
+    constexpr int N = Block<D>::N;
+    while (cur >= 0) {
+        Block<D> &B = block_state<D, SLOT>();
+        const int ib = n % N;
+        if (!__all_sync(0xffffffffu, ring_wait(B, &B.ready[ib], (uint32_t)(n / N) & 1u, B.lim))) return -1;
+        if (*(volatile int *)&B.chunk[ib].type != TYPE) return cur;
+        cur = chunk(cur, ib);
+        ++n;
+    }
+    return cur;
+}
+
+}  // namespace
+
+// One streaming launch: stress pass PS (-1: none), then velocity pass PV (-1: none, EFM_IMG: the
+// imaging).  With both,
+// two independent half-steps share a grid: the gradient's adjoint chain and its reverse-time
+// rebuild touch disjoint fields within a step, so (adjoint stress, rebuild velocity) and (rebuild
+// stress, adjoint velocity) fill the SMs together instead of running back to back.  Each pass has
+// a loop of its own: one loop over both kinds of chunks needs more registers than there are
+// (spills of 200 to 500 bytes per thread, and a third more time).
+template <int PS, int PV, int NT, int D, bool ILLUM>
+__global__ void __launch_bounds__(NT + 32, efm_stream_blocks(NT, D)) efm_stream(const __grid_constant__ EfmStream A) {
+    constexpr int SLOT = efm_slot_bytes(NT, PV == EFM_IMG);
+    Block<D> &B = block_state<D, SLOT>();
+    efm_pdl_trigger();
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < D; ++s) {
+            efm_mbar_init(&B.full[s], 1);
+            efm_mbar_init(&B.empty[s], NT / 32);
+        }
+        for (int s = 0; s < Block<D>::N; ++s) efm_mbar_init(&B.ready[s], 1);
+        B.abort = 0;
+        B.lim = A.lim;
+        B.err = A.err;
+        efm_fence_barrier_init();
+    }
+    __syncthreads();
+    // what comes before efm_pdl_wait (a chunk's set-up, here and in the consumers) reads only the
+    // call's static tables; the fields and the counter come after the preceding kernel has finished
+    if (threadIdx.x >= NT) {
+        Producer<NT, D, SLOT, PV == EFM_IMG ? 2 : 1> P(A);
+        P.prepare();
+        efm_pdl_wait();
+        P.run();
+        return;
+    }
+    constexpr int S = PS < 0 ? 0 : PS, V = PV < 0 || PV == EFM_IMG ? 0 : PV;
+    int cur = Ctx<D, SLOT>::START, n = 0;
+    if (PS >= 0)
+        cur = consume<0, D, SLOT>(cur, n, [&](int c, int b) { return stress_chunk<S, NT, D, SLOT>(c, b, A.it); });
+    if (PV == EFM_IMG)
+        consume<2, D, SLOT>(cur, n, [&](int c, int b) { return image_chunk<NT, D, SLOT>(c, b); });
+    else if (PV >= 0)
+        consume<1, D, SLOT>(
+            cur, n, [&](int c, int b) { return velocity_chunk<V, NT, D, SLOT, ILLUM, (PS >= 0)>(c, b, A.it); });
 }
 
 // 1/mu and 1/rho for the streaming kernels (once per call; the model may change in place).
@@ -887,14 +1329,8 @@ __global__ void efm_model_reciprocals(const float *__restrict__ mu, const float 
     }
 }
 
-cudaError_t efm_image_init_attributes();
 
 // ---------------------------------------------------------------------------- launchers
-template <int ROWS, int SR>
-constexpr int kSmemStress = efm_stream_smem(ROWS, SR, 4, 7);
-template <int ROWS, int SR>
-constexpr int kSmemVelocity = efm_stream_smem(ROWS, SR, 6, 4);
-
 // Launch with the programmatic-serialization attribute when enabled: the kernel's prologue
 // overlaps the tail of the preceding kernel (every streaming kernel waits in
 // efm_pdl_wait before it reads or writes fields).  Set by each efm_forward / efm_gradient
@@ -903,23 +1339,15 @@ static thread_local int g_pdl = 1;
 
 extern "C" void efm_stream_set_pdl(int enable) { g_pdl = enable != 0; }
 
-// the programmatic-serialization attribute (when enabled) for another launcher's config
-extern "C" void efm_stream_pdl_config(cudaLaunchConfig_t *cfg, cudaLaunchAttribute *attr) {
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg->attrs = attr;
-    cfg->numAttrs = g_pdl ? 1 : 0;
-}
-
 // Errors surface through the launcher's cudaGetLastError(); a failed cudaLaunchKernelEx is
 // recorded there too, but keep its own status for the first failure of a sequence.
 static thread_local cudaError_t g_launch_err = cudaSuccess;
 
 template <typename... KArgs, typename... Args>
-static void launch_k(void (*k)(KArgs...), int grid, int smem, cudaStream_t s, Args... args) {
+static void launch_k(void (*k)(KArgs...), int grid, int threads, int smem, cudaStream_t s, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(EFM_STHREADS);
+    cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
@@ -938,64 +1366,57 @@ static cudaError_t take_launch_err() {
     return e != cudaSuccess ? e : l;
 }
 
-template <int ROWS, int SR>
-static void launch_rows(int pass, int kind, const EfmInst *insts, int ninst, int tiles, int it,
-                        cudaStream_t s) {
-    constexpr int SS = kSmemStress<ROWS, SR>, SV = kSmemVelocity<ROWS, SR>;
-    if (kind == 0) {
-        switch (pass) {
-            case EFM_FWD: launch_k(efm_stress_stream<EFM_FWD, ROWS, SR>, tiles, SS, s, insts, ninst, it); break;
-            case EFM_ADJ: launch_k(efm_stress_stream<EFM_ADJ, ROWS, SR>, tiles, SS, s, insts, ninst, it); break;
-            default: launch_k(efm_stress_stream<EFM_REV, ROWS, SR>, tiles, SS, s, insts, ninst, it); break;
-        }
-    } else if (kind == 2) {
-        launch_k(efm_velocity_illum_stream<ROWS, SR>, tiles, SV, s, insts, ninst, it);
-    } else {
-        switch (pass) {
-            case EFM_FWD: launch_k(efm_velocity_stream<EFM_FWD, ROWS, SR>, tiles, SV, s, insts, ninst, it); break;
-            case EFM_ADJ: launch_k(efm_velocity_stream<EFM_ADJ, ROWS, SR>, tiles, SV, s, insts, ninst, it); break;
-            default: launch_k(efm_velocity_stream<EFM_REV, ROWS, SR>, tiles, SV, s, insts, ninst, it); break;
-        }
-    }
+template <int NT, int D>
+constexpr int smem_bytes(bool image) {
+    return (D + 1) * efm_slot_bytes(NT, image) + (int)sizeof(Block<D>);
+}
+static_assert(2 * (smem_bytes<224, 3>(true) + 1024) <= 228 * 1024, "two blocks of 224 consumers per SM");
+static_assert(4 * (smem_bytes<96, 3>(true) + 1024) <= 228 * 1024, "four blocks of 96 consumers per SM");
+static_assert(3 * (smem_bytes<96, 5>(true) + 1024) <= 228 * 1024, "three with the deeper ring");
+
+// Blocks that fill the device.
+extern "C" int efm_stream_slots(int rows, int ring) {
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess)
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms * efm_stream_blocks(efm_st_nt(rows), rows == 1 && ring == 6 ? 5 : 3);
 }
 
-template <int ROWS, int SR>
-static void launch_pair_rows(int which, const EfmInst *ts, int tiles_s, const EfmInst *tv,
-                             int tiles_v, int ninst, int it, cudaStream_t s) {
-    constexpr int SM = kSmemStress<ROWS, SR> > kSmemVelocity<ROWS, SR> ? kSmemStress<ROWS, SR>
-                                                                       : kSmemVelocity<ROWS, SR>;
-    if (which == 0)
-        launch_k(efm_pair_stream<EFM_ADJ, EFM_REV, ROWS, SR>, tiles_s + tiles_v, SM, s, ts, tiles_s, tv, ninst, it);
-    else
-        launch_k(efm_pair_stream<EFM_REV, EFM_ADJ, ROWS, SR>, tiles_s + tiles_v, SM, s, ts, tiles_s, tv, ninst, it);
+// Kernels by stress and velocity pass; f is called with each one.
+template <int NT, int D, class F>
+static void each_stream(F &&f) {
+    f(EFM_FWD, -1, 0, efm_stream<EFM_FWD, -1, NT, D, false>);
+    f(EFM_ADJ, -1, 0, efm_stream<EFM_ADJ, -1, NT, D, false>);
+    f(EFM_REV, -1, 0, efm_stream<EFM_REV, -1, NT, D, false>);
+    f(-1, EFM_FWD, 0, efm_stream<-1, EFM_FWD, NT, D, false>);
+    f(-1, EFM_FWD, 1, efm_stream<-1, EFM_FWD, NT, D, true>);
+    f(-1, EFM_ADJ, 0, efm_stream<-1, EFM_ADJ, NT, D, false>);
+    f(-1, EFM_REV, 0, efm_stream<-1, EFM_REV, NT, D, false>);
+    f(-1, EFM_IMG, 0, efm_stream<-1, EFM_IMG, NT, D, false>);
+    f(EFM_ADJ, EFM_REV, 0, efm_stream<EFM_ADJ, EFM_REV, NT, D, false>);
+    f(EFM_REV, EFM_ADJ, 0, efm_stream<EFM_REV, EFM_ADJ, NT, D, false>);
 }
 
-// which 0: adjoint stress (ts) + rebuild velocity (tv); 1: rebuild stress (ts) + adjoint
-// velocity (tv).
-extern "C" cudaError_t efm_launch_pair(int which, int rows, int ring, const EfmInst *ts,
-                                       int tiles_s, const EfmInst *tv, int tiles_v, int ninst,
-                                       int it, cudaStream_t s) {
+template <int NT, int D>
+static void launch_stream_k(int ps, int pv, int illum, int grid, const EfmStream &A, cudaStream_t s) {
+    each_stream<NT, D>([&](int a, int b, int i, auto k) {
+        if (a == ps && b == pv && i == illum) launch_k(k, grid, NT + 32, smem_bytes<NT, D>(pv == EFM_IMG), s, A);
+    });
+}
+
+// Stress pass ps of the leading ns entries of table ts (cs chunks) and / or velocity pass pv of
+// table tv's; a pass not wanted is -1 with no chunks.  illum: the forward velocity also sums the
+// illumination.
+extern "C" cudaError_t efm_launch_stream(int ps, int pv, int illum, int rows, int ring, const EfmInst *ts, int ns,
+                                         int cs, const EfmInst *tv, int nv, int cv, int grid, int it, int *counter,
+                                         unsigned int lim, unsigned int *err, cudaStream_t s) {
+    const EfmStream A = {ts, tv, ns, nv, cs, cv, it, counter, lim, err};
     if (rows == 1 && ring == 6)
-        launch_pair_rows<1, 6>(which, ts, tiles_s, tv, tiles_v, ninst, it, s);
+        launch_stream_k<96, 5>(ps, pv, illum, grid, A, s);
     else if (rows == 1)
-        launch_pair_rows<1, 4>(which, ts, tiles_s, tv, tiles_v, ninst, it, s);
+        launch_stream_k<96, 3>(ps, pv, illum, grid, A, s);
     else
-        launch_pair_rows<2, 4>(which, ts, tiles_s, tv, tiles_v, ninst, it, s);
-    return take_launch_err();
-}
-
-// kind 0 = stress, 1 = velocity, 2 = forward velocity that also sums the illumination;
-// rows = cells per thread (1 or 2) and ring = stages (4, or 6 with one row), matching the
-// tile layout and tensor-map boxes the table was built with.
-extern "C" cudaError_t efm_launch_stream(int pass, int kind, int rows, int ring,
-                                         const EfmInst *insts, int ninst, int tiles, int it,
-                                         cudaStream_t s) {
-    if (rows == 1 && ring == 6)
-        launch_rows<1, 6>(pass, kind, insts, ninst, tiles, it, s);
-    else if (rows == 1)
-        launch_rows<1, 4>(pass, kind, insts, ninst, tiles, it, s);
-    else
-        launch_rows<2, 4>(pass, kind, insts, ninst, tiles, it, s);
+        launch_stream_k<224, 3>(ps, pv, illum, grid, A, s);
     return take_launch_err();
 }
 
@@ -1007,27 +1428,19 @@ extern "C" cudaError_t efm_launch_reciprocals(const float *mu, const float *rho,
     return cudaGetLastError();
 }
 
-template <int ROWS, int SR>
-static cudaError_t set_rows_attributes() {
-    cudaError_t e;
-    const int ss = kSmemStress<ROWS, SR>, sv = kSmemVelocity<ROWS, SR>;
-    const auto A = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    if ((e = cudaFuncSetAttribute(efm_stress_stream<EFM_FWD, ROWS, SR>, A, ss))) return e;
-    if ((e = cudaFuncSetAttribute(efm_stress_stream<EFM_ADJ, ROWS, SR>, A, ss))) return e;
-    if ((e = cudaFuncSetAttribute(efm_stress_stream<EFM_REV, ROWS, SR>, A, ss))) return e;
-    if ((e = cudaFuncSetAttribute(efm_velocity_stream<EFM_FWD, ROWS, SR>, A, sv))) return e;
-    if ((e = cudaFuncSetAttribute(efm_velocity_stream<EFM_ADJ, ROWS, SR>, A, sv))) return e;
-    if ((e = cudaFuncSetAttribute(efm_velocity_stream<EFM_REV, ROWS, SR>, A, sv))) return e;
-    if ((e = cudaFuncSetAttribute(efm_velocity_illum_stream<ROWS, SR>, A, sv))) return e;
-    const int sp = ss > sv ? ss : sv;
-    if ((e = cudaFuncSetAttribute(efm_pair_stream<EFM_ADJ, EFM_REV, ROWS, SR>, A, sp))) return e;
-    return cudaFuncSetAttribute(efm_pair_stream<EFM_REV, EFM_ADJ, ROWS, SR>, A, sp);
+template <int NT, int D>
+static cudaError_t set_attributes() {
+    cudaError_t e = cudaSuccess;
+    each_stream<NT, D>([&](int, int pv, int, auto k) {
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<NT, D>(pv == EFM_IMG));
+    });
+    return e;
 }
 
 extern "C" cudaError_t efm_stream_init_attributes() {
     cudaError_t e;
-    if ((e = set_rows_attributes<1, 4>())) return e;
-    if ((e = set_rows_attributes<1, 6>())) return e;
-    if ((e = set_rows_attributes<2, 4>())) return e;
-    return efm_image_init_attributes();
+    if ((e = set_attributes<96, 3>())) return e;
+    if ((e = set_attributes<96, 5>())) return e;
+    return set_attributes<224, 3>();
 }

@@ -1,32 +1,51 @@
 // Geometry of the plane-streaming kernels (efm_stream.cu).
 //
-// A block owns a 64-wide (x) column of 4 * ROWS z-rows and marches along y; each of its 256
-// threads computes ROWS cells per plane (rows r, r + 4, ...).  ROWS = 2 (64 x 8 tiles, two
-// blocks per SM) and ROWS = 1 (64 x 4 tiles, three blocks per SM with a 4-deep ring, two
-// with a 6-deep ring that keeps four planes in flight) are built.
+// A block owns one (x, z) tile of tw x th cells at a time and marches it along y; each of its
+// consumer threads computes a pair of x-neighbours (one 8-byte shared-memory access per operand
+// and pair) of every plane.  Two block sizes are built: 224 consumer threads (tiles up to 448
+// cells, two blocks per SM) and 96 (up to 192 cells, four): with the producer warp that is 16
+// warps per SM, four per scheduler, and 128 registers per thread (a ninth warp per block would
+// leave 96).  The tile's shape is chosen per grid
+// (shape_of in efm_capi.cu) so that ragged grids do not leave threads idle; the shared-memory
+// slots below bound it.
 #pragma once
 
-#define EFM_STX 64          // tile width along x (cells) = threads per z-row
-#define EFM_STZ 8           // tile rows along z of the two-row variant
-#define EFM_STHREADS 256
-#define EFM_SR 4            // default ring depth: planes j-1, j, j+1 resident, j+2 in flight
-#define EFM_HX 72           // halo box width: x0-4 .. x0+67 (TMA x start stays 16-byte aligned)
-#define EFM_HX_OFF 4
-#define EFM_REC_TZ 4        // z granularity of the per-tile receiver map
-#define EFM_MAX_YCHUNK 64   // planes per block (bit mask of receiver planes is 64 bits)
+#define EFM_MAX_YCHUNK 64
+#define EFM_IMG 3  // the imaging pass, beside EFM_FWD, EFM_ADJ, EFM_REV
 
-// Box and shared-memory sizes of the variant computing `rows` cells per thread.
-__host__ __device__ constexpr int efm_st_tz(int rows) { return 4 * rows; }
-__host__ __device__ constexpr int efm_st_hz(int rows) { return 4 * rows + 2; }  // z0-1 .. z0+tz
-__host__ __device__ constexpr int efm_halo_tx(int rows) { return EFM_HX * efm_st_hz(rows) * 4; }
-__host__ __device__ constexpr int efm_halo_bytes(int rows) {
-    return (efm_halo_tx(rows) + 127) / 128 * 128;
+// Consumer threads of the variant with `rows` (EFM_OPT_TILE_ROWS); a producer warp comes on top.
+__host__ __device__ constexpr int efm_st_nt(int rows) { return rows == 1 ? 96 : 224; }
+__host__ __device__ constexpr int efm_st_cells(int nt) { return 2 * nt; }
+// Shared-memory slot of one plane's field: the cells alone, or a box with x neighbours (tw + 4
+// columns, so that the TMA x start stays 16-byte aligned), with one z neighbour row, with both,
+// or with x neighbours and two z rows.
+__host__ __device__ constexpr int efm_slot_c(int nt) { return 8 * nt; }
+__host__ __device__ constexpr int efm_slot_x(int nt) { return nt == 224 ? 2048 : 1024; }
+__host__ __device__ constexpr int efm_slot_z(int nt) { return nt == 224 ? 2304 : 1024; }
+__host__ __device__ constexpr int efm_slot_xz(int nt) { return nt == 224 ? 2432 : 1152; }
+__host__ __device__ constexpr int efm_slot_xz2(int nt) { return nt == 224 ? 2816 : 1408; }
+
+// Whether a tile of tw x th cells fits the slots.
+__host__ __device__ constexpr bool efm_shape_ok(int nt, int tw, int th) {
+    return tw >= 4 && tw % 4 == 0 && tw <= 252 && th >= 1 && tw * th <= efm_st_cells(nt) &&
+           (tw + 4) * th * 4 <= efm_slot_x(nt) && tw * (th + 1) * 4 <= efm_slot_z(nt) &&
+           (tw + 4) * (th + 1) * 4 <= efm_slot_xz(nt) && (tw + 4) * (th + 2) * 4 <= efm_slot_xz2(nt);
 }
-__host__ __device__ constexpr int efm_center_bytes(int rows) { return EFM_STX * efm_st_tz(rows) * 4; }
-__host__ __device__ constexpr int efm_stream_smem(int rows, int sr, int nh, int nc) {
-    return sr * (nh * efm_halo_bytes(rows) + nc * efm_center_bytes(rows));
+
+// Bytes of one plane: fields with neighbours (kept for planes j and j+1) and cell-only fields.
+__host__ __device__ constexpr int efm_halo_s(int nt) { return 4 * efm_slot_xz(nt); }
+__host__ __device__ constexpr int efm_cell_s(int nt) { return 7 * efm_slot_c(nt); }
+__host__ __device__ constexpr int efm_halo_v(int nt) {
+    return 2 * efm_slot_x(nt) + 2 * efm_slot_z(nt) + 2 * efm_slot_xz(nt) + efm_slot_c(nt);
 }
-// resident blocks per SM the launch bounds promise: 2 for two rows or a 6-deep ring, else 3
-__host__ __device__ constexpr int efm_stream_blocks(int rows, int sr) {
-    return rows == 1 && sr == 4 ? 3 : 2;
+__host__ __device__ constexpr int efm_cell_v(int nt) { return 3 * efm_slot_c(nt); }
+__host__ __device__ constexpr int efm_halo_i(int nt) { return 3 * efm_slot_xz(nt) + efm_slot_xz2(nt); }
+__host__ __device__ constexpr int efm_cell_i(int nt) { return 7 * efm_slot_c(nt); }
+// One ring slot: a plane's neighbour and cell fields (of the stress and velocity passes, or of the imaging).
+__host__ __device__ constexpr int efm_slot_bytes(int nt, bool image) {
+    return image                                                                ? efm_halo_i(nt) + efm_cell_i(nt)
+           : efm_halo_s(nt) + efm_cell_s(nt) > efm_halo_v(nt) + efm_cell_v(nt) ? efm_halo_s(nt) + efm_cell_s(nt)
+                                                                                 : efm_halo_v(nt) + efm_cell_v(nt);
 }
+// resident blocks per SM the launch bounds promise (d: ring depth)
+__host__ __device__ constexpr int efm_stream_blocks(int nt, int d) { return nt == 96 ? (d > 3 ? 3 : 4) : 2; }

@@ -91,10 +91,6 @@ __device__ __forceinline__ void efm_mma_commit(uint64_t *bar) {
         : "memory");
 }
 
-__device__ __forceinline__ void efm_mbar_arrive(uint64_t *bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(efm_smem_addr(bar)) : "memory");
-}
-
 // 16 consecutive FP32 columns of this thread's TMEM lane (32x32b shape: warp w of a
 // warpgroup reads lanes 32 (w % 4) .. 32 (w % 4) + 31).
 __device__ __forceinline__ void efm_tmem_ld16(uint32_t taddr, float *v) {

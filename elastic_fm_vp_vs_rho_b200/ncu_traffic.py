@@ -23,22 +23,16 @@ import sys
 CSRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), "csrc")
 
 # ncu kernel names (demangled templates) -> the bench's kernel kinds
-_KINDS = [
-    (re.compile(r"efm_pair_stream<\s*1\s*,\s*2\b"), "adj_stress+rev_velocity"),
-    (re.compile(r"efm_pair_stream<\s*2\s*,\s*1\b"), "rev_stress+adj_velocity"),
-    (re.compile(r"efm_image_stream"), "imaging"),
-    (re.compile(r"efm_stress_stream<\s*0\b"), "fwd_stress"),
-    (re.compile(r"efm_velocity_stream<\s*0\b"), "fwd_velocity"),
-    (re.compile(r"efm_stress_stream<\s*1\b"), "adj_stress"),
-    (re.compile(r"efm_velocity_stream<\s*1\b"), "adj_velocity"),
-    (re.compile(r"efm_stress_stream<\s*2\b"), "rev_stress"),
-    (re.compile(r"efm_velocity_stream<\s*2\b"), "rev_velocity"),
-]
+_PASS = r"\s*(?:\(int\)\s*)?"
+_KINDS = [(re.compile(r"efm_stream<" + _PASS + str(a) + r"\s*," + _PASS + str(b) + r"\s*,"), kind) for a, b, kind in (
+    (1, 2, "adj_stress+rev_velocity"), (2, 1, "rev_stress+adj_velocity"), (-1, 3, "imaging"),
+    (0, -1, "fwd_stress"), (-1, 0, "fwd_velocity"), (1, -1, "adj_stress"), (-1, 1, "adj_velocity"),
+    (2, -1, "rev_stress"), (-1, 2, "rev_velocity"))]
 _UNITS = {"byte": 1.0, "kbyte": 1e3, "mbyte": 1e6, "gbyte": 1e9, "tbyte": 1e12}
 
 
 # the files that determine what the plane-streaming and imaging kernels read and write
-STENCIL_SOURCES = ("efm_image.cu", "efm_internal.cuh", "efm_stream.cu", "efm_stream.cuh",
+STENCIL_SOURCES = ("efm_internal.cuh", "efm_stream.cu", "efm_stream.cuh",
                    "efm_tma.cuh")
 
 

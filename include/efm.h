@@ -200,8 +200,8 @@ EFM_API int efm_residual_misfit_noalloc(const float *mod_dev, const float *obs_d
 /* 1 (default): TMA plane-streaming stencil kernels wherever every instance allows them
  * (nx a multiple of 4, 16-byte aligned model pointers); 0: one-thread-per-cell kernels. */
 #define EFM_OPT_STREAM_KERNELS 1
-/* Planes per block of the plane-streaming kernels; 0 (default) picks the chunk that fills
- * whole waves of blocks best. */
+/* Planes per chunk of the plane-streaming kernels (their blocks take chunks one by one); 0
+ * (default) picks the chunk with the least expected time. */
 #define EFM_OPT_YCHUNK 2
 /* Steps K between full-state checkpoints of EFM_SAVE_CHECKPOINTS; memory per instance ~
  * (nt/K - 1) checkpoints + (K+1) stored steps of the 9 fields.  The exact gradient replays
@@ -210,11 +210,11 @@ EFM_API int efm_residual_misfit_noalloc(const float *mod_dev, const float *obs_d
  * the free device memory when it is first allocated (K = nt, no replay, when it fits; at
  * least ~sqrt(nt), the smallest-memory interval). */
 #define EFM_OPT_CHECKPOINT_EVERY 3
-/* Cells per thread of the plane-streaming stress/velocity kernels: 2 (64 x 8 tiles, two
- * blocks per SM) or 1 (64 x 4 tiles, three blocks per SM); 0 (default) = 2. */
+/* Block size of the plane-streaming kernels: 2 (tiles of up to 448 cells, two blocks per SM) or
+ * 1 (up to 192 cells, four blocks per SM); 0 (default) = 2. */
 #define EFM_OPT_TILE_ROWS 4
-/* Shared-memory ring depth of the plane-streaming kernels: 4 (default) or 6 (with one-row
- * tiles only: four planes in flight per block, two blocks per SM); 0 = 4. */
+/* Shared-memory ring slots of the plane-streaming kernels: 4 (default) or 6 (with the small
+ * blocks only: four planes in flight per block, three blocks per SM); 0 = 4. */
 #define EFM_OPT_RING_DEPTH 5
 /* 1 (default): in the imaging gradient, launch the adjoint and rebuild half-steps of a
  * time step pairwise in one grid (they touch disjoint fields); 0: five launches per step. */
