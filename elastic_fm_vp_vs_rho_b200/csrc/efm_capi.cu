@@ -97,7 +97,8 @@ struct Inst {
 struct Scratch {
     double *partial = nullptr;
     int64_t *seg = nullptr;
-    size_t cap = 0, seg_cap = 0;
+    double *gram = nullptr;  // efm_lbfgs_direction
+    size_t cap = 0, seg_cap = 0, gram_cap = 0;
 };
 std::mutex g_scratch_mu;
 Scratch g_scratch[64];
@@ -125,6 +126,25 @@ int get_scratch(int nseg, double **partial, int64_t **seg) {
     }
     *partial = S.partial;
     *seg = S.seg;
+    return EFM_OK;
+}
+
+// Scratch of efm_lbfgs_direction.  It grows with the number of layers, at least twofold, and a
+// smaller one stays allocated: a captured direction may be replayed with it.
+int get_gram_scratch(size_t need, double **out) {
+    int dev = 0;
+    EFM_CK(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return fail(EFM_ERR_ARG, "device ordinal out of range");
+    std::lock_guard<std::mutex> lk(g_scratch_mu);
+    Scratch &S = g_scratch[dev];
+    if (S.gram_cap < need) {
+        double *p = nullptr;
+        need = std::max(need, 2 * S.gram_cap);
+        EFM_CK(cudaMalloc(&p, need * sizeof(double)));
+        S.gram = p;
+        S.gram_cap = need;
+    }
+    *out = S.gram;
     return EFM_OK;
 }
 
@@ -1772,15 +1792,10 @@ int efm_lbfgs_direction(const float *sk, const float *yk, const float *g, float 
                         int layers, int64_t n, int iter, void *stream) {
     if (!sk || !yk || !g || !r || !work || layers < 2 || n < 0 || iter < 0)
         return fail(EFM_ERR_ARG, "bad argument");
-    double *partial;
-    int64_t *seg;
-    int rc = get_scratch(1, &partial, &seg);
+    double *scratch;
+    const int rc = get_gram_scratch((size_t)efm_util_lbfgs_scratch(layers), &scratch);
     if (rc) return rc;
-    cudaStream_t s = (cudaStream_t)stream;
-    const int64_t h[2] = {0, n};
-    EFM_CK(cudaMemcpyAsync(seg, h, sizeof(h), cudaMemcpyHostToDevice, s));
-    EFM_CK(efm_util_lbfgs_direction(sk, yk, g, r, work, layers, n, iter, partial, EFM_RED_BLOCKS,
-                                    seg, s));
+    EFM_CK(efm_util_lbfgs_direction(sk, yk, g, r, work, layers, n, iter, scratch, (cudaStream_t)stream));
     return EFM_OK;
 }
 

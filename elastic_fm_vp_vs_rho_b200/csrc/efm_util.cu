@@ -7,6 +7,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <math.h>
+#include <algorithm>
+#include <initializer_list>
 
 #include "efm_util.cuh"
 
@@ -59,6 +61,34 @@ k_finish(const double *__restrict__ partial, int nblk, double scale, double *__r
 }
 
 // ----------------------------------------------------------------------- L-BFGS pieces
+template <int V>
+struct Vec {
+    float a[V];
+};
+
+template <int V>
+__device__ __forceinline__ Vec<V> vload(const float *p) {
+    Vec<V> r;
+    if (V == 4) {
+        const float4 q = *reinterpret_cast<const float4 *>(p);
+        r.a[0] = q.x;
+        r.a[1 % V] = q.y;
+        r.a[2 % V] = q.z;
+        r.a[3 % V] = q.w;
+    } else {
+        r.a[0] = *p;
+    }
+    return r;
+}
+
+template <int V>
+__device__ __forceinline__ void vstore(float *p, const Vec<V> &v) {
+    if (V == 4)
+        *reinterpret_cast<float4 *>(p) = make_float4(v.a[0], v.a[1 % V], v.a[2 % V], v.a[3 % V]);
+    else
+        *p = v.a[0];
+}
+
 __global__ void k_sub(float *__restrict__ out, const float *__restrict__ a,
                       const float *__restrict__ b, int64_t n) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
@@ -66,42 +96,187 @@ __global__ void k_sub(float *__restrict__ out, const float *__restrict__ a,
         out[i] = a[i] - b[i];
 }
 
-// w: [0] y1.y1  [1] s1.y1  [2] scratch dot  [3] gamma  [4..4+L) sigma  [4+L..4+2L) eps
-__global__ void k_lbfgs_gamma(double *w) {
-    w[3] = (w[0] == 0.0) ? 0.0 : w[1] / w[0];
+// The two-loop recursion from inner products.  Its direction is a combination of g and the used
+// history vectors whose coefficients follow from the products s_i.y_j (i >= j, layers newest
+// first), y_i.y_j, s_i.g and y_i.g: one pass forms all of them, a small kernel runs the two loops
+// on them, one pass forms the combination (49 us at 200 x 200 x 100, 8 pairs: the DRAM rate).  Each
+// vector is read twice, 272 MB each time; vector by vector, every step of the recursion read and
+// wrote the direction and two more vectors (1.5 GB, about 70 launches, 740 us; now 130 us).  Products and combination are in float64;
+// the direction is rounded once, at the end, instead of after every step.
+//
+// The products: a warp takes groups a >= b of eight layers and runs the float64 matrix instruction
+// (8 x 8 products, four cells per step) for y_a.y_b and s_a.y_b; a lane's four consecutive cells of
+// one vector serve as operand in four steps, as row or as column alike.  Bound by the latency of
+// its loads (fetched a step ahead; without that 109 us), then conversions and the matrix rate.  With 4 x 4 products per
+// warp on the vector unit (52 conversions) the pass took 116 us at 200 x 200 x 100, this 72 us.
+// Per pair of groups 64 + 64 products and, on the diagonal, 8 + 8 with g.
+constexpr int GT = 144;
+
+__host__ __device__ constexpr int gram_groups(int u) { return (u + 7) / 8; }
+__host__ __device__ constexpr int gram_tiles(int u) { return gram_groups(u) * (gram_groups(u) + 1) / 2; }
+
+__device__ __forceinline__ int gram_at(bool s, int i, int j) {  // group of i >= group of j
+    const int a = i / 8, b = j / 8;
+    return (a * (a + 1) / 2 + b) * GT + (s ? 64 : 0) + (i % 8) * 8 + j % 8;
+}
+__device__ __forceinline__ int gram_g(bool s, int i) {
+    const int a = i / 8;
+    return (a * (a + 1) / 2 + a) * GT + 128 + (s ? 8 : 0) + i % 8;
 }
 
-// after dot(y_{k+1}, s_{k+1}) -> w[2]: sigma_k; after dot(s_{k+1}, q) -> w[2]: eps_k
-__global__ void k_lbfgs_sigma(double *w, int L, int k) {
-    w[4 + k] = (w[2] == 0.0) ? 0.0 : 1.0 / w[2];
-}
-__global__ void k_lbfgs_eps(double *w, int L, int k) { w[4 + L + k] = w[4 + k] * w[2]; }
-
-// q -= eps_k * y   (first loop)
-__global__ void k_lbfgs_axpy1(float *__restrict__ q, const float *__restrict__ y,
-                              const double *__restrict__ w, int L, int k, int64_t n) {
-    const double e = w[4 + L + k];
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x)
-        q[i] = (float)((double)q[i] - e * (double)y[i]);
+// c (8 x 8: row lane / 4, columns 2 (lane % 4) and the next) += a (row lane / 4, cell lane % 4) b
+// (cell lane % 4, column lane / 4)
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(c[0]), "+d"(c[1])
+                 : "d"(a), "d"(b));
 }
 
-// r = gamma * q
-__global__ void k_lbfgs_scale(float *__restrict__ r, const float *__restrict__ q,
-                              const double *__restrict__ w, int64_t n) {
-    const double gmm = w[3];
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x)
-        r[i] = (float)(gmm * (double)q[i]);
+template <int V>
+__device__ __forceinline__ void cells4(const float *p, int64_t i, int64_t n, float (&v)[4]) {
+    if (V == 4 && i < n) {
+        const Vec<V> q = vload<V>(p + i);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = q.a[k % V];
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = i + k < n ? p[i + k] : 0.f;
+    }
 }
 
-// after dot(y_k, r) -> w[2]: r += s_k * (eps_{k-1} - sigma_{k-1} * w[2])   (second loop)
-__global__ void k_lbfgs_axpy2(float *__restrict__ r, const float *__restrict__ s,
-                              const double *__restrict__ w, int L, int km1, int64_t n) {
-    const double coef = w[4 + L + km1] - w[4 + km1] * w[2];
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x)
-        r[i] = (float)((double)r[i] + (double)s[i] * coef);
+template <int V>
+__global__ void __launch_bounds__(256, 3)
+k_lbfgs_gram(const float *__restrict__ s1, const float *__restrict__ y1, const float *__restrict__ g, int64_t n,
+             int u, double *__restrict__ partial) {
+    __shared__ double sh[8][GT];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int a = 0;
+    while ((a + 1) * (a + 2) / 2 <= (int)blockIdx.y) ++a;
+    const int b = blockIdx.y - a * (a + 1) / 2;
+    // this lane's vectors (past the last one: the last one again, its products unused)
+    const int64_t ra = (int64_t)min(8 * a + lane / 4, u - 1) * n, rb = (int64_t)min(8 * b + lane / 4, u - 1) * n;
+    double yy[2] = {}, sy[2] = {}, yg = 0.0, sg = 0.0;
+    const int64_t step = (int64_t)gridDim.x * 8 * 16;
+    float now[4][4], next[4][4];  // y_a, s_a, y_b, g: this step's and the next one's cells
+    auto load = [&](int64_t e, float (&f)[4][4]) {
+        const int64_t i = e + 4 * (lane % 4);
+        cells4<V>(y1 + ra, i, n, f[0]);
+        cells4<V>(s1 + ra, i, n, f[1]);
+        if (a != b) cells4<V>(y1 + rb, i, n, f[2]);
+        if (a == b) cells4<V>(g, i, n, f[3]);
+    };
+    int64_t e = ((int64_t)blockIdx.x * 8 + warp) * 16;
+    load(e, now);
+    for (; e < n; e += step) {
+        load(e + step, next);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const double y = (double)now[0][k], s = (double)now[1][k], c = a == b ? y : (double)now[2][k];
+            dmma(yy, y, c);
+            dmma(sy, s, c);
+            if (a == b) {
+                const double q = (double)now[3][k];
+                yg += y * q;
+                sg += s * q;
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) now[q][k] = next[q][k];
+    }
+    yg += __shfl_xor_sync(0xffffffffu, yg, 1);
+    yg += __shfl_xor_sync(0xffffffffu, yg, 2);
+    sg += __shfl_xor_sync(0xffffffffu, sg, 1);
+    sg += __shfl_xor_sync(0xffffffffu, sg, 2);
+    const int at = (lane / 4) * 8 + 2 * (lane % 4);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        sh[warp][at + k] = yy[k];
+        sh[warp][64 + at + k] = sy[k];
+    }
+    if (lane % 4 == 0) {
+        sh[warp][128 + lane / 4] = yg;
+        sh[warp][136 + lane / 4] = sg;
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < GT; k += 256) {
+        double v = 0.0;
+        for (int w = 0; w < 8; ++w) v += sh[w][k];
+        partial[((int64_t)blockIdx.y * GT + k) * gridDim.x + blockIdx.x] = v;
+    }
+}
+
+// The two loops on the products (one block).  w: [0] y1.y1  [1] s1.y1  [3] gamma  [4..4+L) sigma
+// [4+L..4+2L) eps  [4+2L..4+3L) coefficients of s; those of y are -gamma eps.
+__global__ void __launch_bounds__(128)
+k_lbfgs_solve(const double *__restrict__ G, double *__restrict__ w, int L, int u, int used) {
+    double *sigma = w + 4, *eps = w + 4 + L, *coef = w + 4 + 2 * L, *run = w + 4 + 3 * L;
+    const int t = threadIdx.x;
+    const double yy = G[gram_at(false, 0, 0)], sy = G[gram_at(true, 0, 0)];
+    const double gamma = yy == 0.0 ? 0.0 : sy / yy;
+    if (t == 0) {
+        w[0] = yy;
+        w[1] = sy;
+        w[3] = gamma;
+    }
+    for (int m = t; m < used; m += 128) {
+        const double d = G[gram_at(true, m, m)];
+        sigma[m] = d == 0.0 ? 0.0 : 1.0 / d;
+        run[m] = G[gram_g(true, m)];  // s_m . q
+    }
+    __syncthreads();
+    for (int k = 0; k < used; ++k) {
+        if (t == 0) eps[k] = sigma[k] * run[k];
+        __syncthreads();
+        const double e = eps[k];
+        for (int m = k + 1 + t; m < used; m += 128) run[m] -= e * G[gram_at(true, m, k)];
+        __syncthreads();
+    }
+    for (int k = t; k < used; k += 128) {  // y_k . gamma q
+        double v = G[gram_g(false, k)];
+        for (int j = 0; j < used; ++j) v -= eps[j] * G[j <= k ? gram_at(false, k, j) : gram_at(false, j, k)];
+        run[k] = gamma * v;
+    }
+    __syncthreads();
+    for (int k = used - 1; k >= 0; --k) {
+        if (t == 0) coef[k] = eps[k] - sigma[k] * run[k];
+        __syncthreads();
+        const double c = coef[k];
+        for (int m = t; m < k; m += 128) run[m] += c * G[gram_at(true, k, m)];
+        __syncthreads();
+    }
+}
+
+// r = gamma g - sum_k gamma eps_k y_k + sum_k coef_k s_k
+template <int V>
+__global__ void __launch_bounds__(256)
+k_lbfgs_combine(const float *__restrict__ s1, const float *__restrict__ y1, const float *g, float *r,
+                const double *__restrict__ w, int L, int used, int64_t n) {
+    extern __shared__ double sh[];  // [used] of y, [used] of s
+    const double gamma = w[3];
+    for (int k = threadIdx.x; k < used; k += 256) {
+        sh[k] = -gamma * w[4 + L + k];
+        sh[used + k] = w[4 + 2 * L + k];
+    }
+    __syncthreads();
+    for (int64_t i = ((int64_t)blockIdx.x * 256 + threadIdx.x) * V; i < n; i += (int64_t)gridDim.x * 256 * V) {
+        const Vec<V> vg = vload<V>(g + i);
+        double acc[V];
+#pragma unroll
+        for (int v = 0; v < V; ++v) acc[v] = gamma * (double)vg.a[v];
+#pragma unroll 4
+        for (int k = 0; k < used; ++k) {
+            const Vec<V> vy = vload<V>(y1 + k * n + i), vs = vload<V>(s1 + k * n + i);
+            const double cy = sh[k], cs = sh[used + k];
+#pragma unroll
+            for (int v = 0; v < V; ++v) acc[v] += cy * (double)vy.a[v] + cs * (double)vs.a[v];
+        }
+        Vec<V> o;
+#pragma unroll
+        for (int v = 0; v < V; ++v) o.a[v] = (float)acc[v];
+        vstore<V>(r + i, o);
+    }
 }
 
 // ------------------------------------------------------------------- smoothing + mask
@@ -119,39 +294,103 @@ __device__ __forceinline__ int reflect_idx(int i, int n) {
     return i;
 }
 
-// one 1-D pass along `axis` (0 = y, 1 = z, 2 = x) of a (ny, nz, nx) volume
-__global__ void k_gauss1d(const float *__restrict__ in, float *__restrict__ out, int nx, int ny,
-                          int nz, int axis, Gauss g) {
-    const int64_t n = (int64_t)nx * ny * nz;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int x = (int)(i % nx);
-        const int z = (int)((i / nx) % nz);
-        const int y = (int)(i / ((int64_t)nx * nz));
-        float acc = 0.f;
-        for (int j = -g.radius; j <= g.radius; ++j) {
-            int64_t idx;
-            if (axis == 0) idx = ((int64_t)reflect_idx(y + j, ny) * nz + z) * nx + x;
-            else if (axis == 1) idx = ((int64_t)y * nz + reflect_idx(z + j, nz)) * nx + x;
-            else idx = ((int64_t)y * nz + z) * nx + reflect_idx(x + j, nx);
-            acc += g.w[j + g.radius] * in[idx];
+// One 1-D pass, S outputs per thread along the axis: each of the S + 2 radius inputs is read once and
+// feeds up to S sums, in ascending order of the taps as a sum by itself would take them.  The
+// volumes of the inversion grids fit in L2, so the passes run at its rate; one thread per output
+// with the index arithmetic of three axes took 57 us per 200 x 200 x 100 pass (issue bound), this
+// 13 us.  A line is `count` cells, `step` floats apart; `outer` sets of `inner` lines side by side.
+template <int V>
+__global__ void __launch_bounds__(256)
+k_gauss_line(const float *__restrict__ in, float *__restrict__ out, int64_t inner, int count, int64_t step,
+             int64_t outer, int64_t outer_step, Gauss g) {
+    constexpr int S = 8;
+    const int64_t x = ((int64_t)blockIdx.x * 32 + threadIdx.x) * V;
+    const int strips = (count + S - 1) / S, R = g.radius;
+    if (x >= inner) return;
+    for (int64_t l = (int64_t)blockIdx.y * 8 + threadIdx.y; l < strips * outer; l += (int64_t)gridDim.y * 8) {
+        const int64_t o = l / strips;
+        const int c0 = (int)(l - o * strips) * S;
+        const float *p = in + o * outer_step + x;
+        float acc[S][V] = {};
+        for (int i0 = -R; i0 < S + R; i0 += 4) {  // (what a batch reads past the last input is not used)
+            Vec<V> in4[4];
+#pragma unroll
+            for (int b = 0; b < 4; ++b) in4[b] = vload<V>(p + reflect_idx(c0 + i0 + b, count) * step);
+#pragma unroll
+            for (int b = 0; b < 4; ++b)
+#pragma unroll
+                for (int k = 0; k < S; ++k) {
+                    const int j = i0 + b - k + R;
+                    if (j < 0 || j > 2 * R) continue;
+#pragma unroll
+                    for (int q = 0; q < V; ++q) acc[k][q] += g.w[j] * in4[b].a[q];
+                }
         }
-        out[i] = acc;
+#pragma unroll
+        for (int k = 0; k < S; ++k) {
+            if (c0 + k >= count) break;
+            Vec<V> r;
+#pragma unroll
+            for (int q = 0; q < V; ++q) r.a[q] = acc[k][q];
+            vstore<V>(out + o * outer_step + (c0 + k) * step + x, r);
+        }
     }
 }
 
-// copy + zero z < top and the (W+2) margins of the x, y and bottom faces (:2484-2504)
-__global__ void k_mask_copy(const float *__restrict__ in, float *__restrict__ out, int nx, int ny,
-                            int nz, int W, int top) {
-    const int64_t n = (int64_t)nx * ny * nz;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int x = (int)(i % nx);
-        const int z = (int)((i / nx) % nz);
-        const int y = (int)(i / ((int64_t)nx * nz));
-        const bool zero = z < top || y < W + 2 || y >= ny - W - 2 || x < W + 2 ||
-                          x >= nx - W - 2 || z >= nz - W - 2;
-        out[i] = zero ? 0.f : in[i];
+// The mask: zero z < top and the (W+2) margins of the x, y and bottom faces (:2484-2504).
+struct Mask {
+    int nx, ny, nz, W, top;
+    __device__ __forceinline__ bool row(int y, int z) const {
+        return z < top || y < W + 2 || y >= ny - W - 2 || z >= nz - W - 2;
+    }
+    __device__ __forceinline__ bool col(int x) const { return x < W + 2 || x >= nx - W - 2; }
+};
+
+// The pass along x, in place, and the mask: a warp per row, held in shared memory; masked rows are
+// only written.
+__global__ void __launch_bounds__(256) k_gauss_row_mask(float *__restrict__ vol, Mask M, Gauss g) {
+    extern __shared__ float rows[];
+    const int lane = threadIdx.x & 31, warps = blockDim.x >> 5, R = g.radius, nx = M.nx, len = nx + 2 * R;
+    float *row = rows + (threadIdx.x >> 5) * len;
+    for (int64_t q = (int64_t)blockIdx.x * warps + (threadIdx.x >> 5); q < (int64_t)M.ny * M.nz;
+         q += (int64_t)gridDim.x * warps) {
+        const int y = (int)(q / M.nz), z = (int)(q - (int64_t)y * M.nz);
+        float *p = vol + q * nx;
+        if (M.row(y, z)) {
+            for (int x = lane; x < nx; x += 32) p[x] = 0.f;
+            continue;
+        }
+#pragma unroll 4
+        for (int x = lane; x < nx; x += 32) row[R + x] = p[x];
+        __syncwarp();
+        if (lane < R) {
+            row[lane] = row[R + reflect_idx(lane - R, nx)];
+            row[R + nx + lane] = row[R + reflect_idx(nx + lane, nx)];
+        }
+        __syncwarp();
+        for (int x0 = lane; x0 < nx; x0 += 128) {
+            float acc[4] = {};
+            for (int j = 0; j <= 2 * R; ++j)
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (x0 + 32 * k < nx) acc[k] += g.w[j] * row[x0 + 32 * k + j];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int x = x0 + 32 * k;
+                if (x < nx) p[x] = M.col(x) ? 0.f : acc[k];
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// The mask by itself.
+__global__ void __launch_bounds__(256) k_mask(float *__restrict__ vol, Mask M) {
+    const int64_t n = (int64_t)M.nx * M.ny * M.nz;
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) {
+        const int x = (int)(i % M.nx);
+        const int64_t q = i / M.nx;
+        if (M.row((int)(q / M.nz), (int)(q % M.nz)) || M.col(x)) vol[i] = 0.f;
     }
 }
 
@@ -175,6 +414,15 @@ int grid_for(int64_t n) {
     if (b < 1) b = 1;
     return (int)b;
 }
+
+// Whether n floats behind each pointer can be read four at a time, layer by layer.
+bool vec4_ok(std::initializer_list<const float *> p, int64_t n) {
+    uintptr_t a = 0;
+    for (const float *q : p) a |= (uintptr_t)q;
+    return n % 4 == 0 && a % 16 == 0;
+}
+
+constexpr int GRAM_BLOCKS = 6 * 148;
 
 }  // namespace
 
@@ -213,42 +461,54 @@ cudaError_t efm_util_lbfgs_history(float *sk, float *yk, const float *m, const f
     return cudaGetLastError();
 }
 
+// Doubles of scratch a direction of L layers needs: per product, the blocks' parts and their sum.
+int64_t efm_util_lbfgs_scratch(int L) { return (int64_t)gram_tiles(L - 1) * GT * (GRAM_BLOCKS + 1); }
+
 cudaError_t efm_util_lbfgs_direction(const float *sk, const float *yk, const float *g, float *r,
-                                     double *w, int L, int64_t n, int iter, double *partial,
-                                     int nblk, const int64_t *seg_dev, cudaStream_t s) {
-    // seg_dev must hold {0, n}
+                                     double *w, int L, int64_t n, int iter, double *scratch,
+                                     cudaStream_t s) {
     const int used = iter < L ? iter : L - 1;
-    const int gb = grid_for(n);
-    cudaError_t e;
-    auto dot = [&](const float *a, const float *b, double *out) {
-        return efm_util_reduce(a, b, nullptr, seg_dev, 1, 1, 1.0, partial, nblk, out, s);
-    };
-    if ((e = dot(yk + n, yk + n, w + 0))) return e;
-    if ((e = dot(sk + n, yk + n, w + 1))) return e;
-    k_lbfgs_gamma<<<1, 1, 0, s>>>(w);
-    // q lives in r
-    if ((e = cudaMemcpyAsync(r, g, n * sizeof(float), cudaMemcpyDeviceToDevice, s))) return e;
-    for (int k = 0; k < used; ++k) {
-        const float *yk1 = yk + (int64_t)(k + 1) * n;
-        const float *sk1 = sk + (int64_t)(k + 1) * n;
-        if ((e = dot(yk1, sk1, w + 2))) return e;
-        k_lbfgs_sigma<<<1, 1, 0, s>>>(w, L, k);
-        if ((e = dot(sk1, r, w + 2))) return e;
-        k_lbfgs_eps<<<1, 1, 0, s>>>(w, L, k);
-        k_lbfgs_axpy1<<<gb, 256, 0, s>>>(r, yk1, w, L, k, n);
-    }
-    k_lbfgs_scale<<<gb, 256, 0, s>>>(r, r, w, n);
-    for (int k = used; k >= 1; --k) {
-        if ((e = dot(yk + (int64_t)k * n, r, w + 2))) return e;
-        k_lbfgs_axpy2<<<gb, 256, 0, s>>>(r, sk + (int64_t)k * n, w, L, k - 1, n);
-    }
+    const int u = used > 0 ? used : 1;  // (gamma takes the newest pair also before any is used)
+    const int T = gram_tiles(u);
+    const dim3 grid(GRAM_BLOCKS, T);
+    const bool v4 = vec4_ok({sk, yk, g, r}, n);
+    if (v4)
+        k_lbfgs_gram<4><<<grid, 256, 0, s>>>(sk + n, yk + n, g, n, u, scratch);
+    else
+        k_lbfgs_gram<1><<<grid, 256, 0, s>>>(sk + n, yk + n, g, n, u, scratch);
+    double *G = scratch + (int64_t)T * GT * GRAM_BLOCKS;
+    k_finish<<<T * GT, RB, 0, s>>>(scratch, GRAM_BLOCKS, 1.0, G);
+    k_lbfgs_solve<<<1, 128, 0, s>>>(G, w, L, u, used);
+    const int csh = 2 * used * (int)sizeof(double);
+    if (v4)
+        k_lbfgs_combine<4><<<grid_for(n / 4), 256, csh, s>>>(sk + n, yk + n, g, r, w, L, used, n);
+    else
+        k_lbfgs_combine<1><<<grid_for(n), 256, csh, s>>>(sk + n, yk + n, g, r, w, L, used, n);
+    return cudaGetLastError();
+}
+
+static cudaError_t gauss_line(const float *in, float *out, int64_t inner, int count, int64_t step, int64_t outer,
+                              int64_t outer_step, const Gauss &g, cudaStream_t s) {
+    const int64_t lines = (count + 7) / 8 * outer;
+    const int by = (int)std::min<int64_t>((lines + 7) / 8, 65535);
+    const dim3 block(32, 8);
+    if (vec4_ok({in, out}, inner) && step % 4 == 0 && outer_step % 4 == 0)
+        k_gauss_line<4><<<dim3((unsigned)((inner + 127) / 128), by), block, 0, s>>>(in, out, inner, count, step, outer,
+                                                                                   outer_step, g);
+    else
+        k_gauss_line<1><<<dim3((unsigned)((inner + 31) / 32), by), block, 0, s>>>(in, out, inner, count, step, outer,
+                                                                                 outer_step, g);
     return cudaGetLastError();
 }
 
 cudaError_t efm_util_smooth_mask(float *gv, float *tmp, int nx, int ny, int nz, float sigma,
                                  int W, int top, cudaStream_t s) {
-    const int64_t n = (int64_t)nx * ny * nz;
-    const int gb = grid_for(n);
+    const int64_t n = (int64_t)nx * ny * nz, plane = (int64_t)nx * nz;
+    const Mask M = {nx, ny, nz, W, top};
+    if (!(sigma > 0.f)) {
+        k_mask<<<grid_for(n), 256, 0, s>>>(gv, M);
+        return cudaGetLastError();
+    }
     Gauss g;
     int radius = (int)(4.0 * sigma + 0.5);
     if (radius > 16) radius = 16;
@@ -259,15 +519,19 @@ cudaError_t efm_util_smooth_mask(float *gv, float *tmp, int nx, int ny, int nz, 
         wsum += ww[j + radius];
     }
     for (int j = 0; j < 2 * radius + 1; ++j) g.w[j] = (float)(ww[j] / wsum);
-    if (sigma > 0.f) {
-        k_gauss1d<<<gb, 256, 0, s>>>(gv, tmp, nx, ny, nz, 0, g);
-        k_gauss1d<<<gb, 256, 0, s>>>(tmp, gv, nx, ny, nz, 1, g);
-        k_gauss1d<<<gb, 256, 0, s>>>(gv, tmp, nx, ny, nz, 2, g);
-        k_mask_copy<<<gb, 256, 0, s>>>(tmp, gv, nx, ny, nz, W, top);
-    } else {
-        k_mask_copy<<<gb, 256, 0, s>>>(gv, tmp, nx, ny, nz, W, top);
-        cudaMemcpyAsync(gv, tmp, n * sizeof(float), cudaMemcpyDeviceToDevice, s);
+    cudaError_t e;
+    if ((e = gauss_line(gv, tmp, plane, ny, plane, 1, 0, g, s))) return e;
+    if ((e = gauss_line(tmp, gv, nx, nz, nx, ny, plane, g, s))) return e;
+    const int row = (nx + 2 * radius) * (int)sizeof(float), smem = 48 * 1024;
+    if (row <= smem) {
+        const int warps = std::max(1, std::min(8, smem / row));
+        k_gauss_row_mask<<<grid_for((int64_t)ny * nz * 256 / warps), warps * 32, warps * row, s>>>(gv, M, g);
+        return cudaGetLastError();
     }
+    // rows longer than 12000 cells: x as lines of neighbouring cells, out of place
+    if ((e = gauss_line(gv, tmp, 1, nx, 1, (int64_t)ny * nz, nx, g, s))) return e;
+    if ((e = cudaMemcpyAsync(gv, tmp, n * sizeof(float), cudaMemcpyDeviceToDevice, s))) return e;
+    k_mask<<<grid_for(n), 256, 0, s>>>(gv, M);
     return cudaGetLastError();
 }
 

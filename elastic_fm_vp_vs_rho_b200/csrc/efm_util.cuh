@@ -12,8 +12,9 @@ cudaError_t efm_util_reduce(const float *a, const float *b, float *res, const in
 cudaError_t efm_util_lbfgs_history(float *sk, float *yk, const float *m, const float *g, int L,
                                    int64_t n, int iter, cudaStream_t s);
 cudaError_t efm_util_lbfgs_direction(const float *sk, const float *yk, const float *g, float *r,
-                                     double *w, int L, int64_t n, int iter, double *partial,
-                                     int nblk, const int64_t *seg_dev, cudaStream_t s);
+                                     double *w, int L, int64_t n, int iter, double *scratch,
+                                     cudaStream_t s);
+int64_t efm_util_lbfgs_scratch(int L);  // doubles
 cudaError_t efm_util_smooth_mask(float *g, float *tmp, int nx, int ny, int nz, float sigma, int W,
                                  int top, cudaStream_t s);
 cudaError_t efm_util_chain_rule(float *gl, float *gm, float *gr, const float *vp, const float *vs,

@@ -299,8 +299,8 @@ EFM_API int efm_kernel_time(efm_ctx *ctx, int kind, int reps, int it, double *ms
 
 /*
  * out[0] = sum(a*b) in float64 (the dot products of L_BFGS, lbfgs.py:39-65).
- * efm_dot and efm_lbfgs_direction share one scratch area per device (block partial sums and
- * the segment bounds, allocated on first use): calls of either that may overlap on the GPU
+ * efm_dot and efm_lbfgs_direction each have one scratch area per device (block partial sums and
+ * segment bounds, allocated on first use): calls of one of them that may overlap on the GPU
  * (issued on different streams without an ordering between them) race on it; issue them on
  * one stream or order the streams.
  */
@@ -315,7 +315,8 @@ EFM_API int efm_lbfgs_history(float *sk_dev, float *yk_dev, const float *m_dev, 
 
 /*
  * lbfgs.L_BFGS (lbfgs.py:27-67) on device: two-loop recursion r = H g with
- * gamma = s1.y1 / y1.y1; every dot product in float64; scalars stay on the device.
+ * gamma = s1.y1 / y1.y1, carried out on the inner products of the history and g, which are
+ * formed in one pass in float64; scalars stay on the device.
  * work_dev: at least 4 * layers + 8 doubles of scratch.
  */
 EFM_API int efm_lbfgs_direction(const float *sk_dev, const float *yk_dev, const float *g_dev,
