@@ -106,6 +106,7 @@ SIGNATURES = {
     "efm_dot": (_I, [_P, _P, _L, _P, _P]),
     "efm_lbfgs_history": (_I, [_P, _P, _P, _P, _I, _L, _I, _P]),
     "efm_lbfgs_direction": (_I, [_P, _P, _P, _P, _P, _I, _L, _I, _P]),
+    "efm_adam_step": (_I, [_I, _P, _P, _P, _P, _P] + [ctypes.c_double] * 6 + [_P]),
     "efm_smooth_mask": (_I, [_P, _P, _I, _I, _I, _F, _I, _I, _P]),
     "efm_chain_rule": (_I, [_P, _P, _P, _P, _P, _P, _L, _P]),
     "efm_xcorr_residual_misfit": (_I, [_P, _P, _P, _P, _I, _I, _P, _P]),

@@ -1799,6 +1799,17 @@ int efm_lbfgs_direction(const float *sk, const float *yk, const float *g, float 
     return EFM_OK;
 }
 
+int efm_adam_step(int count, float *const *params, const float *const *grads, float *const *m, float *const *v,
+                  const int64_t *n, double lr, double beta1, double beta2, double eps, double c1, double c2,
+                  void *stream) {
+    if (count < 0 || (count > 0 && (!params || !grads || !m || !v || !n))) return fail(EFM_ERR_ARG, "bad argument");
+    for (int k = 0; k < count; ++k)
+        if (n[k] < 0 || (n[k] > 0 && (!params[k] || !grads[k] || !m[k] || !v[k])))
+            return fail(EFM_ERR_ARG, "bad argument");
+    EFM_CK(efm_util_adam(count, params, grads, m, v, n, lr, beta1, beta2, eps, c1, c2, (cudaStream_t)stream));
+    return EFM_OK;
+}
+
 int efm_smooth_mask(float *g, float *tmp, int nx, int ny, int nz, float sigma, int lenpml, int top,
                     void *stream) {
     if (!g || !tmp || nx <= 0 || ny <= 0 || nz <= 0 || sigma < 0.f || sigma > 4.f)

@@ -408,6 +408,31 @@ __global__ void k_chain(float *__restrict__ gl, float *__restrict__ gm, float *_
     }
 }
 
+// One Adam step of up to ADAM_MAX tensors (blockIdx.y), in float32 throughout and rounded where
+// elementwise tensor operations would round: a launch instead of eight per tensor.
+constexpr int ADAM_MAX = 16;
+struct AdamArgs {
+    float *p[ADAM_MAX], *m[ADAM_MAX], *v[ADAM_MAX];
+    const float *g[ADAM_MAX];
+    int64_t n[ADAM_MAX];
+    float lr, beta1, beta2, alpha1, alpha2, eps, r1, r2;  // alpha = 1 - beta, r = 1 / (1 - beta^step)
+};
+
+__global__ void __launch_bounds__(256) k_adam(AdamArgs A) {
+    const int k = blockIdx.y;
+    float *const p = A.p[k], *const m = A.m[k], *const v = A.v[k];
+    const float *const g = A.g[k];
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < A.n[k]; i += (int64_t)gridDim.x * 256) {
+        const float a = g[i];
+        const float mi = __fmaf_rn(A.alpha1, a, __fmul_rn(m[i], A.beta1));
+        const float vi = __fmaf_rn(__fmul_rn(A.alpha2, a), a, __fmul_rn(v[i], A.beta2));
+        m[i] = mi;
+        v[i] = vi;
+        const float d = __fadd_rn(__fsqrt_rn(__fmul_rn(vi, A.r2)), A.eps);
+        p[i] = __fmaf_rn(-A.lr, __fdiv_rn(__fmul_rn(mi, A.r1), d), p[i]);
+    }
+}
+
 int grid_for(int64_t n) {
     int64_t b = (n + 255) / 256;
     if (b > 148 * 16) b = 148 * 16;
@@ -538,5 +563,33 @@ cudaError_t efm_util_smooth_mask(float *gv, float *tmp, int nx, int ny, int nz, 
 cudaError_t efm_util_chain_rule(float *gl, float *gm, float *gr, const float *vp, const float *vs,
                                 const float *rho, int64_t n, cudaStream_t s) {
     k_chain<<<grid_for(n), 256, 0, s>>>(gl, gm, gr, vp, vs, rho, n);
+    return cudaGetLastError();
+}
+
+cudaError_t efm_util_adam(int count, float *const *p, const float *const *g, float *const *m, float *const *v,
+                          const int64_t *n, double lr, double beta1, double beta2, double eps, double c1, double c2,
+                          cudaStream_t s) {
+    for (int k0 = 0; k0 < count; k0 += ADAM_MAX) {
+        AdamArgs A = {};
+        const int k1 = std::min(count - k0, ADAM_MAX);
+        int64_t most = 0;
+        for (int k = 0; k < k1; ++k) {
+            A.p[k] = p[k0 + k];
+            A.g[k] = g[k0 + k];
+            A.m[k] = m[k0 + k];
+            A.v[k] = v[k0 + k];
+            A.n[k] = n[k0 + k];
+            most = std::max(most, A.n[k]);
+        }
+        A.lr = (float)lr;
+        A.beta1 = (float)beta1;
+        A.beta2 = (float)beta2;
+        A.alpha1 = (float)(1.0 - beta1);
+        A.alpha2 = (float)(1.0 - beta2);
+        A.eps = (float)eps;
+        A.r1 = 1.f / (float)c1;
+        A.r2 = 1.f / (float)c2;
+        k_adam<<<dim3(grid_for(most), k1), 256, 0, s>>>(A);
+    }
     return cudaGetLastError();
 }

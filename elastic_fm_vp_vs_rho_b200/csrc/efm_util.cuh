@@ -20,4 +20,8 @@ cudaError_t efm_util_smooth_mask(float *g, float *tmp, int nx, int ny, int nz, f
 cudaError_t efm_util_chain_rule(float *gl, float *gm, float *gr, const float *vp, const float *vs,
                                 const float *rho, int64_t n, cudaStream_t s);
 
+cudaError_t efm_util_adam(int count, float *const *p, const float *const *g, float *const *m, float *const *v,
+                          const int64_t *n, double lr, double beta1, double beta2, double eps, double c1, double c2,
+                          cudaStream_t s);
+
 #define EFM_RED_BLOCKS 592  // 4 x 148 SMs: blocks of every deterministic reduction

@@ -41,12 +41,14 @@ gradient evaluation costs one forward and one adjoint solve.
 """
 from __future__ import annotations
 
+import ctypes
 import dataclasses
 import math
 
 import numpy as np
 
-from . import conv3d
+from . import _lib, conv3d
+from ._lib import check, stream_ptr
 
 WIDTHS = (16, 32, 64, 32, 16)
 NFEAT = 8
@@ -132,6 +134,16 @@ class PreconditionerNet:
         self.steps += 1
         c1 = 1.0 - beta1 ** self.steps
         c2 = 1.0 - beta2 ** self.steps
+        moments = [q for pair in self._adam for q in pair]
+        if all(t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() for t in params + flat + moments):
+            # one launch for all tensors (64 elementwise ones before)
+            n = len(params)
+            col = lambda ts: (ctypes.c_void_p * n)(*[t.data_ptr() for t in ts])  # noqa: E731
+            size = (ctypes.c_int64 * n)(*[t.numel() for t in params])
+            check(_lib.load().efm_adam_step(n, col(params), col(flat), col(moments[::2]), col(moments[1::2]), size,
+                                            lr, beta1, beta2, eps, c1, c2, stream_ptr()))
+            self.prep()
+            return
         for p, g, (m, v) in zip(params, flat, self._adam):
             m.mul_(beta1).add_(g, alpha=1.0 - beta1)
             v.mul_(beta2).addcmul_(g, g, value=1.0 - beta2)

@@ -324,6 +324,14 @@ EFM_API int efm_lbfgs_direction(const float *sk_dev, const float *yk_dev, const 
                         void *stream);
 
 /*
+ * One Adam step of `count` float32 tensors: host arrays of device pointers and sizes; m, v the
+ * moments; c1, c2 = 1 - beta1^step, 1 - beta2^step.
+ */
+EFM_API int efm_adam_step(int count, float *const *params_dev, const float *const *grads_dev, float *const *m_dev,
+                          float *const *v_dev, const int64_t *n, double lr, double beta1, double beta2, double eps,
+                          double c1, double c2, void *stream);
+
+/*
  * Gradient post-processing of fwi_Vp_Vs_Rho (:2479-2504): Gaussian filter (sigma, scipy
  * 'reflect' boundaries, radius int(4 sigma + 0.5)) along all three axes, then zero
  * z < top and the (lenpml + 2)-cell margins of the x, y and bottom faces.  In place;

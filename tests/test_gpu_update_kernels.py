@@ -68,3 +68,29 @@ def test_smooth_mask_edges(cuda, shape, width, sigma):
     t = cuda.as_tensor(a).cuda()
     smooth_mask(t, sigma=sigma, lenpml=width, top=2)
     assert np.abs(t.cpu().numpy() - ref).max() <= 6e-6 * max(np.abs(ref).max(), 1e-30)
+
+
+@pytest.mark.parametrize("count", [1, 8, 19])
+def test_adam_step_matches_tensor_operations(cuda, count):
+    """Tensors of unlike sizes, more of them than one launch takes; against the elementwise operations
+    of the step in float64: a dozen float32 roundings, 1e-6 of the largest entry."""
+    from elastic_fm_vp_vs_rho_b200.precond import PreconditionerNet
+    rng = np.random.default_rng(count)
+    net = PreconditionerNet(seed=0)
+    ps = [rng.standard_normal(1 + 97 * k * k) for k in range(2 * ((count + 1) // 2))]
+    net.parameters = lambda: par
+    net.prep = lambda: None
+    par = [cuda.as_tensor(p.astype(np.float32)).cuda() for p in ps]
+    ref = [p.cpu().double() for p in par]
+    mom = [(p * 0, p * 0) for p in ref]
+    for step in range(1, 4):
+        gs = [cuda.as_tensor(rng.standard_normal(p.numel()).astype(np.float32)).cuda() for p in par]
+        net.adam_step(list(zip(gs[::2], gs[1::2])), lr=1e-2)
+        for p, g, (m, v) in zip(ref, gs, mom):
+            g = g.cpu().double()
+            m.mul_(0.9).add_(g, alpha=0.1)
+            v.mul_(0.999).addcmul_(g, g, value=0.001)
+            p.sub_(1e-2 * (m / (1 - 0.9**step)) / ((v / (1 - 0.999**step)).sqrt() + 1e-8))
+    for p, r, (m, v), (m64, v64) in zip(par, ref, net._adam, mom):
+        for a, b in ((p, r), (m, m64), (v, v64)):
+            assert float((a.cpu().double() - b).abs().max()) <= 1e-6 * max(1.0, float(b.abs().max()))
