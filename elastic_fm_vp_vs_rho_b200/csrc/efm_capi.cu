@@ -993,8 +993,21 @@ int exact_gradient(efm_ctx *ctx, const float *res, float *grad, double *mtg, boo
     }
     std::vector<EfmExact> tab(2 * (size_t)n);
     int tiles = 0, st_tiles = 0;
-    const int xs_rows = ctx->opt_rows == 1 ? 1 : 2, xs_tz = efm_exact_stream_tz(xs_rows);
+    // 32 x 16 tiles, or 32 x 8 where those would not fill the device even with the shortest chunks
+    // (48 x 48 x 40, 72 blocks: 29.3 ms a gradient, 27.2 with 32 x 8; 128 x 128 x 96: 85.4, 106)
+    int xs_rows = ctx->opt_rows == 1 ? 1 : 2;
+    if (ctx->opt_rows == 0) {
+        double blocks = 0;
+        const int tz = efm_exact_stream_tz(2);
+        for (const Inst &I : ctx->inst)
+            blocks += (double)((I.nx + 31) / 32) * ((I.nz + tz - 1) / tz) * ((I.ny + 3) / 4);
+        int dev = 0, sms = 148;
+        if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (blocks < sms) xs_rows = 1;
+    }
+    const int xs_tz = efm_exact_stream_tz(xs_rows);
     const int xs_yc = choose_ychunk(ctx, xs_tz, std::max(1, efm_exact_stream_blocks(xs_rows)), 32);
+    efm_stream_set_pdl(ctx->opt_pdl);
     bool xs_fits = true;
     for (const Inst &I : ctx->inst)
         xs_fits = xs_fits && 9 * I.ncell < ((int64_t)1 << 31) && psi_floats(I) < ((size_t)1 << 31);

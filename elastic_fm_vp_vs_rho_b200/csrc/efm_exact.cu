@@ -23,6 +23,7 @@
 #include "efm_internal.cuh"
 
 #include "efm_exact.cuh"
+#include "efm_tma.cuh"
 
 namespace {
 
@@ -149,15 +150,27 @@ __device__ __forceinline__ bool cell_of(const EfmExact &I, int &x, int &y, int &
 
 __global__ void __launch_bounds__(EFM_THREADS)
 efm_exact_inject(const EfmExact *__restrict__ t, int n, int step) {
-    // one block per instance, threads over receivers: vbar(rec) += res[step]
+    // one block per instance, threads over receivers: vbar(rec) += res[step]; the first receiver and
+    // its residuals are fetched before the preceding launch has finished
+    efm_pdl_trigger();
     const EfmExact &I = t[blockIdx.x];
     const int64_t ntr = (int64_t)I.nt * I.nrec;
-    for (int q = threadIdx.x; q < I.nrec; q += blockDim.x) {
-        const int c = I.rec_lin[q], r = I.rec_id[q];
-        const int64_t o = (int64_t)step * I.nrec + r;
-        atomicAdd(&I.bv[0][c], I.res[o]);
-        atomicAdd(&I.bv[1][c], I.res[ntr + o]);
-        atomicAdd(&I.bv[2][c], I.res[2 * ntr + o]);
+    float *const v0 = I.bv[0], *const v1 = I.bv[1], *const v2 = I.bv[2];
+    int q = threadIdx.x, c = 0;
+    float r[3] = {};
+    auto fetch = [&]() {
+        c = I.rec_lin[q];
+        const float *p = I.res + (int64_t)step * I.nrec + I.rec_id[q];
+        for (int k = 0; k < 3; ++k) r[k] = p[k * ntr];
+    };
+    if (q < I.nrec) fetch();
+    efm_pdl_wait();
+    while (q < I.nrec) {
+        atomicAdd(&v0[c], r[0]);
+        atomicAdd(&v1[c], r[1]);
+        atomicAdd(&v2[c], r[2]);
+        q += blockDim.x;
+        if (q < I.nrec) fetch();
     }
 }
 
@@ -537,7 +550,7 @@ extern "C" cudaError_t efm_launch_exact(int kind, const EfmExact *t, int n, int 
     if (kind == 3) {
         efm_exact_averages<<<tiles, EFM_THREADS, 0, s>>>(t, n);
     } else if (kind == 0) {
-        efm_exact_inject<<<n, EFM_THREADS, 0, s>>>(t, n, step);
+        return efm_launch_pdl(efm_exact_inject, n, EFM_THREADS, 0, s, t, n, step);
     } else if (kind == 4) {
         efm_exact_velocity_T<<<tiles, EFM_THREADS, 0, s>>>(t, n, step, slot);
     } else if (kind == 5) {

@@ -1,6 +1,7 @@
 // Table entry of the exact-adjoint kernels (efm_exact.cu, efm_exact_stream.cu), one per
 // instance.
 #pragma once
+#include <cuda_runtime.h>
 #include <stdint.h>
 
 #include "efm_internal.cuh"
@@ -31,3 +32,24 @@ struct EfmExact {
     const float *res;
 };
 
+// Launch as a programmatic dependent (EFM_OPT_PDL of the calling context): the kernel's prologue
+// overlaps the tail of the preceding one.  Every thread of such a kernel waits in efm_pdl_wait, so
+// that its completion implies the preceding kernel's.
+extern "C" int efm_stream_pdl();
+
+template <typename... KArgs, typename... Args>
+cudaError_t efm_launch_pdl(void (*k)(KArgs...), int grid, int threads, int smem, cudaStream_t s, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = efm_stream_pdl() ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, k, args...);
+    const cudaError_t l = cudaGetLastError();
+    return e != cudaSuccess ? e : l;
+}

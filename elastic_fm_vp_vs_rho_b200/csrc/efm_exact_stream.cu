@@ -28,6 +28,7 @@
 
 #include "efm_exact.cuh"
 #include "efm_internal.cuh"
+#include "efm_tma.cuh"
 
 namespace {
 
@@ -431,6 +432,7 @@ __device__ __forceinline__ void vt_store(float *P, int PL, int si, const float (
 template <int ROWS>
 __global__ void __launch_bounds__(XS_THREADS, 2)
 efm_exact_vt_stream(const EfmExact *__restrict__ t, int n, int step, int slot) {
+    efm_pdl_trigger();
     using Gm = XsGeom<ROWS>;
     constexpr int PL = Gm::PL;
     extern __shared__ float xs_smem[];
@@ -456,6 +458,7 @@ efm_exact_vt_stream(const EfmExact *__restrict__ t, int n, int step, int slot) {
 #pragma unroll
     for (int h = 0; h < ROWS; ++h) col[h] = xs_col(C, T.x0 + lx, T.z0 + lr + 8 * h);
     const XsCol hcol = xs_col(C, hx, hz);
+    efm_pdl_wait();  // the volumes come after the preceding launch has finished; above: static tables
 
     // load + form plane y into shared buffer b and o (own cells); own: the block owns plane y
     auto plane = [&](int y, int b, bool own, VtY (&o)[ROWS]) {
@@ -759,6 +762,7 @@ __device__ __forceinline__ void st_store(float *P, int PL, int si, const StCell 
 template <int ROWS>
 __global__ void __launch_bounds__(XS_THREADS, 2)
 efm_exact_st_stream(const EfmExact *__restrict__ t, int n, int step, int slot) {
+    efm_pdl_trigger();
     using Gm = XsGeom<ROWS>;
     constexpr int PL = Gm::PL, TZ = Gm::TZ;
     extern __shared__ float xs_smem[];
@@ -788,6 +792,7 @@ efm_exact_st_stream(const EfmExact *__restrict__ t, int n, int step, int slot) {
 #pragma unroll
     for (int h = 0; h < ROWS; ++h) col[h] = xs_col(C, x, T.z0 + lr + 8 * h);
     const XsCol hcol = xs_col(C, hx, hz);
+    efm_pdl_wait();  // (as above)
     // a source inside the cells this block forms (own and halo, planes ys-1 .. ye)
     bool src_near = false;
     for (int s = 0; s < I.nsrc; ++s)
@@ -905,11 +910,8 @@ cudaError_t xs_launch(int kind, const EfmExact *t, int n, int tiles, int step, i
                       cudaStream_t s) {
     const int vb = xs_smem_bytes<ROWS>(VT_NF), sb = xs_smem_bytes<ROWS>(ST_NF);
     if (const cudaError_t e = xs_attrs<ROWS>()) return e;
-    if (kind == 0)
-        efm_exact_vt_stream<ROWS><<<tiles, XS_THREADS, vb, s>>>(t, n, step, slot);
-    else
-        efm_exact_st_stream<ROWS><<<tiles, XS_THREADS, sb, s>>>(t, n, step, slot);
-    return cudaGetLastError();
+    return kind == 0 ? efm_launch_pdl(efm_exact_vt_stream<ROWS>, tiles, XS_THREADS, vb, s, t, n, step, slot)
+                     : efm_launch_pdl(efm_exact_st_stream<ROWS>, tiles, XS_THREADS, sb, s, t, n, step, slot);
 }
 
 }  // namespace

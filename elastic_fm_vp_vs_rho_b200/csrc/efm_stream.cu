@@ -1338,6 +1338,7 @@ __global__ void efm_model_reciprocals(const float *__restrict__ mu, const float 
 static thread_local int g_pdl = 1;
 
 extern "C" void efm_stream_set_pdl(int enable) { g_pdl = enable != 0; }
+extern "C" int efm_stream_pdl() { return g_pdl; }
 
 // Errors surface through the launcher's cudaGetLastError(); a failed cudaLaunchKernelEx is
 // recorded there too, but keep its own status for the first failure of a sequence.

@@ -237,8 +237,9 @@ EFM_API int efm_residual_misfit_noalloc(const float *mod_dev, const float *obs_d
  * counterpart; the reference's kernels have no waits). */
 #define EFM_OPT_WAIT_LIMIT 9
 /* EFM_GRAD_EXACT: how each transposed half-step runs.  2 (default): one plane-streaming
- * launch (each block marches a 32 x 16 column of cells along y, 32 x 8 with
- * EFM_OPT_TILE_ROWS = 1; y-chunk from EFM_OPT_YCHUNK or chosen for full waves); 0: a
+ * launch (each block marches a 32 x 16 column of cells along y, or 32 x 8 with
+ * EFM_OPT_TILE_ROWS = 1 or, at 0, on grids too small for the wider ones; y-chunk from
+ * EFM_OPT_YCHUNK or chosen for full waves); 0: a
  * per-cell pass into scratch volumes + a gather launch; 1: one gather launch that recomputes
  * its neighbours' terms.  Same expressions in every form; the streaming form adds a few
  * terms in another order (no reference counterpart: the reference has no exact adjoint). */

@@ -16,8 +16,8 @@ def _rel(a, b):
     return np.abs(a - b).max() / np.abs(b).max()
 
 
-def _run(torch, stream, ychunk, rows, pair, grids, nts=(70,)):
-    from elastic_fm_vp_vs_rho_b200 import ShotBatch, _lib, configs
+def _batch(torch, grids, nts):
+    from elastic_fm_vp_vs_rho_b200 import ShotBatch, configs
     b = ShotBatch()
     for i, (nx, ny, nz, W) in enumerate(grids):
         rng = np.random.default_rng(nx)
@@ -34,6 +34,12 @@ def _run(torch, stream, ychunk, rows, pair, grids, nts=(70,)):
               cpml=configs.cpml_profiles(20., dt, dx, W, 3000., nx, ny, nz), lam=dev[0], mu=dev[1], rho=dev[2],
               wavelet=configs.ricker(25., dt, n) * 1e6, src=[[nx // 2, ny // 2, nz // 2], [W, ny // 2, 4]],
               mt=[[1., .5, -.5, .3, .2, .1], [.4, 1., .2, .1, .6, -.2]], rec=rec)
+    return b
+
+
+def _run(torch, stream, ychunk, rows, pair, grids, nts=(70,)):
+    from elastic_fm_vp_vs_rho_b200 import _lib
+    b = _batch(torch, grids, nts)
     b.set_option(_lib.EFM_OPT_STREAM_KERNELS, stream)
     b.set_option(_lib.EFM_OPT_YCHUNK, ychunk)
     b.set_option(_lib.EFM_OPT_TILE_ROWS, rows)
@@ -69,3 +75,24 @@ def test_stream_tiles_of_an_uneven_batch_equal_separate_runs(cuda, ychunk, rows,
     for i, grid in enumerate(GRIDS):
         _, one, _ = _run(cuda, 1, ychunk, rows, pair, [grid], nts[i:])
         assert np.array_equal(g[i], one[0])
+
+
+@pytest.mark.parametrize("grids,rows", [([(40, 36, 30, 6)], 1), ([(100, 90, 80, 10)], 2), (GRIDS[:3], 1)], ids=str)
+def test_exact_gradient_tile_choice_and_dependent_launches(cuda, grids, rows):
+    """Grids that fill the device with 32 x 16 tiles take them, others 32 x 8: bit for bit what that
+    option gives, with dependent launches and plain ones.  (The two tiles' kernels are compiled
+    apart and may round an operand of a small sum differently.)"""
+    from elastic_fm_vp_vs_rho_b200 import _lib
+    out = []
+    for option, pdl in ((0, 1), (0, 0), (rows, 1), (rows, 0)):
+        b = _batch(cuda, grids, [30] * len(grids))
+        b.set_option(_lib.EFM_OPT_TILE_ROWS, option)
+        b.set_option(_lib.EFM_OPT_PDL, pdl)
+        b.set_option(_lib.EFM_OPT_CHECKPOINT_EVERY, 8)
+        mod = b.forward(checkpoints=True)
+        g, m = b.gradient(mod, exact=True, mt=True)
+        b.status()
+        out.append((g.cpu().numpy(), m.cpu().numpy()))
+        b.close()
+    for g, m in out[1:]:
+        assert np.array_equal(g, out[0][0]) and np.array_equal(m, out[0][1])
