@@ -151,12 +151,12 @@ k_lbfgs_gram(const float *__restrict__ s1, const float *__restrict__ y1, const f
     __shared__ double sh[8][GT];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int a = 0;
-    while ((a + 1) * (a + 2) / 2 <= (int)blockIdx.y) ++a;
-    const int b = blockIdx.y - a * (a + 1) / 2;
+    while ((a + 1) * (a + 2) / 2 <= (int)blockIdx.x) ++a;
+    const int b = blockIdx.x - a * (a + 1) / 2;
     // this lane's vectors (past the last one: the last one again, its products unused)
     const int64_t ra = (int64_t)min(8 * a + lane / 4, u - 1) * n, rb = (int64_t)min(8 * b + lane / 4, u - 1) * n;
     double yy[2] = {}, sy[2] = {}, yg = 0.0, sg = 0.0;
-    const int64_t step = (int64_t)gridDim.x * 8 * 16;
+    const int64_t step = (int64_t)gridDim.y * 8 * 16;
     float now[4][4], next[4][4];  // y_a, s_a, y_b, g: this step's and the next one's cells
     auto load = [&](int64_t e, float (&f)[4][4]) {
         const int64_t i = e + 4 * (lane % 4);
@@ -165,7 +165,7 @@ k_lbfgs_gram(const float *__restrict__ s1, const float *__restrict__ y1, const f
         if (a != b) cells4<V>(y1 + rb, i, n, f[2]);
         if (a == b) cells4<V>(g, i, n, f[3]);
     };
-    int64_t e = ((int64_t)blockIdx.x * 8 + warp) * 16;
+    int64_t e = ((int64_t)blockIdx.y * 8 + warp) * 16;
     load(e, now);
     for (; e < n; e += step) {
         load(e + step, next);
@@ -203,7 +203,7 @@ k_lbfgs_gram(const float *__restrict__ s1, const float *__restrict__ y1, const f
     for (int k = threadIdx.x; k < GT; k += 256) {
         double v = 0.0;
         for (int w = 0; w < 8; ++w) v += sh[w][k];
-        partial[((int64_t)blockIdx.y * GT + k) * gridDim.x + blockIdx.x] = v;
+        partial[((int64_t)blockIdx.x * GT + k) * gridDim.y + blockIdx.y] = v;
     }
 }
 
@@ -249,13 +249,14 @@ k_lbfgs_solve(const double *__restrict__ G, double *__restrict__ w, int L, int u
 }
 
 // r = gamma g - sum_k gamma eps_k y_k + sum_k coef_k s_k
-template <int V>
+// (SH: the coefficients in shared memory; more than 2048 pairs read them from w.)
+template <int V, bool SH>
 __global__ void __launch_bounds__(256)
 k_lbfgs_combine(const float *__restrict__ s1, const float *__restrict__ y1, const float *g, float *r,
                 const double *__restrict__ w, int L, int used, int64_t n) {
     extern __shared__ double sh[];  // [used] of y, [used] of s
     const double gamma = w[3];
-    for (int k = threadIdx.x; k < used; k += 256) {
+    for (int k = threadIdx.x; SH && k < used; k += 256) {
         sh[k] = -gamma * w[4 + L + k];
         sh[used + k] = w[4 + 2 * L + k];
     }
@@ -268,7 +269,7 @@ k_lbfgs_combine(const float *__restrict__ s1, const float *__restrict__ y1, cons
 #pragma unroll 4
         for (int k = 0; k < used; ++k) {
             const Vec<V> vy = vload<V>(y1 + k * n + i), vs = vload<V>(s1 + k * n + i);
-            const double cy = sh[k], cs = sh[used + k];
+            const double cy = SH ? sh[k] : -gamma * w[4 + L + k], cs = SH ? sh[used + k] : w[4 + 2 * L + k];
 #pragma unroll
             for (int v = 0; v < V; ++v) acc[v] += cy * (double)vy.a[v] + cs * (double)vs.a[v];
         }
@@ -447,7 +448,8 @@ bool vec4_ok(std::initializer_list<const float *> p, int64_t n) {
     return n % 4 == 0 && a % 16 == 0;
 }
 
-constexpr int GRAM_BLOCKS = 6 * 148;
+// Blocks per pair of groups: three waves of the device, shared by the pairs.
+int gram_blocks(int T) { return std::max(8, 6 * 148 / T); }
 
 }  // namespace
 
@@ -487,7 +489,10 @@ cudaError_t efm_util_lbfgs_history(float *sk, float *yk, const float *m, const f
 }
 
 // Doubles of scratch a direction of L layers needs: per product, the blocks' parts and their sum.
-int64_t efm_util_lbfgs_scratch(int L) { return (int64_t)gram_tiles(L - 1) * GT * (GRAM_BLOCKS + 1); }
+int64_t efm_util_lbfgs_scratch(int L) {
+    const int64_t T = gram_tiles(L - 1);
+    return T * GT + std::max<int64_t>(8 * T, 6 * 148) * GT;
+}
 
 cudaError_t efm_util_lbfgs_direction(const float *sk, const float *yk, const float *g, float *r,
                                      double *w, int L, int64_t n, int iter, double *scratch,
@@ -495,20 +500,23 @@ cudaError_t efm_util_lbfgs_direction(const float *sk, const float *yk, const flo
     const int used = iter < L ? iter : L - 1;
     const int u = used > 0 ? used : 1;  // (gamma takes the newest pair also before any is used)
     const int T = gram_tiles(u);
-    const dim3 grid(GRAM_BLOCKS, T);
+    const int nblk = gram_blocks(T);
+    const dim3 grid(T, nblk);
     const bool v4 = vec4_ok({sk, yk, g, r}, n);
     if (v4)
         k_lbfgs_gram<4><<<grid, 256, 0, s>>>(sk + n, yk + n, g, n, u, scratch);
     else
         k_lbfgs_gram<1><<<grid, 256, 0, s>>>(sk + n, yk + n, g, n, u, scratch);
-    double *G = scratch + (int64_t)T * GT * GRAM_BLOCKS;
-    k_finish<<<T * GT, RB, 0, s>>>(scratch, GRAM_BLOCKS, 1.0, G);
+    double *G = scratch + (int64_t)T * GT * nblk;
+    k_finish<<<T * GT, RB, 0, s>>>(scratch, nblk, 1.0, G);
     k_lbfgs_solve<<<1, 128, 0, s>>>(G, w, L, u, used);
-    const int csh = 2 * used * (int)sizeof(double);
-    if (v4)
-        k_lbfgs_combine<4><<<grid_for(n / 4), 256, csh, s>>>(sk + n, yk + n, g, r, w, L, used, n);
+    const int csh = used <= 2048 ? 2 * used * (int)sizeof(double) : 0;
+    if (v4 && used <= 2048)
+        k_lbfgs_combine<4, true><<<grid_for(n / 4), 256, csh, s>>>(sk + n, yk + n, g, r, w, L, used, n);
+    else if (used <= 2048)
+        k_lbfgs_combine<1, true><<<grid_for(n), 256, csh, s>>>(sk + n, yk + n, g, r, w, L, used, n);
     else
-        k_lbfgs_combine<1><<<grid_for(n), 256, csh, s>>>(sk + n, yk + n, g, r, w, L, used, n);
+        k_lbfgs_combine<1, false><<<grid_for(n), 256, 0, s>>>(sk + n, yk + n, g, r, w, L, used, n);
     return cudaGetLastError();
 }
 

@@ -25,7 +25,7 @@ def _two_loop(sk, yk, g, L, it):
 
 @pytest.mark.parametrize("n", [1, 37, 4096, 100_001, 262_148])
 @pytest.mark.parametrize("layers,it", [(2, 0), (2, 1), (3, 7), (5, 4), (6, 4), (6, 5), (10, 8), (10, 9), (14, 13),
-                                       (28, 26)])
+                                       (28, 26), (90, 88)])
 def test_lbfgs_direction_and_history(cuda, n, layers, it):
     """Groups of four vectors (full, partial, one to seven of them), one and several tiles per
     block, vector lengths on and off 16 bytes.  The direction is rounded to float32 once; its
