@@ -1506,6 +1506,8 @@ int efm_gradient(efm_ctx *ctx, const float *res, float *grad, double *mtg, int f
     const bool st = stream_ok(ctx);
     if (st && (rc = get_encoder())) return rc;
     efm_stream_set_pdl(ctx->opt_pdl);
+    // (the imaging reads and writes pairs of gradient cells)
+    if (st && model && !aligned16(grad)) return fail(EFM_ERR_CUDA, "the gradient buffer must start on 16 bytes");
     const int rows = ctx->rows = ctx->opt_rows == 1 ? 1 : 2;
     ctx->ring = (rows == 1 && ctx->opt_ring == 6) ? 6 : 4;
     const int nt = efm_st_nt(rows);
@@ -1582,7 +1584,6 @@ int efm_gradient(efm_ctx *ctx, const float *res, float *grad, double *mtg, int f
                 rv.tmap = rf.tmap = dm + mv;
                 if (model) {
                     layout_stream(ri, stress_region(I), nt);
-                    ri.gvec = I.nx % 2 == 0 && ((uintptr_t)r.g_lam | (uintptr_t)r.g_mu | (uintptr_t)r.g_rho) % 8 == 0;
                     const int mi = p == 0 ? M_IMG0 : M_IMG1;
                     if ((rc = image_maps(m + mi, I, ri))) return rc;
                     ri.tmap = dm + mi;

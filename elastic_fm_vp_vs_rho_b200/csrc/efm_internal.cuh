@@ -77,7 +77,6 @@ struct EfmInst {
     int tw, th;            // tile (x, z), the first tile's corner and the planes covered
     int ox, oz, ylo, yhi;
     int pitch;             // floats from one row of an internal volume to the next (nx)
-    bool gvec;             // pairs of gradient cells start on 8 bytes
     int64_t vol;           // floats from one internal volume to the next
 };
 // The streaming kernels copy table entries in 16-byte pieces.  (Not alignas(16): the compiler then

@@ -942,7 +942,6 @@ __device__ __forceinline__ int image_chunk(int packed, int ib) {
     const float *bt = I.bt[0] + (int64_t)T.ys * plane + p.z * I.pitch + p.x;
     int64_t go = (int64_t)T.ys * gplane + p.z * I.nx + p.x;
     float *const g_[3] = {I.g_lam, I.g_mu, I.g_rho};
-    const bool vec = I.gvec;  // 8-byte gradient rows
     const float idt = I.inv_dt, idx = I.inv_dx;
     const int ye = T.ye, jlo = EFM_HS, jhi = I.ny - EFM_HS;
     const int i0 = p.i0, i1 = p.i0 + p.hp, i2 = i1 + p.hp;
@@ -956,15 +955,8 @@ __device__ __forceinline__ int image_chunk(int packed, int ib) {
         if (live) {
 #pragma unroll
             for (int q = 0; q < 6; ++q) b[q] = ldgv(bt + q * N);
-            if (vec) {
 #pragma unroll
-                for (int q = 0; q < 3; ++q) g[q] = ldgv(g_[q] + go);
-            } else {
-#pragma unroll
-                for (int q = 0; q < 3; ++q)
-#pragma unroll
-                    for (int v = 0; v < VX; ++v) g[q].v[v] = p.in(v) ? g_[q][go + v] : 0.f;
-            }
+            for (int q = 0; q < 3; ++q) g[q] = ldgv(g_[q] + go);
         }
         if (!__all_sync(0xffffffffu, X.wait())) return -1;
         const unsigned char *h = X.prev(), *hn = X.slot(), *cc = X.slot() + HB;
@@ -1022,22 +1014,14 @@ __device__ __forceinline__ int image_chunk(int packed, int ib) {
                 o[1].v[v] = g[1].v[v] + gmu;
                 o[2].v[v] = g[2].v[v] + grho;
             }
-            if (vec) {
-                if (p.fl & F_PART) {
+            if (p.fl & F_PART) {  // a pair at the edge of the updated cells keeps the other's values
 #pragma unroll
-                    for (int v = 0; v < VX; ++v)
+                for (int v = 0; v < VX; ++v)
 #pragma unroll
-                        for (int q = 0; q < 3; ++q) o[q].v[v] = p.in(v) ? o[q].v[v] : g[q].v[v];
-                }
-#pragma unroll
-                for (int q = 0; q < 3; ++q) stv(g_[q] + go, o[q]);
-            } else {
-#pragma unroll
-                for (int q = 0; q < 3; ++q)
-#pragma unroll
-                    for (int v = 0; v < VX; ++v)
-                        if (p.in(v)) st1(g_[q] + go + v, o[q].v[v]);
+                    for (int q = 0; q < 3; ++q) o[q].v[v] = p.in(v) ? o[q].v[v] : g[q].v[v];
             }
+#pragma unroll
+            for (int q = 0; q < 3; ++q) stv(g_[q] + go, o[q]);
         }
         py2 = py1;
         py1 = py;
