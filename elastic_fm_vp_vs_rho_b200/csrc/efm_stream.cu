@@ -1137,8 +1137,9 @@ __device__ __forceinline__ Chunk chunk_at(const EfmInst &I, int type, int id) {
 // instead, the slowest block of a 256 x 256 x 128 launch ran a quarter longer than the mean.
 // Every block fetches until its first number past the end, `total` fetches in all, so the last
 // one resets the counter for the next launch (which waits for this grid); a call starts with the
-// counter cleared, in case a wait ran out before.  After a wait that gave up it waits (default
-// bound) for its own loads still in flight, so that none outlives the block.
+// counter cleared, in case a wait ran out before.  Before it leaves it waits (default bound) for
+// its own loads still in flight, so that none outlives the block when consumers gave up on them;
+// where nothing gave up the consumers wait for the same loads, and it costs nothing.
 template <int NT, int D, int SLOT, int VT>
 struct Producer {
     static constexpr int PARTS = (int)((sizeof(EfmInst) / 16 + 31) / 32);
@@ -1236,7 +1237,8 @@ struct Producer {
                 break;
             }
         }
-        if (!ok && lane == 0)
+        // whoever gave up, this warp or a consumer that has left: the newest load of every barrier
+        if (lane == 0)
             for (int s = max(0, q - D); s < q; ++s) efm_mbar_wait(&B.full[s % D], (s / D) & 1, nullptr);
     }
 };

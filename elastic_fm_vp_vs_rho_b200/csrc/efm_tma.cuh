@@ -2,7 +2,8 @@
 //
 // Only plain (non-multicast) cp.async.bulk.tensor loads of this GPU's own memory are issued.
 // Every mbarrier wait is bounded: after EFM_WAIT_LIMIT polls (or the context's shorter limit,
-// EFM_OPT_WAIT_LIMIT) it gives up, sets the context's error word and lets the caller drain and return, so a lost transfer reports an error instead of hanging the GPU.
+// EFM_OPT_WAIT_LIMIT) it gives up, sets the context's error word and lets the caller drain and
+// return, so a lost transfer reports an error instead of hanging the GPU.
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
