@@ -69,6 +69,22 @@ class ConvLayer:
         self.wb, self.wt = conv3d.prep_weights(self.w)
 
 
+def _adam_in_one_launch(params, grads, moments) -> bool:
+    """Whether efm_adam_step, one launch for all tensors instead of eight elementwise ones each, can
+    take the step.  It is handed addresses and the parameters' sizes only, so every gradient and
+    moment (two per parameter) has its parameter's shape, and all are contiguous float32 tensors of
+    the current device.  Anything else is left to tensor operations, which broadcast, use each
+    tensor's own device or raise."""
+    import torch
+    if len(grads) != len(params) or len(moments) != 2 * len(params):
+        return False
+    if not all(t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() for t in [*params, *grads, *moments]):
+        return False
+    device = torch.cuda.current_device()
+    return all(t.device.index == device and t.shape == p.shape
+               for p, ts in zip(params, zip(params, grads, moments[::2], moments[1::2])) for t in ts)
+
+
 class PreconditionerNet:
     """4 conv layers (16-64 channels) on the tcgen05 conv3d kernels, with Adam."""
 
@@ -135,8 +151,7 @@ class PreconditionerNet:
         c1 = 1.0 - beta1 ** self.steps
         c2 = 1.0 - beta2 ** self.steps
         moments = [q for pair in self._adam for q in pair]
-        if all(t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() for t in params + flat + moments):
-            # one launch for all tensors (64 elementwise ones before)
+        if _adam_in_one_launch(params, flat, moments):
             n = len(params)
             col = lambda ts: (ctypes.c_void_p * n)(*[t.data_ptr() for t in ts])  # noqa: E731
             size = (ctypes.c_int64 * n)(*[t.numel() for t in params])
