@@ -1665,7 +1665,9 @@ int efm_kernel_time(efm_ctx *ctx, int kind, int reps, int it, double *ms_per_lau
         cudaEventDestroy(e0);
         return fail(EFM_ERR_CUDA, "cudaEventCreate failed");
     }
-    cudaError_t e = cudaEventRecord(e0, s);
+    // (a launch in which a wait ran out leaves its chunk counter anywhere)
+    cudaError_t e = cudaMemsetAsync(ctx->d_count, 0, sizeof(int), s);
+    if (e == cudaSuccess) e = cudaEventRecord(e0, s);
     for (int r = 0; r < reps && e == cudaSuccess; ++r) {
         const int i = it + (r & 1);  // alternate two steps, as the ping-pong tables do
         const int ki = (i & 1) ? T_IMG1 : T_IMG0;
