@@ -21,12 +21,12 @@
 // memory it also left the next stress launch, which starts while it drains, with its smaller L1
 // (256 x 256 x 128 gradient step: 491 us, 465 now).
 //
-// us per launch, before and now: 128 x 128 x 96 forward stress 23.4, 22.5, velocity 24.6, 24.9;
-// 256 x 256 x 128: 114.6, 103.4 and 115.5, 94.2 (the DRAM rate: a pass moves 15 volumes and the
-// memory variables), adjoint stress + rebuild velocity 193.7, 168.9, rebuild stress + adjoint
-// velocity 190.2, 171.7, imaging 127.1, 119.2; 64 x 64 x 64 forward 10.1, 7.0 and 12.0, 8.2
-// (launch and first loads).  Small grids are bound by issue and latency: about 260 instructions
-// per warp and plane of pairs without memory variables, 16 warps per SM.
+// us per launch, before (two cells per thread) and now: 128 x 128 x 96 forward stress 23.4, 22.0,
+// velocity 23.2, 23.1; 256 x 256 x 128: 114.6, 102.3 and 115.5, 94.4 (the DRAM rate: a pass moves
+// 15 volumes and the memory variables), adjoint stress + rebuild velocity 193.7, 164.7, rebuild
+// stress + adjoint velocity 190.2, 167.0, imaging 127.1, 118.2; 64 x 64 x 64 forward 10.1, 6.7 and
+// 12.0, 7.5 (launch and first loads).  Small grids are bound by issue and latency: about 260
+// instructions per warp and plane of pairs without memory variables, 16 warps per SM.
 //
 // Sources are looked up once per chunk, receivers per plane from a map built on the host.
 // Arithmetic, guards, CPML, sources, receivers, strips and MT strain follow efm_stencil.cu
@@ -103,21 +103,27 @@ __device__ __forceinline__ void st1(float *p, float a) {
     asm volatile("st.global.f32 [%0], %1;" ::"l"(p), "f"(a) : "memory");
 }
 
-// A cell's memory variables (one family, three components and a pad).
-__device__ __forceinline__ void ld_psi(const float4 *p, float (&a)[3]) {
-    float pad;
-    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
-                 : "=f"(a[0]), "=f"(a[1]), "=f"(a[2]), "=f"(pad)
+// The memory variables of a pair's cells (one family, three components and a pad each) in one access:
+// 32 bytes, on 32 bytes since x, nx and the slabs' offsets are even.  (By cell, every store filled
+// half of each lane's sector, and with values read where they are used the second cell's load
+// waited behind the first one's store; forward velocity 128 x 128 x 96, 30 layers: 38.7 us, 35.0 now.)
+__device__ __forceinline__ void ld_psi(const float4 *p, float (&a)[3], float (&b)[3]) {
+    float pad0, pad1;
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(a[0]), "=f"(a[1]), "=f"(a[2]), "=f"(pad0), "=f"(b[0]), "=f"(b[1]), "=f"(b[2]), "=f"(pad1)
                  : "l"(p)
                  : "memory");
 }
 
-__device__ __forceinline__ void st_psi_if(bool c, float4 *p, float x, float y, float z) {
-    asm volatile(
-        "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %0, 0;\n\t@q st.global.v4.f32 [%1], {%2, %3, %4, %5};\n\t}" ::"r"(
-            (uint32_t)c),
-        "l"(p), "f"(x), "f"(y), "f"(z), "f"(0.f)
-        : "memory");
+__device__ __forceinline__ void st_psi(float4 *p, const float (&a)[3], const float (&b)[3]) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %7, %4, %5, %6, %7};" ::"l"(p), "f"(a[0]), "f"(a[1]), "f"(a[2]),
+                 "f"(b[0]), "f"(b[1]), "f"(b[2]), "f"(0.f)
+                 : "memory");
+}
+
+__device__ __forceinline__ void st_psi1(float4 *p, const float (&a)[3]) {
+    asm volatile("st.global.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a[0]), "f"(a[1]), "f"(a[2]), "f"(0.f)
+                 : "memory");
 }
 
 // ------------------------------------------------------------------------------- the ring
@@ -324,15 +330,15 @@ __device__ __forceinline__ void prefetch_first(const EfmInst &I, const Pair &p, 
     if ((p.fl & F_IN) && (y < I.W || y >= I.ny - I.W)) prefetch2(P.base + psi_y(I, p, group, y));
 }
 
-// The old memory variables of the pair's cells, [cell][component] by family, zero where the pair has
-// none (a vector next to a slab cell's may be another cell's: it is read and not used).  Each
-// family sits behind a test that is uniform over the warp (x, z) or the block (y).  Requested
-// before the plane's wait, so the wait covers their latency; with YZ false only the x family, and
-// the others (12 registers per pair that would spill beside the plane's operands) are read where
-// they are used, from L1.  YZ pays where it does not spill (forward stress 128 x 128 x 96: 22.5 us,
-// 24.2 without) or little, for the adjoint velocity in a pair with much CPML (100 x 100 x 100, 20
-// layers: 25.3 us, 28.8 without); the adjoint stress and the velocity passes by themselves spill
-// more (forward velocity 256 x 256 x 128: 98.6 us with YZ, 93.9 without).
+// The memory variables of the pair's cells, [cell][component] by family, zero where the pair has none
+// (a vector next to a slab cell's may be another cell's: it is read and not used).  Each family
+// sits behind a test that is uniform over the warp (x, z) or the block (y).  Requested before the
+// plane's wait, so the wait covers their latency; with YZ false only the x family, and the others
+// (12 registers per pair that would spill beside the plane's operands) are read where they are
+// used, from L1.  YZ is for the stress passes, where it does not spill (adjoint stress 128 x 128 x 96:
+// 28.3 us, 29.3 without); in the velocity passes it does (forward velocity at that size: 31.6 us,
+// 29.6 without; 256 x 256 x 128: 102.8 and 98.6; the pair with the adjoint velocity, whole
+// gradient steps of 100 x 100 x 100 with 20 layers: 109.5 us and 105.6).
 template <int PML, bool YZ>
 struct PsiOld {
     static constexpr bool EARLY = YZ && PML == 2;
@@ -340,52 +346,43 @@ struct PsiOld {
     __device__ __forceinline__ void load(const Pair &p, const Psi &P, bool ypml, int py) {
 #pragma unroll
         for (int v = 0; v < VX; ++v) x[v][0] = x[v][1] = x[v][2] = 0.f;
-        if (p.fl & F_PX) {
-#pragma unroll
-            for (int v = 0; v < VX; ++v) ld_psi(P.base + (P.x + v), x[v]);
-        }
+        if (p.fl & F_PX) ld_psi(P.base + P.x, x[0], x[1]);
         if (EARLY) {
 #pragma unroll
             for (int v = 0; v < VX; ++v) y[v][0] = y[v][1] = y[v][2] = z[v][0] = z[v][1] = z[v][2] = 0.f;
-            if (ypml && (p.fl & F_IN)) {
-#pragma unroll
-                for (int v = 0; v < VX; ++v) ld_psi(P.base + (py + v), y[v]);
-            }
-            if (p.fl & F_PZ) {
-#pragma unroll
-                for (int v = 0; v < VX; ++v) ld_psi(P.base + (P.z + v), z[v]);
-            }
+            if (ypml && (p.fl & F_IN)) ld_psi(P.base + py, y[0], y[1]);
+            if (p.fl & F_PZ) ld_psi(P.base + P.z, z[0], z[1]);
         }
+    }
+    // where they are used: o = what was requested early, or read now for pairs that have the family
+    __device__ __forceinline__ void get_y(bool c, const float4 *q, float (&o)[VX][3]) const { get(c, q, y, o); }
+    __device__ __forceinline__ void get_z(bool c, const float4 *q, float (&o)[VX][3]) const { get(c, q, z, o); }
+    static __device__ __forceinline__ void get(bool c, const float4 *q, const float (&early)[EARLY ? VX : 1][3],
+                                               float (&o)[VX][3]) {
+#pragma unroll
+        for (int v = 0; v < VX; ++v)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) o[v][k] = EARLY ? early[EARLY ? v : 0][k] : 0.f;
+        if (!EARLY && c) ld_psi(q, o[0], o[1]);
     }
 };
 
-// psi <- b psi + a d for one cell's three components of a family (o: old in, new out); cells
-// without them (c false) get zeros.
-__device__ __forceinline__ void psi_step(bool c, float4 *q, float (&o)[3], float a, float b, float d0, float d1,
-                                         float d2) {
+// psi <- b psi + a d for one cell's three components of a family; cells without them (c false) get zeros.
+__device__ __forceinline__ void psi_step(bool c, float (&o)[3], float a, float b, float d0, float d1, float d2) {
     const float n0 = b * o[0] + a * d0, n1 = b * o[1] + a * d1, n2 = b * o[2] + a * d2;
     o[0] = c ? n0 : 0.f;
     o[1] = c ? n1 : 0.f;
     o[2] = c ? n2 : 0.f;
-    st_psi_if(c, q, n0, n1, n2);
 }
 
-// The same with the old values read here (late) or handed in (early).
-template <bool EARLY>
-__device__ __forceinline__ void psi_step_yz(bool c, float4 *q, float (&o)[3], const float (&early)[3], float a, float b,
-                                            float d0, float d1, float d2) {
-    o[0] = o[1] = o[2] = 0.f;
-    if (EARLY) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) o[k] = early[k];
-        psi_step(c, q, o, a, b, d0, d1, d2);
-    } else if (c) {
-        ld_psi(q, o);
-        o[0] = b * o[0] + a * d0;
-        o[1] = b * o[1] + a * d1;
-        o[2] = b * o[2] + a * d2;
-        st_psi_if(true, q, o[0], o[1], o[2]);
-    }
+// The x slabs' new values of the pair (an odd slab width leaves pairs with one such cell).
+__device__ __forceinline__ void st_psi_x(const Pair &p, float4 *q, const float (&o)[VX][3]) {
+    if (p.px(0) && p.px(1))
+        st_psi(q, o[0], o[1]);
+    else if (p.px(0))
+        st_psi1(q, o[0]);
+    else if (p.px(1))
+        st_psi1(q + 1, o[1]);
 }
 
 // ------------------------------------------------------------------------------ stress
@@ -398,7 +395,7 @@ template <int PASS, int NT, int PML>
 __device__ __forceinline__ void stress_pair(const EfmInst &I, const unsigned char *h, const unsigned char *hn,
                                             const unsigned char *cc, int it, int y, const Pair &p, bool has_src,
                                             float k, const Psi &P, bool ypml, int py, float ay, float by,
-                                            PsiOld<PML, PASS == EFM_FWD> &O, QV &vym, float *t0, int64_t N) {
+                                            PsiOld<PML, true> &O, QV &vym, float *t0, int64_t N) {
     constexpr int XZ = efm_slot_xz(NT), CF = efm_slot_c(NT);
     const int i0 = p.i0, i1 = p.i0 + p.hp;
     const QV vx = ldv(h, i0 + 4), vxz = ldv(h, i1 + 4), vxj = ldv(hn, i0 + 4);
@@ -415,6 +412,8 @@ __device__ __forceinline__ void stress_pair(const EfmInst &I, const unsigned cha
 #pragma unroll
     for (int q = 0; q < 6; ++q) t[q] = ldv(cc + (1 + q) * CF, p.k0);
     QV o[6];
+    float oy[VX][3], oz[VX][3];
+    const bool wy = PML == 2 && ypml && p.any_in(), wz = PML == 2 && (p.fl & F_PZ);
 #pragma unroll
     for (int v = 0; v < VX; ++v) {
         const float vxc = vx.v[v], vyc = vy.v[v], vzc = vz.v[v];
@@ -449,25 +448,27 @@ __device__ __forceinline__ void stress_pair(const EfmInst &I, const unsigned cha
             float pvx_x = 0.f, pvy_x = 0.f, pvz_x = 0.f, pvy_y = 0.f, pvx_y = 0.f, pvz_y = 0.f;
             float pvz_z = 0.f, pvx_z = 0.f, pvy_z = 0.f;
             if (PML == 1 || (p.fl & F_WX)) {
-                psi_step(p.px(v), P.base + (P.x + v), O.x[v], P.ax[v], P.bx[v], dvx_dx, dvy_dx, dvz_dx);
+                psi_step(p.px(v), O.x[v], P.ax[v], P.bx[v], dvx_dx, dvy_dx, dvz_dx);
                 pvx_x = O.x[v][0];
                 pvy_x = O.x[v][1];
                 pvz_x = O.x[v][2];
+                if (v == VX - 1) st_psi_x(p, P.base + P.x, O.x);
             }
-            float oy[3], oz[3];
             if (PML == 2 && ypml) {
-                psi_step_yz<O.EARLY>(p.in(v), P.base + (py + v), oy, O.y[O.EARLY ? v : 0], ay, by, dvy_dy, dvx_dy,
-                                     dvz_dy);
-                pvy_y = oy[0];
-                pvx_y = oy[1];
-                pvz_y = oy[2];
+                if (v == 0) O.get_y(wy, P.base + py, oy);
+                psi_step(wy, oy[v], ay, by, dvy_dy, dvx_dy, dvz_dy);
+                pvy_y = oy[v][0];
+                pvx_y = oy[v][1];
+                pvz_y = oy[v][2];
+                if (v == VX - 1 && wy) st_psi(P.base + py, oy[0], oy[1]);
             }
             if (PML == 2 && (p.fl & F_WZ)) {
-                psi_step_yz<O.EARLY>((p.fl & F_PZ) && p.in(v), P.base + (P.z + v), oz, O.z[O.EARLY ? v : 0], P.az,
-                                     P.bz, dvz_dz, dvx_dz, dvy_dz);
-                pvz_z = oz[0];
-                pvx_z = oz[1];
-                pvy_z = oz[2];
+                if (v == 0) O.get_z(wz, P.base + P.z, oz);
+                psi_step(wz, oz[v], P.az, P.bz, dvz_dz, dvx_dz, dvy_dz);
+                pvz_z = oz[v][0];
+                pvx_z = oz[v][1];
+                pvy_z = oz[v][2];
+                if (v == VX - 1 && wz) st_psi(P.base + P.z, oz[0], oz[1]);
             }
             txx = t[0].v[v] + k * two_products(l2m, (dvx_dx + pvx_x), lam, (dvy_dy + dvz_dz + pvy_y + pvz_z));
             tyy = t[1].v[v] + k * two_products(l2m, (dvy_dy + pvy_y), lam, (dvx_dx + dvz_dz + pvx_x + pvz_z));
@@ -476,19 +477,31 @@ __device__ __forceinline__ void stress_pair(const EfmInst &I, const unsigned cha
             txz = t[4].v[v] + k * mu_xz * ((dvx_dz + pvx_z) + (dvz_dx + pvz_x));
             tyz = t[5].v[v] + k * mu_yz * ((dvy_dz + pvy_z) + (dvz_dy + pvz_y));
         }
-        if (has_src && p.in(v)) {
+        o[0].v[v] = txx;
+        o[1].v[v] = tyy;
+        o[2].v[v] = tzz;
+        o[3].v[v] = txy;
+        o[4].v[v] = txz;
+        o[5].v[v] = tyz;
+    }
+    // few chunks hold a source: its cell's operands are read again, instead of keeping them for all
+    if (has_src) {
+#pragma unroll
+        for (int v = 0; v < VX; ++v) {
+            if (!p.in(v)) continue;
             for (int s = 0; s < I.nsrc; ++s) {
                 if (p.x + v != I.sx[s] || y != I.sy[s] || p.z != I.sz[s]) continue;
                 if (PASS != EFM_ADJ) {
                     const float w = I.wav[PASS == EFM_FWD ? it : I.nt - 1 - it];
                     const float sg = PASS == EFM_FWD ? 1.f : -1.f;
-                    txx = __fadd_rn(txx, sg * __fmul_rn(I.mt[s][0], w));
-                    tyy = __fadd_rn(tyy, sg * __fmul_rn(I.mt[s][1], w));
-                    tzz = __fadd_rn(tzz, sg * __fmul_rn(I.mt[s][2], w));
-                    txy = __fadd_rn(txy, sg * __fmul_rn(I.mt[s][3], w));
-                    txz = __fadd_rn(txz, sg * __fmul_rn(I.mt[s][4], w));
-                    tyz = __fadd_rn(tyz, sg * __fmul_rn(I.mt[s][5], w));
+#pragma unroll
+                    for (int q = 0; q < 6; ++q) o[q].v[v] = __fadd_rn(o[q].v[v], sg * __fmul_rn(I.mt[s][q], w));
                 } else if (I.mtg != nullptr) {
+                    const unsigned char *r = h + 3 * XZ, *rn = hn + 3 * XZ;
+                    const float r0 = ld1(r, i0 + v), ri = ld1(r, i0 + v + 1), rk = ld1(r, i1 + v);
+                    const float rik = ld1(r, i1 + v + 1), rj = ld1(rn, i0 + v), rjk = ld1(rn, i1 + v);
+                    const float rij = ld1(rn, i0 + v + 1), mu0 = frcp(r0), lam = ld1(cc, p.k0 + v);
+                    const float txx = o[0].v[v], tyy = o[1].v[v], tzz = o[2].v[v];
                     const float w = I.wav[I.nt - 1 - it];
                     const float f = __frcp_rn(2.f * mu0 * (3.f * lam + 2.f * mu0));
                     const float lpm2 = 2.f * (lam + mu0);
@@ -497,18 +510,12 @@ __device__ __forceinline__ void stress_pair(const EfmInst &I, const unsigned cha
                     atomicAdd(g + 0, (double)(w * (f * (lpm2 * txx - lam * tyy - lam * tzz))));
                     atomicAdd(g + 1, (double)(w * (f * (lpm2 * tyy - lam * txx - lam * tzz))));
                     atomicAdd(g + 2, (double)(w * (f * (lpm2 * tzz - lam * txx - lam * tyy))));
-                    atomicAdd(g + 3, (double)(w * (txy * __frcp_rn(mu_xy))));
-                    atomicAdd(g + 4, (double)(w * (txz * __frcp_rn(mu_xz))));
-                    atomicAdd(g + 5, (double)(w * (tyz * __frcp_rn(mu_yz))));
+                    atomicAdd(g + 3, (double)(w * (o[3].v[v] * __frcp_rn(4.f * frcp(r0 + ri + rj + rij)))));
+                    atomicAdd(g + 4, (double)(w * (o[4].v[v] * __frcp_rn(4.f * frcp(r0 + ri + rk + rik)))));
+                    atomicAdd(g + 5, (double)(w * (o[5].v[v] * __frcp_rn(4.f * frcp(r0 + rj + rk + rjk)))));
                 }
             }
         }
-        o[0].v[v] = txx;
-        o[1].v[v] = tyy;
-        o[2].v[v] = tzz;
-        o[3].v[v] = txy;
-        o[4].v[v] = txz;
-        o[5].v[v] = tyz;
     }
     vym = vy;
     if (p.fl & F_PART) {  // a pair at the edge of the updated cells keeps the others' values
@@ -550,7 +557,7 @@ __device__ __forceinline__ int stress_chunk(int packed, int ib, int it) {
         const bool ypml = PASS != EFM_REV && (j < ylo_in || j >= yhi_in);
         auto update = [&](auto tag) -> bool {
             constexpr int PML = decltype(tag)::value;
-            PsiOld<PML, PASS == EFM_FWD> O;
+            PsiOld<PML, true> O;
             float ay = 0.f, by = 0.f;
             int py = 0;
             if (PML) {
@@ -636,7 +643,7 @@ __device__ __forceinline__ VelIn velocity_in(const Pair &p, const unsigned char 
     return a;
 }
 
-template <int PASS, int NT, int D, int SLOT, bool ILLUM, bool YZ>
+template <int PASS, int NT, int D, int SLOT, bool ILLUM>
 __device__ __forceinline__ int velocity_chunk(int packed, int ib, int it) {
     using OF = VOff<NT>;
     Ctx<D, SLOT> X(packed);
@@ -752,7 +759,7 @@ __device__ __forceinline__ int velocity_chunk(int packed, int ib, int it) {
             auto update = [&](auto tag) -> bool {
                 constexpr int PML = decltype(tag)::value;
                 constexpr bool REC = PML == 2;
-                PsiOld<PML, YZ> O;
+                PsiOld<PML, false> O;
                 float ay = 0.f, by_ = 0.f;
                 int py = 0;
                 if (PML) {
@@ -781,6 +788,8 @@ __device__ __forceinline__ int velocity_chunk(int packed, int ib, int it) {
                 QV old[3], o[3];
 #pragma unroll
                 for (int c = 0; c < 3; ++c) old[c] = ldv(X.slot() + HB + c * OF::CF, p.k0);
+                float oy[VX][3], oz[VX][3];
+                const bool wy = PML == 2 && ypml && p.any_in(), wz = PML == 2 && (p.fl & F_PZ);
 #pragma unroll
                 for (int v = 0; v < VX; ++v) {
                     const float dtxx_dx = (v < VX - 1 ? a.txx.v[v + 1] : a.txxi) - a.txx.v[v];
@@ -808,25 +817,27 @@ __device__ __forceinline__ int velocity_chunk(int packed, int ib, int it) {
                     float q1 = 0.f, q2 = 0.f, q3 = 0.f, q4 = 0.f, q5 = 0.f, q6 = 0.f, q7 = 0.f, q8 = 0.f, q9 = 0.f;
                     if (PML && plane_in) {
                         if (PML == 1 || (p.fl & F_WX)) {
-                            psi_step(p.px(v), P.base + (P.x + v), O.x[v], P.ax[v], P.bx[v], dtxx_dx, dtxy_dx, dtxz_dx);
+                            psi_step(p.px(v), O.x[v], P.ax[v], P.bx[v], dtxx_dx, dtxy_dx, dtxz_dx);
                             q1 = O.x[v][0];
                             q2 = O.x[v][1];
                             q3 = O.x[v][2];
+                            if (v == VX - 1) st_psi_x(p, P.base + P.x, O.x);
                         }
-                        float oy[3], oz[3];
                         if (PML == 2 && ypml) {
-                            psi_step_yz<O.EARLY>(p.in(v), P.base + (py + v), oy, O.y[O.EARLY ? v : 0], ay, by_,
-                                                 dtyy_dy, dtxy_dy, dtyz_dy);
-                            q4 = oy[0];
-                            q5 = oy[1];
-                            q6 = oy[2];
+                            if (v == 0) O.get_y(wy, P.base + py, oy);
+                            psi_step(wy, oy[v], ay, by_, dtyy_dy, dtxy_dy, dtyz_dy);
+                            q4 = oy[v][0];
+                            q5 = oy[v][1];
+                            q6 = oy[v][2];
+                            if (v == VX - 1 && wy) st_psi(P.base + py, oy[0], oy[1]);
                         }
                         if (PML == 2 && (p.fl & F_WZ)) {
-                            psi_step_yz<O.EARLY>((p.fl & F_PZ) && p.in(v), P.base + (P.z + v), oz, O.z[O.EARLY ? v : 0],
-                                                 P.az, P.bz, dtzz_dz, dtxz_dz, dtyz_dz);
-                            q7 = oz[0];
-                            q8 = oz[1];
-                            q9 = oz[2];
+                            if (v == 0) O.get_z(wz, P.base + P.z, oz);
+                            psi_step(wz, oz[v], P.az, P.bz, dtzz_dz, dtxz_dz, dtyz_dz);
+                            q7 = oz[v][0];
+                            q8 = oz[v][1];
+                            q9 = oz[v][2];
+                            if (v == VX - 1 && wz) st_psi(P.base + P.z, oz[0], oz[1]);
                         }
                     }
                     o[0].v[v] = old[0].v[v] + k * b_x * ((dtxx_dx + q1) + (dtxy_dy + q5) + (dtxz_dz + q8));
@@ -1302,7 +1313,7 @@ __global__ void __launch_bounds__(NT + 32, efm_stream_blocks(NT, D)) efm_stream(
         consume<2, D, SLOT>(cur, n, [&](int c, int b) { return image_chunk<NT, D, SLOT>(c, b); });
     else if (PV >= 0)
         consume<1, D, SLOT>(
-            cur, n, [&](int c, int b) { return velocity_chunk<V, NT, D, SLOT, ILLUM, (PS >= 0)>(c, b, A.it); });
+            cur, n, [&](int c, int b) { return velocity_chunk<V, NT, D, SLOT, ILLUM>(c, b, A.it); });
 }
 
 // 1/mu and 1/rho for the streaming kernels (once per call; the model may change in place).
