@@ -1604,15 +1604,18 @@ int efm_gradient(efm_ctx *ctx, const float *res, float *grad, double *mtg, int f
         for (const EfmInst &e : tab)
             if (!fields_contiguous(e)) return fail(EFM_ERR_STATE, "field volumes not contiguous");
     if (st) {
-        // the pairs' tables share a launch's rounds (unpaired launches use the same chunks)
+        // a pair's tables share a launch's rounds; by themselves (300 x 44 x 52, a gradient step with
+        // the pair's chunks: 100 us, with their own 82) each has its own
         const int slots = efm_stream_slots(rows, ctx->ring);
+        const bool pairs = model && ctx->opt_pair;
         for (int q = 0; q < 2; ++q) {
             EfmInst *a = &slot(q ? T_ADJ_V : T_ADJ_S, 0), *r = &slot(q ? T_REV_S0 : T_REV_V0, 0);
-            const int yc = model ? chunk_planes(ctx, {a, r}, n, slots) : chunk_planes(ctx, {a}, n, slots);
+            const int yc = pairs ? chunk_planes(ctx, {a, r}, n, slots) : chunk_planes(ctx, {a}, n, slots);
+            const int yr = pairs || !model ? yc : chunk_planes(ctx, {r}, n, slots);
             finish_stream(ctx, q ? T_ADJ_V : T_ADJ_S, a, n, yc);
             if (!model) continue;
             for (int k : {T_REV_S0, T_REV_S1, T_REV_V0, T_REV_V1, T_REV_VF0, T_REV_VF1})
-                if ((k == T_REV_S0 || k == T_REV_S1) == (q == 1)) finish_stream(ctx, k, &slot(k, 0), n, yc);
+                if ((k == T_REV_S0 || k == T_REV_S1) == (q == 1)) finish_stream(ctx, k, &slot(k, 0), n, yr);
         }
         if (model)
             for (int k : {T_IMG0, T_IMG1})
