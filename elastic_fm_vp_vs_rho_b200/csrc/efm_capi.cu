@@ -821,8 +821,8 @@ int image_maps(CUtensorMap *m, const Inst &I, const EfmInst &d) {
     return EFM_OK;
 }
 
-// Regions of the passes.  Stress and imaging: the updated cells [2, n-2).  Velocity: the same, or the whole
-// grid when a receiver lies outside them (it records zeros and takes the adjoint source).
+// Regions of the passes.  Stress and imaging: the updated cells [2, n-2), all of x.  Velocity: the same,
+// extended in y and z to receivers outside them (which record zeros and take the adjoint source).
 // Rebuild: the non-CPML box; its velocity over the whole grid in the first two steps, which
 // write the zeros outside the box into both ping-pong buffers.
 Region stress_region(const Inst &I) {
@@ -832,13 +832,15 @@ Region stress_region(const Inst &I) {
 Region whole_grid(const Inst &I) { return {0, I.nx, 0, I.nz, 0, I.ny}; }
 
 Region velocity_region(const Inst &I) {
-    for (int r = 0; r < I.nrec; ++r) {
-        const int x = I.rec[3 * r], y = I.rec[3 * r + 1], z = I.rec[3 * r + 2];
-        if (x < EFM_HS || x >= I.nx - EFM_HS || y < EFM_HS || y >= I.ny - EFM_HS || z < EFM_HS ||
-            z >= I.nz - EFM_HS)
-            return whole_grid(I);
+    Region r = stress_region(I);
+    for (int q = 0; q < I.nrec; ++q) {
+        const int y = I.rec[3 * q + 1], z = I.rec[3 * q + 2];
+        r.y0 = std::min(r.y0, y);
+        r.y1 = std::max(r.y1, y + 1);
+        r.z0 = std::min(r.z0, z);
+        r.z1 = std::max(r.z1, z + 1);
     }
-    return stress_region(I);
+    return r;
 }
 
 Region box_region(const Inst &I) {
