@@ -300,20 +300,24 @@ __device__ __forceinline__ int reflect_idx(int i, int n) {
 // volumes of the inversion grids fit in L2, so the passes run at its rate; one thread per output
 // with the index arithmetic of three axes took 57 us per 200 x 200 x 100 pass (issue bound), this
 // 13 us.  A line is `count` cells, `step` floats apart; `outer` sets of `inner` lines side by side.
+// The block has as many threads side by side as there are lines, up to a warp's, and the rest along
+// them: with always 32, planes 4 cells wide left 31 lanes of a warp idle (400 x 400 x 4: 98 us, 32 now).
 template <int V>
 __global__ void __launch_bounds__(256)
 k_gauss_line(const float *__restrict__ in, float *__restrict__ out, int64_t inner, int count, int64_t step,
              int64_t outer, int64_t outer_step, Gauss g) {
     constexpr int S = 8;
-    const int64_t x = ((int64_t)blockIdx.x * 32 + threadIdx.x) * V;
+    const int64_t x = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * V;
     const int strips = (count + S - 1) / S, R = g.radius;
     if (x >= inner) return;
-    for (int64_t l = (int64_t)blockIdx.y * 8 + threadIdx.y; l < strips * outer; l += (int64_t)gridDim.y * 8) {
+    for (int64_t l = (int64_t)blockIdx.y * blockDim.y + threadIdx.y; l < strips * outer;
+         l += (int64_t)gridDim.y * blockDim.y) {
         const int64_t o = l / strips;
         const int c0 = (int)(l - o * strips) * S;
         const float *p = in + o * outer_step + x;
         float acc[S][V] = {};
-        for (int i0 = -R; i0 < S + R; i0 += 4) {  // (what a batch reads past the last input is not used)
+        const int end = min(S, count - c0) + R;
+        for (int i0 = -R; i0 < end; i0 += 4) {  // (what a batch reads past the last input is not used)
             Vec<V> in4[4];
 #pragma unroll
             for (int b = 0; b < 4; ++b) in4[b] = vload<V>(p + reflect_idx(c0 + i0 + b, count) * step);
@@ -385,13 +389,17 @@ __global__ void __launch_bounds__(256) k_gauss_row_mask(float *__restrict__ vol,
     }
 }
 
-// The mask by itself.
-__global__ void __launch_bounds__(256) k_mask(float *__restrict__ vol, Mask M) {
+// The mask by itself: of `vol` in place, or of a copy of `in`.
+template <bool COPY>
+__global__ void __launch_bounds__(256) k_mask(const float *__restrict__ in, float *__restrict__ vol, Mask M) {
     const int64_t n = (int64_t)M.nx * M.ny * M.nz;
     for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) {
         const int x = (int)(i % M.nx);
         const int64_t q = i / M.nx;
-        if (M.row((int)(q / M.nz), (int)(q % M.nz)) || M.col(x)) vol[i] = 0.f;
+        if (M.row((int)(q / M.nz), (int)(q % M.nz)) || M.col(x))
+            vol[i] = 0.f;
+        else if (COPY)
+            vol[i] = in[i];
     }
 }
 
@@ -523,14 +531,16 @@ cudaError_t efm_util_lbfgs_direction(const float *sk, const float *yk, const flo
 static cudaError_t gauss_line(const float *in, float *out, int64_t inner, int count, int64_t step, int64_t outer,
                               int64_t outer_step, const Gauss &g, cudaStream_t s) {
     const int64_t lines = (count + 7) / 8 * outer;
-    const int by = (int)std::min<int64_t>((lines + 7) / 8, 65535);
-    const dim3 block(32, 8);
-    if (vec4_ok({in, out}, inner) && step % 4 == 0 && outer_step % 4 == 0)
-        k_gauss_line<4><<<dim3((unsigned)((inner + 127) / 128), by), block, 0, s>>>(in, out, inner, count, step, outer,
-                                                                                   outer_step, g);
+    const bool v4 = vec4_ok({in, out}, inner) && step % 4 == 0 && outer_step % 4 == 0;
+    const int64_t wide = v4 ? inner / 4 : inner;  // threads that have cells side by side
+    int bx = 32;
+    while (bx > 1 && bx / 2 >= wide) bx /= 2;
+    const dim3 block(bx, 256 / bx);
+    const dim3 grid((unsigned)((wide + bx - 1) / bx), (unsigned)std::min<int64_t>((lines + block.y - 1) / block.y, 65535));
+    if (v4)
+        k_gauss_line<4><<<grid, block, 0, s>>>(in, out, inner, count, step, outer, outer_step, g);
     else
-        k_gauss_line<1><<<dim3((unsigned)((inner + 31) / 32), by), block, 0, s>>>(in, out, inner, count, step, outer,
-                                                                                 outer_step, g);
+        k_gauss_line<1><<<grid, block, 0, s>>>(in, out, inner, count, step, outer, outer_step, g);
     return cudaGetLastError();
 }
 
@@ -539,7 +549,7 @@ cudaError_t efm_util_smooth_mask(float *gv, float *tmp, int nx, int ny, int nz, 
     const int64_t n = (int64_t)nx * ny * nz, plane = (int64_t)nx * nz;
     const Mask M = {nx, ny, nz, W, top};
     if (!(sigma > 0.f)) {
-        k_mask<<<grid_for(n), 256, 0, s>>>(gv, M);
+        k_mask<false><<<grid_for(n), 256, 0, s>>>(nullptr, gv, M);
         return cudaGetLastError();
     }
     Gauss g;
@@ -555,16 +565,19 @@ cudaError_t efm_util_smooth_mask(float *gv, float *tmp, int nx, int ny, int nz, 
     cudaError_t e;
     if ((e = gauss_line(gv, tmp, plane, ny, plane, 1, 0, g, s))) return e;
     if ((e = gauss_line(tmp, gv, nx, nz, nx, ny, plane, g, s))) return e;
-    const int row = (nx + 2 * radius) * (int)sizeof(float), smem = 48 * 1024;
-    if (row <= smem) {
-        const int warps = std::max(1, std::min(8, smem / row));
-        k_gauss_row_mask<<<grid_for((int64_t)ny * nz * 256 / warps), warps * 32, warps * row, s>>>(gv, M, g);
+    // Along x: rows in shared memory, where a row gives a warp work and the rows give the device
+    // warps; otherwise lines of neighbouring cells out of place (us for sigma 1 and 4, rows | lines:
+    // 400 x 400 rows of 16 cells 76, 192 | 48, 75, of 32 85, 209 | 75, 123, of 48 97, 233 | 101, 173;
+    // 100 x 100 rows of 2000 164, 343 | 239, 419, of 4000 406, 851 | 460, 815, of 8000 1198, 2636 |
+    // 892, 1593; 8 x 8 rows of 500 22, 34 | 27, 32, of 2000 33, 63 | 28, 33).
+    const int64_t rows = (int64_t)ny * nz;
+    if (nx > 32 && nx <= 4096 && 8 * rows >= nx) {
+        const int row = (nx + 2 * radius) * (int)sizeof(float), warps = std::min(8, 48 * 1024 / row);
+        k_gauss_row_mask<<<grid_for(rows * 256 / warps), warps * 32, warps * row, s>>>(gv, M, g);
         return cudaGetLastError();
     }
-    // rows longer than 12000 cells: x as lines of neighbouring cells, out of place
-    if ((e = gauss_line(gv, tmp, 1, nx, 1, (int64_t)ny * nz, nx, g, s))) return e;
-    if ((e = cudaMemcpyAsync(gv, tmp, n * sizeof(float), cudaMemcpyDeviceToDevice, s))) return e;
-    k_mask<<<grid_for(n), 256, 0, s>>>(gv, M);
+    if ((e = gauss_line(gv, tmp, 1, nx, 1, rows, nx, g, s))) return e;
+    k_mask<true><<<grid_for(n), 256, 0, s>>>(tmp, gv, M);
     return cudaGetLastError();
 }
 
