@@ -249,14 +249,13 @@ k_lbfgs_solve(const double *__restrict__ G, double *__restrict__ w, int L, int u
 }
 
 // r = gamma g - sum_k gamma eps_k y_k + sum_k coef_k s_k
-// (SH: the coefficients in shared memory; more than 2048 pairs read them from w.)
-template <int V, bool SH>
+template <int V>
 __global__ void __launch_bounds__(256)
 k_lbfgs_combine(const float *__restrict__ s1, const float *__restrict__ y1, const float *g, float *r,
                 const double *__restrict__ w, int L, int used, int64_t n) {
     extern __shared__ double sh[];  // [used] of y, [used] of s
     const double gamma = w[3];
-    for (int k = threadIdx.x; SH && k < used; k += 256) {
+    for (int k = threadIdx.x; k < used; k += 256) {
         sh[k] = -gamma * w[4 + L + k];
         sh[used + k] = w[4 + 2 * L + k];
     }
@@ -269,7 +268,7 @@ k_lbfgs_combine(const float *__restrict__ s1, const float *__restrict__ y1, cons
 #pragma unroll 4
         for (int k = 0; k < used; ++k) {
             const Vec<V> vy = vload<V>(y1 + k * n + i), vs = vload<V>(s1 + k * n + i);
-            const double cy = SH ? sh[k] : -gamma * w[4 + L + k], cs = SH ? sh[used + k] : w[4 + 2 * L + k];
+            const double cy = sh[k], cs = sh[used + k];
 #pragma unroll
             for (int v = 0; v < V; ++v) acc[v] += cy * (double)vy.a[v] + cs * (double)vs.a[v];
         }
@@ -278,6 +277,43 @@ k_lbfgs_combine(const float *__restrict__ s1, const float *__restrict__ y1, cons
         for (int v = 0; v < V; ++v) o.a[v] = (float)acc[v];
         vstore<V>(r + i, o);
     }
+}
+
+// The recursion vector by vector, for histories whose products cost more (by_products).  The
+// direction is read, changed and written once per vector.  w as in k_lbfgs_solve, [2] the last dot.
+enum { LB_GAMMA, LB_SIGMA, LB_EPS };
+
+__global__ void k_lbfgs_scalar(double *w, int L, int k, int what) {
+    if (what == LB_GAMMA) w[3] = w[0] == 0.0 ? 0.0 : w[1] / w[0];
+    if (what == LB_SIGMA) w[4 + k] = w[2] == 0.0 ? 0.0 : 1.0 / w[2];
+    if (what == LB_EPS) w[4 + L + k] = w[4 + k] * w[2];
+}
+
+__global__ void k_lbfgs_bounds(int64_t *seg, int64_t n) {
+    seg[0] = 0;
+    seg[1] = n;
+}
+
+// q -= eps_k y   (first loop)
+__global__ void k_lbfgs_axpy1(float *__restrict__ q, const float *__restrict__ y, const double *__restrict__ w, int L,
+                              int k, int64_t n) {
+    const double e = w[4 + L + k];
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        q[i] = (float)((double)q[i] - e * (double)y[i]);
+}
+
+__global__ void k_lbfgs_scale(float *__restrict__ r, const double *__restrict__ w, int64_t n) {
+    const double gmm = w[3];
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        r[i] = (float)(gmm * (double)r[i]);
+}
+
+// r += s_k (eps_k - sigma_k w[2]), w[2] = y_k . r   (second loop)
+__global__ void k_lbfgs_axpy2(float *__restrict__ r, const float *__restrict__ s, const double *__restrict__ w, int L,
+                              int k, int64_t n) {
+    const double coef = w[4 + L + k] - w[4 + k] * w[2];
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        r[i] = (float)((double)r[i] + (double)s[i] * coef);
 }
 
 // ------------------------------------------------------------------- smoothing + mask
@@ -459,6 +495,22 @@ bool vec4_ok(std::initializer_list<const float *> p, int64_t n) {
 // Blocks per pair of groups: three waves of the device, shared by the pairs.
 int gram_blocks(int T) { return std::max(8, 6 * 148 / T); }
 
+// Whether the products of u pairs take less time than the recursion vector by vector.  A pair of
+// groups costs the products 24 vectors' reads (17 on the diagonal) whatever the groups hold; the
+// recursion takes seven launches and twelve reads and writes of a vector per pair of vectors, from
+// L2 while a few of them fit.  us measured, products and vectors: 4 000 000 cells, 65 pairs 3627, 4313;
+// 81 pairs 5717, 5401; 97 pairs 7693, 6397; rows off 16 bytes, 65 pairs 4593, 4305; 1 000 000 cells,
+// 199 pairs 5688, 8987; 32 000 000 cells, 33 pairs 9954, 11483; 41 pairs 14244, 14224; 64 000 000
+// cells, 1 pair 1035, 993.  Beyond MAX_PRODUCTS pairs the products' scratch would pass 90 MB.
+constexpr int MAX_PRODUCTS = 1024;
+
+bool by_products(int u, int64_t n, bool v4) {
+    if (u > MAX_PRODUCTS) return false;
+    const double cells = (double)n, groups = gram_groups(u), reads = 17 * groups + 12 * groups * (groups - 1);
+    const double products = cells * (8.8e-7 * (v4 ? 1 : 1.2) * reads + 6.2e-7 * (2 * u + 2));
+    return products <= 30 + 4.2e-6 * cells + u * std::max(37 + 7.2e-6 * cells, 25 + 1e-5 * cells);
+}
+
 }  // namespace
 
 // ------------------------------------------------------------------------- entry points
@@ -496,10 +548,38 @@ cudaError_t efm_util_lbfgs_history(float *sk, float *yk, const float *m, const f
     return cudaGetLastError();
 }
 
-// Doubles of scratch a direction of L layers needs: per product, the blocks' parts and their sum.
+// Doubles of scratch a direction of L layers needs: per product, the blocks' parts and their sum
+// (more than what the recursion by vectors uses, the parts of one dot and its bounds).
 int64_t efm_util_lbfgs_scratch(int L) {
-    const int64_t T = gram_tiles(L - 1);
+    const int64_t T = gram_tiles(std::min(L - 1, MAX_PRODUCTS));
     return T * GT + std::max<int64_t>(8 * T, 6 * 148) * GT;
+}
+
+static cudaError_t lbfgs_by_vectors(const float *s1, const float *y1, const float *g, float *r, double *w, int L,
+                                    int64_t n, int used, double *scratch, cudaStream_t s) {
+    const int gb = grid_for(n);
+    int64_t *const seg = reinterpret_cast<int64_t *>(scratch + EFM_RED_BLOCKS);
+    cudaError_t e;
+    auto dot = [&](const float *a, const float *b, double *out) {
+        return efm_util_reduce(a, b, nullptr, seg, 1, 1, 1.0, scratch, EFM_RED_BLOCKS, out, s);
+    };
+    k_lbfgs_bounds<<<1, 1, 0, s>>>(seg, n);
+    if ((e = dot(y1, y1, w + 0)) || (e = dot(s1, y1, w + 1))) return e;
+    k_lbfgs_scalar<<<1, 1, 0, s>>>(w, L, 0, LB_GAMMA);
+    if (r != g && (e = cudaMemcpyAsync(r, g, n * sizeof(float), cudaMemcpyDeviceToDevice, s))) return e;
+    for (int k = 0; k < used; ++k) {
+        if ((e = dot(y1 + k * n, s1 + k * n, w + 2))) return e;
+        k_lbfgs_scalar<<<1, 1, 0, s>>>(w, L, k, LB_SIGMA);
+        if ((e = dot(s1 + k * n, r, w + 2))) return e;
+        k_lbfgs_scalar<<<1, 1, 0, s>>>(w, L, k, LB_EPS);
+        k_lbfgs_axpy1<<<gb, 256, 0, s>>>(r, y1 + k * n, w, L, k, n);
+    }
+    k_lbfgs_scale<<<gb, 256, 0, s>>>(r, w, n);
+    for (int k = used - 1; k >= 0; --k) {
+        if ((e = dot(y1 + k * n, r, w + 2))) return e;
+        k_lbfgs_axpy2<<<gb, 256, 0, s>>>(r, s1 + k * n, w, L, k, n);
+    }
+    return cudaGetLastError();
 }
 
 cudaError_t efm_util_lbfgs_direction(const float *sk, const float *yk, const float *g, float *r,
@@ -507,10 +587,11 @@ cudaError_t efm_util_lbfgs_direction(const float *sk, const float *yk, const flo
                                      cudaStream_t s) {
     const int used = iter < L ? iter : L - 1;
     const int u = used > 0 ? used : 1;  // (gamma takes the newest pair also before any is used)
+    const bool v4 = vec4_ok({sk, yk, g, r}, n);
+    if (!by_products(u, n, v4)) return lbfgs_by_vectors(sk + n, yk + n, g, r, w, L, n, used, scratch, s);
     const int T = gram_tiles(u);
     const int nblk = gram_blocks(T);
     const dim3 grid(T, nblk);
-    const bool v4 = vec4_ok({sk, yk, g, r}, n);
     if (v4)
         k_lbfgs_gram<4><<<grid, 256, 0, s>>>(sk + n, yk + n, g, n, u, scratch);
     else
@@ -518,13 +599,11 @@ cudaError_t efm_util_lbfgs_direction(const float *sk, const float *yk, const flo
     double *G = scratch + (int64_t)T * GT * nblk;
     k_finish<<<T * GT, RB, 0, s>>>(scratch, nblk, 1.0, G);
     k_lbfgs_solve<<<1, 128, 0, s>>>(G, w, L, u, used);
-    const int csh = used <= 2048 ? 2 * used * (int)sizeof(double) : 0;
-    if (v4 && used <= 2048)
-        k_lbfgs_combine<4, true><<<grid_for(n / 4), 256, csh, s>>>(sk + n, yk + n, g, r, w, L, used, n);
-    else if (used <= 2048)
-        k_lbfgs_combine<1, true><<<grid_for(n), 256, csh, s>>>(sk + n, yk + n, g, r, w, L, used, n);
+    const int csh = 2 * used * (int)sizeof(double);
+    if (v4)
+        k_lbfgs_combine<4><<<grid_for(n / 4), 256, csh, s>>>(sk + n, yk + n, g, r, w, L, used, n);
     else
-        k_lbfgs_combine<1, false><<<grid_for(n), 256, 0, s>>>(sk + n, yk + n, g, r, w, L, used, n);
+        k_lbfgs_combine<1><<<grid_for(n), 256, csh, s>>>(sk + n, yk + n, g, r, w, L, used, n);
     return cudaGetLastError();
 }
 

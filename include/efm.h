@@ -317,7 +317,9 @@ EFM_API int efm_lbfgs_history(float *sk_dev, float *yk_dev, const float *m_dev, 
 /*
  * lbfgs.L_BFGS (lbfgs.py:27-67) on device: two-loop recursion r = H g with
  * gamma = s1.y1 / y1.y1, carried out on the inner products of the history and g, which are
- * formed in one pass in float64; scalars stay on the device.
+ * formed in one pass in float64, or vector by vector (rounded to float32 after every step) where
+ * the products would take longer: long histories of large vectors, more than 1024 pairs.  Scalars
+ * stay on the device.
  * work_dev: at least 4 * layers + 8 doubles of scratch.
  */
 EFM_API int efm_lbfgs_direction(const float *sk_dev, const float *yk_dev, const float *g_dev,
