@@ -1,30 +1,34 @@
 """Autotuner for the plane-streaming kernels' launch shape, with a JSON cache.
 
-Three knobs decide how the stress/velocity kernels map a batch onto the 148 SMs: the tile
-height (``EFM_OPT_TILE_ROWS``: 64 x 8 tiles with two cells per thread and two blocks per SM,
-or 64 x 4 tiles with one cell per thread), the shared-memory ring depth
-(``EFM_OPT_RING_DEPTH``: 4, or 6 with one-row tiles -- more planes in flight, fewer blocks)
-and the planes each block marches along y (``EFM_OPT_YCHUNK``; 0 = the wave-filling
-heuristic).  :func:`tune` times a
+Three knobs decide how the passes map a batch onto the 148 SMs: the block size
+(``EFM_OPT_TILE_ROWS``: 2, tiles of up to 448 cells with two blocks per SM, or 1, up to 192 cells
+with four), the shared-memory ring depth (``EFM_OPT_RING_DEPTH``: 4, or 6 with the small blocks --
+more planes in flight, three blocks per SM) and the planes per chunk (``EFM_OPT_YCHUNK``; 0 = the
+library's cost rule, per launch).  :func:`tune` times a
 short probe of the batch -- the same grids, sources and receivers, ``nt_probe`` steps of
 forward (with strips) + misfit + model/MT gradient -- for every candidate, applies the
-fastest to the batch and caches it under a key made of the device name and the instance
-geometries, so later batches of the same shape skip the probe.
+fastest to the batch and caches it under a key made of the device name, the kernels' sources
+and the instance geometries, so later batches of the same shape skip the probe and a choice made
+for other kernels is not taken.
 
 Cache file: ``$EFM_AUTOTUNE_CACHE``, else ``~/.cache/elastic_fm_vp_vs_rho_b200/autotune.json``.
 """
 from __future__ import annotations
 
+import hashlib
 import json
 import os
 
 import numpy as np
 
 from . import _lib
+from .ncu_traffic import CSRC, STENCIL_SOURCES
 
-# (tile rows, ring depth, y-chunk)
+# (tile rows, ring depth, planes per chunk).  The rule (0) was the best of all lengths or within
+# 0.5 % of it on eight grids of 64^3 to 256 x 256 x 128 and four of 200 x 200 x 100; of the set ones 3 to 8
+# planes came next (160 x 128 x 100, 5 planes: 0.995 of the rule's time).
 DEFAULT_CANDIDATES = tuple((rows, ring, yc) for rows, ring in ((2, 4), (1, 4), (1, 6))
-                           for yc in (0, 8, 16, 32))
+                           for yc in (0, 4, 5, 8))
 
 
 def cache_path() -> str:
@@ -35,11 +39,20 @@ def cache_path() -> str:
                         "autotune.json")
 
 
+def kernels(csrc=CSRC) -> str:
+    """Which kernels a choice belongs to: a hash of the streaming kernels and the rules that launch them."""
+    h = hashlib.sha256()
+    for name in (*STENCIL_SOURCES, "efm_capi.cu"):
+        with open(os.path.join(csrc, name), "rb") as f:
+            h.update(f.read())
+    return h.hexdigest()[:16]
+
+
 def batch_key(batch) -> str:
     import torch
     dev = torch.cuda.get_device_name() if torch.cuda.is_available() else "cpu"
     geo = sorted((s["nx"], s["ny"], s["nz"], s["lenpml"]) for s in batch.specs)
-    return json.dumps({"device": dev, "grids": geo}, sort_keys=True)
+    return json.dumps({"device": dev, "kernels": kernels(), "grids": geo}, sort_keys=True)
 
 
 def load_cache(path=None) -> dict:
