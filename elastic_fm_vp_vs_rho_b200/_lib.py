@@ -36,6 +36,7 @@ EFM_OPT_GRAPH = 8
 EFM_OPT_WAIT_LIMIT = 9
 EFM_OPT_EXACT_FORM = 10
 EFM_OPT_EXACT_FUSED = EFM_OPT_EXACT_FORM
+EFM_OPT_EXACT_SHAPE = 11
 EFM_EXACT_TWO_PASS, EFM_EXACT_GATHER, EFM_EXACT_STREAM = 0, 1, 2
 EFM_NKERN = 11
 KERNEL_NAMES = ("fwd_stress", "fwd_velocity", "adj_stress", "adj_velocity", "rev_velocity",

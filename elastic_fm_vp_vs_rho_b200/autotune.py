@@ -77,6 +77,8 @@ def apply(batch, choice: dict):
     batch.set_option(_lib.EFM_OPT_TILE_ROWS, int(choice["rows"]))
     batch.set_option(_lib.EFM_OPT_RING_DEPTH, int(choice.get("ring", 4)))
     batch.set_option(_lib.EFM_OPT_YCHUNK, int(choice["ychunk"]))
+    # (timed with the stencil passes: the exact adjoint keeps choosing its own tiles and chunks)
+    batch.set_option(_lib.EFM_OPT_EXACT_SHAPE, 1)
 
 
 def _probe(batch, nt_probe):

@@ -183,6 +183,7 @@ struct efm_ctx {
     unsigned int opt_wait = 0;  // polls per tile wait (0: the kernels' default bound)
     int opt_exact_form = 2;     // exact adjoint: 0 per-cell + gather launches, 1 one gather
                                 // launch, 2 one plane-streaming launch per transposed half-step
+    int opt_exact_shape = 0;    // its tiles and chunks: 0 opt_rows / opt_ychunk where set, 1 its own
     // kernel kinds whose device tables (and tensor maps) are loaded now, for efm_kernel_time,
     // and the step count of those tables
     unsigned int timeable = 0;
@@ -498,11 +499,10 @@ Active active(const efm_ctx *ctx, int slot, int it) {
     return {n, n ? ctx->cum[slot][n - 1] : 0};
 }
 
-// Planes per block of the kernels that march one chunk per block (imaging, exact adjoint): the
-// chunk that fills whole waves of blocks best, for tiles of tx x tz cells and `per_sm` resident
-// blocks per SM.
+// Planes per block of the exact adjoint, whose blocks march one chunk each: the chunk that fills
+// whole waves of blocks best, for tiles of tx x tz cells and `per_sm` resident blocks per SM.
 int choose_ychunk(const efm_ctx *ctx, int tz, int per_sm, int tx) {
-    if (ctx->opt_ychunk > 0) return ctx->opt_ychunk;
+    if (ctx->opt_ychunk > 0 && !ctx->opt_exact_shape) return ctx->opt_ychunk;
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess)
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -997,8 +997,9 @@ int exact_gradient(efm_ctx *ctx, const float *res, float *grad, double *mtg, boo
     int tiles = 0, st_tiles = 0;
     // 32 x 16 tiles, or 32 x 8 where those would not fill the device even with the shortest chunks
     // (48 x 48 x 40, 72 blocks: 29.3 ms a gradient, 27.2 with 32 x 8; 128 x 128 x 96: 85.4, 106)
-    int xs_rows = ctx->opt_rows == 1 ? 1 : 2;
-    if (ctx->opt_rows == 0) {
+    const int rows = ctx->opt_exact_shape ? 0 : ctx->opt_rows;
+    int xs_rows = rows == 1 ? 1 : 2;
+    if (rows == 0) {
         double blocks = 0;
         const int tz = efm_exact_stream_tz(2);
         for (const Inst &I : ctx->inst)
@@ -1730,6 +1731,7 @@ int efm_set_option(efm_ctx *ctx, int option, int value) {
             if (value < 0 || value > 2) return fail(EFM_ERR_ARG, "EFM_OPT_EXACT_FORM must be 0, 1 or 2");
             ctx->opt_exact_form = value;
             break;
+        case EFM_OPT_EXACT_SHAPE: ctx->opt_exact_shape = value != 0; break;
         case EFM_OPT_WAIT_LIMIT:
             if (value < 0) return fail(EFM_ERR_ARG, "wait limit must be >= 0 (0 = default)");
             ctx->opt_wait = (unsigned int)value;

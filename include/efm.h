@@ -239,7 +239,7 @@ EFM_API int efm_residual_misfit_noalloc(const float *mod_dev, const float *obs_d
 /* EFM_GRAD_EXACT: how each transposed half-step runs.  2 (default): one plane-streaming
  * launch (each block marches a 32 x 16 column of cells along y, or 32 x 8 with
  * EFM_OPT_TILE_ROWS = 1 or, at 0, on grids too small for the wider ones; y-chunk from
- * EFM_OPT_YCHUNK or chosen for full waves); 0: a
+ * EFM_OPT_YCHUNK or chosen for full waves; see EFM_OPT_EXACT_SHAPE); 0: a
  * per-cell pass into scratch volumes + a gather launch; 1: one gather launch that recomputes
  * its neighbours' terms.  Same expressions in every form; the streaming form adds a few
  * terms in another order (no reference counterpart: the reference has no exact adjoint). */
@@ -248,6 +248,11 @@ EFM_API int efm_residual_misfit_noalloc(const float *mod_dev, const float *obs_d
 #define EFM_EXACT_TWO_PASS 0
 #define EFM_EXACT_GATHER 1
 #define EFM_EXACT_STREAM 2
+/* Tiles and y-chunks of the exact adjoint's streaming form: 0 (default): as EFM_OPT_TILE_ROWS and
+ * EFM_OPT_YCHUNK say where they are set; 1: chosen for the grid whatever those say.  The two
+ * options are timed for the stencil passes, whose blocks and chunks mean something else (the
+ * autotuner sets 1; no reference counterpart). */
+#define EFM_OPT_EXACT_SHAPE 11
 EFM_API int efm_set_option(efm_ctx *ctx, int option, int value);
 
 /*
