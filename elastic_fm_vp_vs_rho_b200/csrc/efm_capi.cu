@@ -66,8 +66,8 @@ struct Inst {
     uint32_t *rec_mask = nullptr;
     int *rec_lin = nullptr, *rec_id = nullptr;
     int *rec_wfirst = nullptr;    // per mask word: first sorted entry of its cells, or -1
-    uint8_t *rec_col = nullptr;   // [tile][ny] of the streaming layout rec_shape
-    int rec_shape[6] = {};        // tw th ox oz tiles_x tiles_z rec_col was built for
+    uint8_t *rec_col = nullptr;   // [tile][ny] of the velocity pass's tiles, large blocks' and small ones'
+    size_t rec_small = 0;         // where the small blocks' begin
     float *aux = nullptr;         // 1/mu, 1/rho
     float *fields = nullptr;  // va(3) t(6) | vb(3) bv(3) bt(6) when gradient-capable
     bool fields_grad = false;
@@ -176,8 +176,9 @@ struct efm_ctx {
     int opt_ring = 0;
     int opt_pair = 1;
     int opt_pdl = 1;
-    int rows = 2;  // cells per thread of the tables last built for the streaming kernels
+    int rows = 2;  // block size (EFM_OPT_TILE_ROWS) of the tables last built for the streaming kernels
     int ring = 4;  // ring depth of those tables' kernels
+    int slots = 0;  // blocks of them that fill the device
     int opt_ck_every = 0;       // 0: the longest interval whose workspace fits (checkpoint_interval)
     int ck_auto = 0;            // that interval, chosen at the first allocation for the instance set
     unsigned int opt_wait = 0;  // polls per tile wait (0: the kernels' default bound)
@@ -847,24 +848,27 @@ Region box_region(const Inst &I) {
     return {I.W / 4 * 4, I.nx - I.W, EFM_HS, I.nz - I.W, I.W, I.ny - I.W};
 }
 
-// Receiver map of the tiles of a velocity table entry, rebuilt when their shape changes.
-int ensure_rec_col(Inst &I, EfmInst &d, cudaStream_t s) {
-    const int shape[6] = {d.tw, d.th, d.ox, d.oz, d.tiles_x, d.tiles_z};
-    if (I.rec_col == nullptr || std::memcmp(shape, I.rec_shape, sizeof(shape)) != 0) {
-        std::vector<uint8_t> m((size_t)d.tiles_x * d.tiles_z * I.ny, 0);
+// The velocity pass's tiles and their receiver map, for either block size.
+void layout_velocity(EfmInst &d, const Inst &I, int nt) {
+    layout_stream(d, velocity_region(I), nt);
+    d.rec_col = I.rec_col + (nt == efm_st_nt(1) ? I.rec_small : 0);
+}
+
+// Both maps (the model calls neither allocate nor wait for them).
+std::vector<uint8_t> receiver_maps(Inst &I) {
+    std::vector<uint8_t> m;
+    for (int rows : {2, 1}) {
+        EfmInst d = {};
+        layout_stream(d, velocity_region(I), efm_st_nt(rows));
+        const size_t at = m.size();
+        if (rows == 1) I.rec_small = at;
+        m.resize(at + (size_t)d.tiles_x * d.tiles_z * I.ny, 0);
         for (int r = 0; r < I.nrec; ++r) {
             const int tx = (I.rec[3 * r] - d.ox) / d.tw, tz = (I.rec[3 * r + 2] - d.oz) / d.th;
-            m[((size_t)tz * d.tiles_x + tx) * I.ny + I.rec[3 * r + 1]] = 1;
+            m[at + ((size_t)tz * d.tiles_x + tx) * I.ny + I.rec[3 * r + 1]] = 1;
         }
-        EFM_CK(cudaStreamSynchronize(s));  // launches in flight may still read the old map
-        cudaFree(I.rec_col);
-        I.rec_col = nullptr;
-        EFM_CK(cudaMalloc(&I.rec_col, m.size()));
-        EFM_CK(cudaMemcpy(I.rec_col, m.data(), m.size(), cudaMemcpyHostToDevice));
-        std::memcpy(I.rec_shape, shape, sizeof(shape));
     }
-    d.rec_col = I.rec_col;
-    return EFM_OK;
+    return m;
 }
 
 // Forward tables (slots T_FWD_S, T_FWD_V) and tensor maps; gathers / strips optional.
@@ -877,6 +881,7 @@ int prepare_forward(efm_ctx *ctx, float *gathers, bool strips, bool recips, cuda
     efm_stream_set_pdl(ctx->opt_pdl);
     const int rows = ctx->rows = ctx->opt_rows == 1 ? 1 : 2;
     ctx->ring = (rows == 1 && ctx->opt_ring == 6) ? 6 : 4;
+    const int slots = ctx->slots = efm_stream_slots(rows, ctx->ring);
     const int nt = efm_st_nt(rows);
     std::vector<EfmInst> tab(2 * (size_t)n);
     std::vector<CUtensorMap> maps(st ? (size_t)n * EFM_MAPS_PER_INST : 0);
@@ -894,8 +899,7 @@ int prepare_forward(efm_ctx *ctx, float *gathers, bool strips, bool recips, cuda
         EfmInst ds = d, dv = d;
         if (st) {
             layout_stream(ds, stress_region(I), nt);
-            layout_stream(dv, velocity_region(I), nt);
-            if ((rc = ensure_rec_col(I, dv, s))) return rc;
+            layout_velocity(dv, I, nt);
             CUtensorMap *m = maps.data() + (size_t)i * EFM_MAPS_PER_INST;
             const float *v[3] = {I.va(0), I.va(1), I.va(2)};
             const float *t[6] = {I.tt(0), I.tt(1), I.tt(2), I.tt(3), I.tt(4), I.tt(5)};
@@ -914,7 +918,6 @@ int prepare_forward(efm_ctx *ctx, float *gathers, bool strips, bool recips, cuda
         for (const EfmInst &e : tab)
             if (!fields_contiguous(e)) return fail(EFM_ERR_STATE, "field volumes not contiguous");
     if (st) {
-        const int slots = efm_stream_slots(rows, ctx->ring);
         finish_stream(ctx, T_FWD_S, tab.data(), n, chunk_planes(ctx, {tab.data()}, n, slots));
         finish_stream(ctx, T_FWD_V, tab.data() + n, n, chunk_planes(ctx, {tab.data() + n}, n, slots));
     } else {
@@ -945,7 +948,7 @@ cudaError_t launch_stream(const efm_ctx *ctx, int ps, int ss, int pv, int sv, bo
     const size_t n = ctx->inst.size();
     return efm_launch_stream(ps, pv, illum, ctx->rows, ctx->ring, ctx->d_tab + (ps >= 0 ? ss : 0) * n, a.n, a.chunks,
                              ctx->d_tab + (pv >= 0 ? sv : 0) * n, b.n, b.chunks,
-                             std::min(a.chunks + b.chunks, efm_stream_slots(ctx->rows, ctx->ring)), it, ctx->d_count,
+                             std::min(a.chunks + b.chunks, ctx->slots), it, ctx->d_count,
                              ctx->opt_wait, ctx->d_err, s);
 }
 
@@ -1356,6 +1359,9 @@ int efm_add_instance(efm_ctx *ctx, const efm_instance_desc *d, int *id) {
     if ((e = cudaMemcpy(I.rec_id, rid.data(), I.nrec * sizeof(int), cudaMemcpyHostToDevice))) return bad(e);
     if ((e = cudaMemcpy(I.rec_wfirst, wfirst.data(), wfirst.size() * sizeof(int), cudaMemcpyHostToDevice)))
         return bad(e);
+    const std::vector<uint8_t> rm = receiver_maps(I);
+    if ((e = cudaMalloc(&I.rec_col, rm.size()))) return bad(e);
+    if ((e = cudaMemcpy(I.rec_col, rm.data(), rm.size(), cudaMemcpyHostToDevice))) return bad(e);
     ctx->inst.push_back(std::move(I));
     ctx->ck_auto = 0;  // the automatic checkpoint interval is chosen for the new instance set
     ctx->layout_ready = false;
@@ -1513,6 +1519,7 @@ int efm_gradient(efm_ctx *ctx, const float *res, float *grad, double *mtg, int f
     if (st && model && !aligned16(grad)) return fail(EFM_ERR_CUDA, "the gradient buffer must start on 16 bytes");
     const int rows = ctx->rows = ctx->opt_rows == 1 ? 1 : 2;
     ctx->ring = (rows == 1 && ctx->opt_ring == 6) ? 6 : 4;
+    const int slots = ctx->slots = efm_stream_slots(rows, ctx->ring);
     const int nt = efm_st_nt(rows);
     std::vector<EfmInst> tab((size_t)T_NSLOT * n);
     std::vector<CUtensorMap> maps(st ? (size_t)n * EFM_MAPS_PER_INST : 0);
@@ -1538,8 +1545,7 @@ int efm_gradient(efm_ctx *ctx, const float *res, float *grad, double *mtg, int f
         EfmInst as = a, av = a;
         if (st) {
             layout_stream(as, stress_region(I), nt);
-            layout_stream(av, velocity_region(I), nt);
-            if ((rc = ensure_rec_col(I, av, s))) return rc;
+            layout_velocity(av, I, nt);
             const float *v[3] = {I.bv(0), I.bv(1), I.bv(2)};
             const float *t[6] = {I.bt(0), I.bt(1), I.bt(2), I.bt(3), I.bt(4), I.bt(5)};
             if ((rc = stress_maps(m + M_ADJ_S, I, as, v, t)) || (rc = velocity_maps(m + M_ADJ_V, I, av, v, t)))
@@ -1609,7 +1615,6 @@ int efm_gradient(efm_ctx *ctx, const float *res, float *grad, double *mtg, int f
     if (st) {
         // a pair's tables share a launch's rounds; by themselves (300 x 44 x 52, a gradient step with
         // the pair's chunks: 100 us, with their own 82) each has its own
-        const int slots = efm_stream_slots(rows, ctx->ring);
         const bool pairs = model && ctx->opt_pair;
         for (int q = 0; q < 2; ++q) {
             EfmInst *a = &slot(q ? T_ADJ_V : T_ADJ_S, 0), *r = &slot(q ? T_REV_S0 : T_REV_V0, 0);
