@@ -891,8 +891,9 @@ __device__ __forceinline__ int velocity_chunk(int packed, int ib, int it) {
 #pragma unroll
                         for (int v = 0; v < VX; ++v) {
                             const float nvx = o[0].v[v], nvy = o[1].v[v], nvz = o[2].v[v];
-                            if (p.in(v))
-                                I.illum[p.x + v + I.nx * (p.z + I.nz * j)] += nvx * nvx + nvy * nvy + nvz * nvz;
+                            if (!p.in(v)) continue;
+                            float *const e = I.illum + (p.x + v + I.nx * (p.z + I.nz * j));
+                            *e = __fadd_rn(*e, __fmaf_rn(nvz, nvz, two_products(nvy, nvy, nvx, nvx)));
                         }
                     }
                     // the strips the pair's box cells belong to (sf is zero without strips)
