@@ -470,7 +470,7 @@ __global__ void __launch_bounds__(256) k_adam(AdamArgs A) {
     for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < A.n[k]; i += (int64_t)gridDim.x * 256) {
         const float a = g[i];
         const float mi = __fmaf_rn(A.alpha1, a, __fmul_rn(m[i], A.beta1));
-        const float vi = __fmaf_rn(__fmul_rn(A.alpha2, a), a, __fmul_rn(v[i], A.beta2));
+        const float vi = __fmaf_rn(A.alpha2, __fmul_rn(a, a), __fmul_rn(v[i], A.beta2));
         m[i] = mi;
         v[i] = vi;
         const float d = __fadd_rn(__fsqrt_rn(__fmul_rn(vi, A.r2)), A.eps);
@@ -687,8 +687,8 @@ cudaError_t efm_util_adam(int count, float *const *p, const float *const *g, flo
         A.alpha1 = (float)(1.0 - beta1);
         A.alpha2 = (float)(1.0 - beta2);
         A.eps = (float)eps;
-        A.r1 = 1.f / (float)c1;
-        A.r2 = 1.f / (float)c2;
+        A.r1 = (float)(1.0 / c1);
+        A.r2 = (float)(1.0 / c2);
         k_adam<<<dim3(grid_for(most), k1), 256, 0, s>>>(A);
     }
     return cudaGetLastError();

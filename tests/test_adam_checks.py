@@ -121,3 +121,22 @@ def test_moments_and_updates_to_their_own_scale(cuda):
             assert float((a.cpu().double() - b).abs().max()) <= 1e-6 * float(b.abs().max())
         change = float((r - s).abs().max())
         assert float((p.cpu().double() - r).abs().max()) <= 2e-6 * change + 3 * 2.0**-24 * float(r.abs().max())
+
+
+@pytest.mark.gpu
+def test_one_launch_rounds_as_the_tensor_operations_do(cuda):
+    """Bit for bit what the elementwise operations give, moments and parameters, over five steps."""
+    gen = cuda.Generator(device="cuda").manual_seed(7)
+    net = precond.PreconditionerNet(widths=(16, 32, 16))
+    ref = [p.clone() for p in net.parameters()]
+    mom = [(cuda.zeros_like(p), cuda.zeros_like(p)) for p in ref]
+    lr, b1, b2, eps = 1e-2, 0.9, 0.999, 1e-8
+    for step in range(1, 6):
+        gs = [0.1 * cuda.randn(p.shape, device="cuda", generator=gen) for p in ref]
+        net.adam_step([(gs[i], gs[i + 1]) for i in range(0, len(gs), 2)], lr=lr)
+        for p, g, (m, v) in zip(ref, gs, mom):
+            m.mul_(b1).add_(g, alpha=1.0 - b1)
+            v.mul_(b2).addcmul_(g, g, value=1.0 - b2)
+            p.addcdiv_(m / (1.0 - b1**step), (v / (1.0 - b2**step)).sqrt_().add_(eps), value=-lr)
+    for p, r, (m, v), (m2, v2) in zip(net.parameters(), ref, net._adam, mom):
+        assert cuda.equal(m, m2) and cuda.equal(v, v2) and cuda.equal(p, r)
