@@ -378,7 +378,8 @@ struct Region {
 // The tile of at most 2 nt cells that covers a region's planes at least cost: per tile the cells,
 // a third for the neighbour columns and rows they load, and a fixed part as large as a full tile
 // (a plane takes a block nearly the same time whatever it holds).  128 x 92: 28 tiles of 64 x 7,
-// forward stress and velocity 22.4 and 26.0 us; 31 tiles of 128 x 3, 28.0 and 32.6.
+// forward stress and velocity 22.1 and 23.1 us; 31 tiles of 128 x 3, 24.0 and 25.4; 32 of 32 x 13, 24.1
+// and 25.2.
 void shape_of(const Region &r, int nt, int *tw, int *th) {
     double best = 1e30;
     *tw = 64;
@@ -420,8 +421,8 @@ void layout_stream(EfmInst &d, const Region &r, int nt, const int *shape = nullp
 // the launch lasts the rounds of chunks; a single round also lasts its slowest (CPML) chunk.
 // Larger grids wait for DRAM: the first slot loads about 0.45 of a plane's bytes, and the blocks
 // finish within most of a chunk of each other.  Forward stress, us: 128 x 128 x 96, 4 planes
-// 23.7, 6 planes 22.4 (two rounds), 8 planes 26.7, 16 planes (one round) 27.5; 256 x 256 x 128,
-// 4 planes 105.5, 8 planes 103.9, 16 planes 108.3; the rule takes 6 and 8.
+// 23.6, 6 planes 21.8 (two rounds), 8 planes 26.5, 16 planes (one round) 25.9; 256 x 256 x 128,
+// 4 planes 104.3, 8 planes 102.4, 16 planes 106.4; the rule takes 6 and 8.
 int chunk_planes(const efm_ctx *ctx, std::initializer_list<const EfmInst *> tables, int n, int slots) {
     if (ctx->opt_ychunk > 0) return ctx->opt_ychunk;
     double cells = 0;

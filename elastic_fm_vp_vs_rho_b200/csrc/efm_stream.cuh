@@ -5,9 +5,12 @@
 // and pair) of every plane.  Two block sizes are built: 224 consumer threads (tiles up to 448
 // cells, two blocks per SM) and 96 (up to 192 cells, four): with the producer warp that is 16
 // warps per SM, four per scheduler, and 128 registers per thread (a ninth warp per block would
-// leave 96).  The tile's shape is chosen per grid
-// (shape_of in efm_capi.cu) so that ragged grids do not leave threads idle; the shared-memory
-// slots below bound it.
+// leave 96).  The large blocks are the default on every grid: their wider tiles load fewer
+// neighbours per cell and hide more behind one another (forward + gradient, ms, large and the
+// better of the small ones' two rings: 64 x 64 x 64 1.92, 2.14; 96 x 96 x 64 3.36, 3.50; 128 x 128 x 96
+// 7.21, 8.23; 256 x 256 x 128 19.3, 21.2); the small ones are an option the autotuner times.  The
+// tile's shape is chosen per grid (shape_of in efm_capi.cu) so that ragged grids do not leave
+// threads idle; the shared-memory slots below bound it.
 #pragma once
 
 #define EFM_MAX_YCHUNK 64
