@@ -100,9 +100,10 @@ __global__ void k_sub(float *__restrict__ out, const float *__restrict__ a,
 // history vectors whose coefficients follow from the products s_i.y_j (i >= j, layers newest
 // first), y_i.y_j, s_i.g and y_i.g: one pass forms all of them, a small kernel runs the two loops
 // on them, one pass forms the combination (49 us at 200 x 200 x 100, 8 pairs: the DRAM rate).  Each
-// vector is read twice, 272 MB each time; vector by vector, every step of the recursion read and
-// wrote the direction and two more vectors (1.5 GB, about 70 launches, 740 us; now 130 us).  Products and combination are in float64;
-// the direction is rounded once, at the end, instead of after every step.
+// vector is read twice, 272 MB each time; vector by vector, every step of the recursion reads and
+// writes the direction and two more vectors (1.5 GB, about 70 launches, 740 us; this way 130 us).
+// Products and combination are in float64; the direction is rounded once, at the end, instead of
+// after every step.  Long histories of large vectors take the vectors (by_products).
 //
 // The products: a warp takes groups a >= b of eight layers and runs the float64 matrix instruction
 // (8 x 8 products, four cells per step) for y_a.y_b and s_a.y_b; a lane's four consecutive cells of
@@ -615,7 +616,8 @@ static cudaError_t gauss_line(const float *in, float *out, int64_t inner, int co
     int bx = 32;
     while (bx > 1 && bx / 2 >= wide) bx /= 2;
     const dim3 block(bx, 256 / bx);
-    const dim3 grid((unsigned)((wide + bx - 1) / bx), (unsigned)std::min<int64_t>((lines + block.y - 1) / block.y, 65535));
+    const dim3 grid((unsigned)((wide + bx - 1) / bx),
+                    (unsigned)std::min<int64_t>((lines + block.y - 1) / block.y, 65535));
     if (v4)
         k_gauss_line<4><<<grid, block, 0, s>>>(in, out, inner, count, step, outer, outer_step, g);
     else

@@ -233,8 +233,8 @@ EFM_API int efm_residual_misfit_noalloc(const float *mod_dev, const float *obs_d
  * latency or a plane's computation, so n = 1 gives up on a tile still in flight).  A wait that
  * runs out sets the context's error word (efm_status -> EFM_ERR_TIMEOUT), its block waits for
  * its own loads still in flight (default bound) and returns; the call completes with invalid
- * outputs, and the next call with the default limit is unaffected.  Small values exist for failure-detection tests (no reference
- * counterpart; the reference's kernels have no waits). */
+ * outputs, and the next call with the default limit is unaffected.  Small values exist for
+ * failure-detection tests (no reference counterpart; the reference's kernels have no waits). */
 #define EFM_OPT_WAIT_LIMIT 9
 /* EFM_GRAD_EXACT: how each transposed half-step runs.  2 (default): one plane-streaming
  * launch (each block marches a 32 x 16 column of cells along y, or 32 x 8 with
